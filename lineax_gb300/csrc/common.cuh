@@ -109,4 +109,51 @@ __device__ __forceinline__ void warp_argmax_first_key(long long& v, int& idx) {
   }
 }
 
+// Programmatic dependent launch.  A kernel launched by launch_pdl may start
+// while the kernel before it on the stream is still running; it must call
+// pdl_wait() (all threads) before it touches anything that kernel writes, and
+// may load data that no earlier kernel of the chain writes before that.
+// pdl_trigger() lets the next kernel of the chain start; the next kernel's
+// pdl_wait() still waits until this one has finished and its writes are
+// visible, so where the trigger stands never changes a result.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launch `fn` with programmatic stream serialisation (and a thread-block
+// cluster of `cluster` CTAs along x when cluster > 1).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*fn)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t st, int cluster, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, fn, static_cast<KArgs>(args)...);
+}
+
+// First maximum over a warp of (key, idx) with the lowest idx winning ties:
+// three 32-bit warp reductions (REDUX) instead of a five-step 64-bit shuffle
+// tree.  key 0 with idx INT_MAX marks a lane without a candidate.
+__device__ __forceinline__ void warp_first_max(unsigned long long& key, int& idx) {
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const unsigned mi =
+      __reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? (unsigned)idx : 0x7FFFFFFFu);
+  key = ((unsigned long long)mh << 32) | ml;
+  idx = (int)mi;
+}
+
 }  // namespace lxgb
