@@ -26,7 +26,7 @@
 #include <utility>
 
 #include "common.cuh"
-#include "tri.cuh"
+#include "trisolve.cuh"
 
 namespace lxgb {
 
@@ -759,52 +759,103 @@ int getrf_blocked(int n, double* a, int32_t* piv, int32_t* info, cudaStream_t st
 }
 
 // ---------------------------------------------------------------------------
-// getrs: one CTA per (system, right-hand side).  The vector and the pivots
-// are staged in shared memory when they fit.
+// getrs for n > kSmallMax: the row interchanges as one gather or scatter per
+// vector, then two multi-CTA triangular solves (trisolve.cu).
 // ---------------------------------------------------------------------------
 constexpr int kSolveThreads = 256;
+constexpr int kPermThreads = 1024;
+constexpr int kPermMaxN = 11000;   // 20 bytes of shared memory per row
 
-__global__ void __launch_bounds__(kSolveThreads)
-getrs_kernel(int n, int nrhs, const double* __restrict__ lu, int64_t stride_a,
-             const int32_t* __restrict__ piv, int64_t stride_piv, double* __restrict__ b,
-             int64_t stride_b, int trans, int in_smem) {
+// x = P x (or Pᵀ x) for the interchanges x_k <-> x_{p_k}, k = 0..n-1, p_k >= k:
+// one CTA per vector.  (P x)_i is final after interchange i, so its source is
+// found by walking back: position p_i before interchange i holds what the last
+// earlier interchange with the same partner put there, that is the value of a
+// position j < i before interchange j, and so on.  The interchanges of each
+// partner form a linked list; every row then walks a few links, instead of one
+// thread running n dependent exchanges (40 us at n = 2000, 3 us so).
+__global__ void __launch_bounds__(kPermThreads)
+getrs_perm_kernel(int n, const int32_t* __restrict__ piv, int64_t stride_piv,
+                  double* __restrict__ b, int64_t stride_b, int trans) {
   extern __shared__ double smem_x[];
-  __shared__ TrsvSmem<double> tsm;
-  const int sys = blockIdx.x / nrhs;
-  const int r = blockIdx.x % nrhs;
-  const double* A = lu + (int64_t)sys * stride_a;
-  const int32_t* P = piv + (int64_t)sys * stride_piv;
-  double* g = b + (int64_t)sys * stride_b + (int64_t)r * n;
-  double* x = g;
-  int32_t* sp = nullptr;
-  if (in_smem) {
-    x = smem_x;
-    sp = reinterpret_cast<int32_t*>(smem_x + n);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) { x[i] = g[i]; sp[i] = P[i]; }
-    __syncthreads();
+  double* x = smem_x;
+  int* head = reinterpret_cast<int*>(x + n);   // last-inserted interchange with partner q
+  int* next = head + n;                        // its list
+  int* last = next + n;                        // the latest interchange with partner k (all < k)
+  const int32_t* p = piv + (int64_t)blockIdx.y * stride_piv;
+  double* g = b + (int64_t)blockIdx.y * stride_b + (int64_t)blockIdx.x * n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    x[i] = g[i];
+    head[i] = -1;
   }
-  const int32_t* pp = in_smem ? sp : P;
-  if (!trans) {
+  __syncthreads();
+  int odd = 0;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const int q = p[j];
+    if (q < j || q >= n) odd = 1;
+    else if (q != j) next[j] = atomicExch(&head[q], j);
+  }
+  if (__syncthreads_or(odd)) {
+    // not a pivot sequence of getrf (a partner above the diagonal): in order
     if (threadIdx.x == 0)
-      for (int k = 0; k < n; ++k) {
-        const int p = pp[k];
-        if (p != k) { const double t = x[k]; x[k] = x[p]; x[p] = t; }
+      for (int s = 0; s < n; ++s) {
+        const int k = trans ? n - 1 - s : s;
+        const int q = p[k];
+        if (q != k && q >= 0 && q < n) { const double v = x[k]; x[k] = x[q]; x[q] = v; }
       }
     __syncthreads();
-    cta_trsv<double>(A, n, n, /*lower=*/true, /*trans=*/false, /*unit=*/true, x, tsm);
-    cta_trsv<double>(A, n, n, /*lower=*/false, /*trans=*/false, /*unit=*/false, x, tsm);
-  } else {
-    cta_trsv<double>(A, n, n, /*lower=*/false, /*trans=*/true, /*unit=*/false, x, tsm);
-    cta_trsv<double>(A, n, n, /*lower=*/true, /*trans=*/true, /*unit=*/true, x, tsm);
-    if (threadIdx.x == 0)
-      for (int k = n - 1; k >= 0; --k) {
-        const int p = pp[k];
-        if (p != k) { const double t = x[k]; x[k] = x[p]; x[p] = t; }
-      }
-    __syncthreads();
-  }
-  if (in_smem)
     for (int i = threadIdx.x; i < n; i += blockDim.x) g[i] = x[i];
+    return;
+  }
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    int m = -1;
+    for (int j = head[k]; j >= 0; j = next[j]) m = max(m, j);
+    last[k] = m;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int q = p[i];
+    int src = q;                               // the position before interchange i
+    int from = -1;
+    if (q == i) {
+      from = last[i];
+    } else {
+      for (int j = head[q]; j >= 0; j = next[j])
+        if (j < i) from = max(from, j);
+    }
+    while (from >= 0) {
+      src = from;
+      from = last[src];
+    }
+    if (trans) g[src] = x[i];
+    else g[i] = x[src];
+  }
+}
+
+// The same, in order and in global memory, for n above kPermMaxN.
+__global__ void getrs_swap_kernel(int n, const int32_t* __restrict__ piv, int64_t stride_piv,
+                                  double* __restrict__ b, int64_t stride_b, int trans) {
+  const int32_t* p = piv + (int64_t)blockIdx.y * stride_piv;
+  double* x = b + (int64_t)blockIdx.y * stride_b + (int64_t)blockIdx.x * n;
+  for (int s = 0; s < n; ++s) {
+    const int k = trans ? n - 1 - s : s;
+    const int q = p[k];
+    if (q != k) { const double v = x[k]; x[k] = x[q]; x[q] = v; }
+  }
+}
+
+static int getrs_perm(int64_t batch, int n, int nrhs, const int32_t* piv, int64_t stride_piv,
+                      double* b, int64_t stride_b, int trans, cudaStream_t st) {
+  const dim3 grid((unsigned)nrhs, (unsigned)batch);
+  if (n > kPermMaxN) {
+    getrs_swap_kernel<<<grid, 1, 0, st>>>(n, piv, stride_piv, b, stride_b, trans);
+    return check_launch("getrs swap");
+  }
+  const size_t smem = (size_t)n * (sizeof(double) + 3 * sizeof(int));
+  LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(getrs_perm_kernel), (int)smem),
+                "getrs: set smem");
+  const int threads = n < kPermThreads ? (n + 31) / 32 * 32 : kPermThreads;
+  getrs_perm_kernel<<<grid, threads, smem, st>>>(n, piv, stride_piv, b, stride_b, trans);
+  return check_launch("getrs perm");
 }
 
 // ---------------------------------------------------------------------------
@@ -1013,13 +1064,23 @@ extern "C" int lxgb_getrs_batched_f64(int64_t batch, int32_t n, int32_t nrhs, co
         n, nrhs, lu, stride_a, piv, stride_piv, b, stride_b, trans);
     return check_launch("getrs small");
   }
-  const size_t need = (size_t)n * (sizeof(double) + sizeof(int32_t));
-  const int in_smem = need <= 160 * 1024;
-  const size_t smem = in_smem ? need : 0;
-  if (in_smem)
-    LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(getrs_kernel), (int)smem),
-                  "getrs: set smem");
-  getrs_kernel<<<(unsigned)(batch * nrhs), kSolveThreads, smem, as_stream(stream)>>>(
-      n, nrhs, lu, stride_a, piv, stride_piv, b, stride_b, trans, in_smem);
-  return check_launch("getrs");
+  cudaStream_t st = as_stream(stream);
+  constexpr int64_t kMaxGrid = 65535;               // vectors and systems per launch
+  for (int64_t s0 = 0; s0 < batch; s0 += kMaxGrid) {
+    const int64_t sb = batch - s0 < kMaxGrid ? batch - s0 : kMaxGrid;
+    for (int64_t r0 = 0; r0 < nrhs; r0 += kMaxGrid) {
+      const int kb = (int)(nrhs - r0 < kMaxGrid ? nrhs - r0 : kMaxGrid);
+      const double* t = lu + s0 * stride_a;
+      const int32_t* p = piv + s0 * stride_piv;
+      double* x = b + s0 * stride_b + r0 * n;
+      int rc = trans ? LXGB_SUCCESSFUL : getrs_perm(sb, n, kb, p, stride_piv, x, stride_b, 0, st);
+      if (!rc)  // L y = P b, or Uᵀ z = b
+        rc = trisolve_blocked(sb, n, kb, t, n, stride_a, !trans, trans, !trans, x, stride_b, st);
+      if (!rc)  // U x = y, or Lᵀ w = z
+        rc = trisolve_blocked(sb, n, kb, t, n, stride_a, trans, trans, trans, x, stride_b, st);
+      if (!rc && trans) rc = getrs_perm(sb, n, kb, p, stride_piv, x, stride_b, 1, st);
+      if (rc) return rc;
+    }
+  }
+  return LXGB_SUCCESSFUL;
 }

@@ -1,0 +1,198 @@
+// Multi-CTA FP64 triangular solve, right-looking by blocks of 64 unknowns.
+//
+// Unknowns are numbered in solve order (u = 0 is solved first: row u of a
+// lower op(T), row n - 1 - u of an upper one), so every case is a forward
+// substitution with the matrix op(u, v) = op(T)[row(u)][row(v)], v <= u.
+// Launch b of the chain
+//   * CTA 0: subtracts block b-1's contribution from block b and solves it;
+//   * CTAs 1..: subtract block b-1's contribution from the rows after block b,
+//     64 rows each.
+// So each block costs one launch; matrix entries are loaded into registers
+// before the kernel waits for the launch before it (they do not depend on it).
+//
+// What bounds it: the chain of CTA 0.  A 64-unknown step takes about 8 us:
+// two 32-step substitutions by one warp (a shuffle and a dependent FP64 FMA
+// per step), the 64x64 update (2 FP64 FMA per clock and SM: 1 us) and the
+// hand-over between launches.  Four lanes share a row in the updates: 16 FMAs
+// and two shuffle additions per lane, against 2 FMAs and five additions with
+// a warp per row.  Measured (one vector, us): n = 128 26, n = 1000 128, n =
+// 2003 268; one CTA per vector with a division per unknown took 68 and 452 at
+// n = 128 and 767, and a diagonal and an update launch per block 549 and 1104
+// at n = 1000 and 2003.  getrs at n = 2003: 511 us against 2500 to 6200 (the
+// more interchanges, the longer: one thread ran them in order).
+#include "trisolve.cuh"
+
+namespace lxgb {
+
+constexpr int kTsThreads = 256;
+
+struct TsView {
+  const double* t;
+  int64_t ldt;
+  int n;
+  bool fwd, trans;
+  __device__ __forceinline__ int64_t row(int u) const { return fwd ? u : n - 1 - u; }
+  __device__ __forceinline__ double op(int u, int v) const {
+    const int64_t i = row(u), j = row(v);
+    return trans ? t[j * ldt + i] : t[i * ldt + j];
+  }
+};
+
+// Whether x is zero or of moderate size (2^-500 < |x| < 2^500), by its exponent.
+__device__ __forceinline__ bool ts_moderate(double x, bool zero_ok) {
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
+  const unsigned e = hi >> 20;
+  if (zero_ok && hi == 0u && __double2loint(x) == 0) return true;
+  return e > 523u && e < 1523u;
+}
+
+// One warp solves a 32-unknown block: lane l holds v = b_l and d[t] = op(l, t)
+// (0 for t >= l, or past the block's end), dd = op(l, l) (1 for unit
+// diagonals and past the end).  `scaled`: d[t] was multiplied by 1/op(t, t),
+// so a step is v_l -= d[t] v_t on unscaled v and x_l = v_l / op(l, l) at the
+// end: a shuffle and an FMA per step.  Otherwise (entries whose scaling could
+// overflow or underflow, zeros and non-finite values on the diagonal) every
+// unknown is divided in turn.
+__device__ __forceinline__ double ts_solve32(double v, const double (&d)[32], double dd,
+                                             double rinv, bool scaled) {
+  if (scaled) {
+#pragma unroll
+    for (int t = 0; t < 31; ++t) {
+      const double vt = __shfl_sync(0xffffffffu, v, t);
+      v = fma(-d[t], vt, v);  // d[t] = 0 for t >= lane
+    }
+    return v * rinv;
+  }
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < 32; ++t) {
+    double xt = (lane == t) ? v / dd : 0.0;
+    xt = __shfl_sync(0xffffffffu, xt, t);
+    if (lane == t) v = xt;
+    if (lane > t) v = fma(-d[t], xt, v);
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(kTsThreads)
+trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t stride_t,
+                     int fwd, int trans, int unit, int b, double* __restrict__ x,
+                     int64_t stride_x) {
+  __shared__ double xp[kTsNB], xc[kTsNB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const TsView T{t + (int64_t)blockIdx.z * stride_t, ldt, n, fwd != 0, trans != 0};
+  double* xv = x + (int64_t)blockIdx.z * stride_x + (int64_t)blockIdx.y * n;
+  const int u0 = b * kTsNB;
+  const int p0 = u0 - kTsNB;                       // the block solved by the launch before
+  const bool chain = blockIdx.x == 0;
+  // rows this CTA updates: its block (CTA 0) or 64 rows after it
+  const int w0 = u0 + (int)blockIdx.x * kTsNB;
+  const int wi = tid >> 2, wq = tid & 3;           // row, part: columns 4 pp + wq
+  double cu[16];
+  if (b > 0) {
+#pragma unroll
+    for (int pp = 0; pp < 16; ++pp)
+      cu[pp] = (w0 + wi < n) ? T.op(w0 + wi, p0 + 4 * pp + wq) : 0.0;
+  }
+  // CTA 0: the diagonal block.  Warp 0 holds its first 32 unknowns' matrix,
+  // warp 1 the second 32's; every thread 4 entries of the block below the
+  // first (row tid >> 3, columns 8 pp + (tid & 7)).
+  double d[32], dd = 1.0, rinv = 1.0, cs[4];
+  bool scaled = true;
+  if (chain) {
+    if (warp < 2) {
+      const int ul = u0 + 32 * warp + lane;
+      bool ok = true;
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        const int uk = u0 + 32 * warp + k;
+        d[k] = (ul < n && k < lane) ? T.op(ul, uk) : 0.0;
+        ok = ok && ts_moderate(d[k], true);
+      }
+      if (!unit) {
+        if (ul < n) dd = T.op(ul, ul);
+        ok = ok && ts_moderate(dd, false);
+        scaled = __all_sync(0xffffffffu, ok);
+        if (scaled) {
+          rinv = 1.0 / dd;
+#pragma unroll
+          for (int k = 0; k < 32; ++k) d[k] *= __shfl_sync(0xffffffffu, rinv, k);
+        }
+      }
+    }
+#pragma unroll
+    for (int pp = 0; pp < 4; ++pp) {
+      const int ur = u0 + 32 + (tid >> 3);
+      cs[pp] = (ur < n) ? T.op(ur, u0 + 8 * pp + (tid & 7)) : 0.0;
+    }
+  }
+  pdl_wait();
+  pdl_trigger();
+  double* mine = (b > 0 && tid < kTsNB) ? &xp[tid] : nullptr;
+  if (mine) *mine = xv[T.row(p0 + tid)];
+  if (tid >= kTsNB && tid < 2 * kTsNB) {
+    const int u = w0 + tid - kTsNB;
+    xc[tid - kTsNB] = (u < n) ? xv[T.row(u)] : 0.0;
+  }
+  __syncthreads();
+  if (b > 0) {
+    double acc[2] = {0.0, 0.0};
+#pragma unroll
+    for (int pp = 0; pp < 16; ++pp) acc[pp & 1] = fma(cu[pp], xp[4 * pp + wq], acc[pp & 1]);
+    double s = acc[0] + acc[1];
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (wq == 0) {
+      const double v = xc[wi] - s;
+      if (chain) xc[wi] = v;
+      else if (w0 + wi < n) xv[T.row(w0 + wi)] = v;
+    }
+  }
+  if (!chain) return;
+  __syncthreads();
+  if (warp == 0) {
+    const double v = ts_solve32(xc[lane], d, dd, rinv, scaled);
+    xc[lane] = v;
+    if (u0 + lane < n) xv[T.row(u0 + lane)] = v;
+  }
+  if (u0 + 32 >= n) return;                        // uniform
+  __syncthreads();
+  {
+    double s = 0.0;
+#pragma unroll
+    for (int pp = 0; pp < 4; ++pp) s = fma(cs[pp], xc[8 * pp + (tid & 7)], s);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    if ((tid & 7) == 0) xc[32 + (tid >> 3)] -= s;
+  }
+  __syncthreads();
+  if (warp == 1) {
+    const double v = ts_solve32(xc[32 + lane], d, dd, rinv, scaled);
+    if (u0 + 32 + lane < n) xv[T.row(u0 + 32 + lane)] = v;
+  }
+}
+
+int trisolve_blocked(int64_t batch, int n, int nrhs, const double* t, int64_t ldt,
+                     int64_t stride_t, int lower, int trans, int unit, double* x,
+                     int64_t stride_x, cudaStream_t st) {
+  const int fwd = (lower != 0) != (trans != 0);
+  const int nblk = (n + kTsNB - 1) / kTsNB;
+  for (int b = 0; b < nblk; ++b) {
+    const int after = n - (b + 1) * kTsNB;         // rows after this block
+    const unsigned gx = 1u + (unsigned)((b > 0 && after > 0) ? (after + kTsNB - 1) / kTsNB : 0);
+    const dim3 grid(gx, (unsigned)nrhs, (unsigned)batch);
+    if (b == 0) {
+      // not a dependent launch: the kernel before it may still write the matrix
+      trisolve_step_kernel<<<grid, kTsThreads, 0, st>>>(n, t, ldt, stride_t, fwd, trans, unit, b,
+                                                        x, stride_x);
+    } else {
+      LXGB_CUDA_TRY(launch_pdl(trisolve_step_kernel, grid, dim3(kTsThreads), 0, st, 1, n, t, ldt,
+                               stride_t, fwd, trans, unit, b, x, stride_x),
+                    "trisolve: launch");
+    }
+  }
+  return check_launch("trisolve");
+}
+
+}  // namespace lxgb

@@ -1,0 +1,78 @@
+"""GPU parity of the multi-CTA triangular solve and of the LU solve's row
+interchanges, at the edges of their 32- and 64-unknown blocks."""
+
+import numpy as np
+import pytest
+import torch
+
+from lineax_gb300 import _dense
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+def _t(x, dev):
+    return torch.tensor(np.asarray(x), dtype=torch.float64, device=dev)
+
+
+@pytest.mark.parametrize("lower,trans", [(True, False), (False, False), (True, True),
+                                         (False, True)])
+@pytest.mark.parametrize("n", [1, 32, 33, 63, 64, 65, 96, 97, 129, 200])
+def test_trsm_block_edges(dev, n, lower, trans):
+    """Componentwise backward error of substitution with rounded reciprocals:
+    |op(T) x - b| <= (n + 4) u |op(T)| |x| (residual in extended precision),
+    for three vectors and rows longer than the matrix."""
+    rng = np.random.default_rng(n)
+    m = rng.standard_normal((n, n + 5))
+    m[np.arange(n), np.arange(n)] += np.sign(m[np.arange(n), np.arange(n)])
+    b = rng.standard_normal((3, n))
+    x = _dense.trsv(_t(m, dev)[:, :n] if n == 1 else _t(m, dev), _t(b, dev), lower=lower,
+                    trans=trans, unit=False).cpu().numpy()
+    tri = np.tril(m[:, :n]) if lower else np.triu(m[:, :n])
+    tri = tri.T if trans else tri
+    for c in range(3):
+        res = np.abs(tri.astype(np.longdouble) @ x[c].astype(np.longdouble) - b[c])
+        assert (res <= (n + 4) * U * (np.abs(tri) @ np.abs(x[c]))).all()
+
+
+@pytest.mark.parametrize("scale", [1e-250, 1e250])
+def test_trsm_extreme_scaling_divides(dev, scale):
+    """Entries too large or small to be scaled ahead take the dividing path:
+    the backward error bound of test_trsm_block_edges."""
+    n = 70
+    rng = np.random.default_rng(3)
+    m = np.tril(np.sign(rng.standard_normal((n, n))) * 2.0 ** rng.integers(-2, 3, (n, n)))
+    m[40:, :] *= scale
+    m[np.arange(n), np.arange(n)] = np.where(np.arange(n) < 40, 1.0, scale)
+    b = m.sum(1)
+    x = _dense.trsv(_t(m, dev), _t(b, dev), lower=True, trans=False, unit=False).cpu().numpy()
+    res = np.abs(m.astype(np.longdouble) @ x.astype(np.longdouble) - b)
+    assert (res <= (n + 4) * U * (np.abs(m) @ np.abs(x))).all()
+
+
+def test_trsm_zero_diagonal_is_not_finite(dev):
+    m = np.eye(100)
+    m[70, 70] = 0.0
+    x = _dense.trsv(_t(m, dev), _t(np.ones(100), dev), lower=True, trans=False,
+                    unit=False).cpu().numpy()
+    assert np.isinf(x[70]) and np.isfinite(x[:70]).all()
+
+
+@pytest.mark.parametrize("n", [169, 300, 1200])
+@pytest.mark.parametrize("kind", ["random", "shift", "last", "none", "any"])
+def test_getrs_interchanges(dev, n, kind):
+    """P b and Pᵀ b of pivot sequences with long and short chains (and of one
+    with partners above the diagonal), through identity factors: exact."""
+    rng = np.random.default_rng(n)
+    k = np.arange(n)
+    piv = {"random": k + (rng.random(n) * (n - k)).astype(int), "shift": np.minimum(k + 1, n - 1),
+           "last": np.full(n, n - 1), "none": k, "any": rng.integers(0, n, n)}[kind]
+    b = rng.standard_normal((2, 3, n))
+    lu = _t(np.stack([np.eye(n)] * 2), dev)
+    pv = torch.tensor(np.stack([piv] * 2).astype(np.int32), device=dev)
+    for trans in (0, 1):
+        ref = b.copy()
+        for i in (range(n) if not trans else range(n - 1, -1, -1)):
+            ref[..., [i, piv[i]]] = ref[..., [piv[i], i]]
+        got = _dense.lu_solve_batched(lu, pv, _t(b, dev), trans=trans).cpu().numpy()
+        np.testing.assert_array_equal(got, ref)
