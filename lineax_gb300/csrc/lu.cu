@@ -392,32 +392,48 @@ panel_getf2_kernel(int n, int j0, int nb, double* __restrict__ a, int32_t* __res
 // split over up to 16 CTAs (R each) and every row lives in the registers of
 // TPR threads (thread t of a row holds the columns q * TPR + t), so the
 // rank-1 updates run on 16 SMs without touching memory.
-// Per column: warp and CTA first-maximum of |a| by integer reductions; every
-// CTA pushes its candidate (key, row index, the row itself, and row kk from
-// its owner) into all CTAs' shared memory, then one cluster barrier; after it
-// each CTA picks the same winner from local data.  The slots alternate with
-// the column's parity: a CTA rewrites a slot only after the barrier of the
-// next column, which every CTA reaches after it has read the slot.
-// Arithmetic and pivot choice are those of panel_getf2_kernel (getf2).
-// Measured: n = 1000, 59 us a panel on average against 158 us on one CTA;
-// n = 2003, 72 us against 301 us.  A column costs about 1.8 us, most of it the
-// exchange (two block barriers, the push, the cluster barrier) and the pivot's
-// reciprocal, not the arithmetic.
+// A column costs an exchange over the cluster, and what bounds it is latency
+// (measured, cycles: cluster barrier 380, plus 35 for each CTA that a candidate
+// is stored to, remote load 350, division 330, FP64 FMA 64 and as much for
+// every further warp on the sub-partition).  So per column kk:
+//   1. the first maximum of |a| over the CTA by integer reductions (warp, one
+//      block barrier, again), its (key, row) stored into every CTA's slots;
+//   2. while those stores travel, the columns after kk take the update of step
+//      kk - 1 (only column kk took it at once), a warp without rows forms
+//      the reciprocal of the CTA's candidate, and the candidate's row and row kk
+//      are laid out in this CTA's shared memory;
+//   3. one cluster barrier; every warp picks the same winner from local slots;
+//      the winning row and its reciprocal are read from the winner's CTA;
+//   4. rows swapped, column kk scaled, column kk + 1 updated.
+// Slots and staging alternate with the column's parity: a CTA rewrites one
+// only after the barrier of the next column, which every CTA reaches after it
+// has read it.  Arithmetic and pivot choice are those of panel_getf2_kernel.
+// Measured, a 32-column panel on average: n = 1000 50 us (158 us on one CTA),
+// n = 2003 60 us (301 us); 1.5 us a column at n = 1000: search 0.35, update
+// beside division 0.35, barrier 0.25, winner and its row 0.4, scaling 0.2.
 // ---------------------------------------------------------------------------
 constexpr int kPcluMax = 16;        // CTAs per cluster
-constexpr int kPcluThreads = 512;
+constexpr int kPcluRowThreads = 512;                  // threads that hold rows
+constexpr int kPcluThreads = kPcluRowThreads + 32;    // and the warp that divides
+// Unused dynamic shared memory that a panel CTA reserves, so that no CTA of
+// the trailing update running beside it (17 KB each) shares its SM's FP64 pipe.
+constexpr int kPcluReserve = 212 * 1024;
 constexpr int kPcluRows = 32;       // aimed rows per CTA (fewer CTAs for short panels)
-constexpr int kPcluMaxM = kPcluMax * kPcluThreads;  // tallest panel (one thread per row)
+constexpr int kPcluMaxM = kPcluMax * kPcluRowThreads;  // tallest panel (one thread per row)
 
-struct PanelSlots {
-  double row[2][kPcluMax][kNB];     // candidate rows by parity and CTA
-  double rowk[2][kNB];              // row kk
-  unsigned long long key[2][kPcluMax];
-  int idx[2][kPcluMax];
-  double mine[kNB], minek[kNB];     // staging for the push
-  unsigned long long wkey[kPcluThreads / 32];
-  int widx[kPcluThreads / 32];
-  double rcp[2];
+struct __align__(16) PanelKey {
+  unsigned long long key;
+  long long idx;
+};
+
+struct PanelSmem {
+  PanelKey slot[2][kPcluMax];            // candidates of all CTAs, by parity
+  PanelKey cand[2][kPcluThreads / 32];   // this CTA's, by parity and warp
+  double cval[2][kPcluThreads / 32];     // and their values
+  __align__(16) double mine[2][kNB + 2]; // this CTA's candidate row, then its reciprocal
+  __align__(16) double minek[2][kNB + 2];  // row kk (its owner's; no reciprocal)
+  __align__(16) double prow[2][kNB + 2]; // the pivot row and reciprocal, received
+  __align__(16) double rowk[kNB];        // row kk, received by the pivot row's owner
 };
 
 template <int TPR>
@@ -426,7 +442,7 @@ panel_getf2_cluster_kernel(int n, int j0, int nb, int rows_per_cta, double* __re
                            int32_t* __restrict__ piv, int32_t* __restrict__ info) {
   namespace cg = cooperative_groups;
   constexpr int Q = kNB / TPR;      // columns per thread
-  __shared__ PanelSlots sm;
+  __shared__ PanelSmem sm;
   cg::cluster_group cluster = cg::this_cluster();
   const int ncta = (int)cluster.num_blocks();
   const int rank = (int)cluster.block_rank();
@@ -438,12 +454,17 @@ panel_getf2_cluster_kernel(int n, int j0, int nb, int rows_per_cta, double* __re
   const bool has = lr < R && gi < m;
   double r[Q];
   pdl_wait();
+  // everything before this panel is finished: the rest of the previous
+  // panel's trailing update may start beside it
+  pdl_trigger();
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int c = q * TPR + t;
     r[q] = (has && c < nb) ? a[(int64_t)(j0 + gi) * n + j0 + c] : 0.0;
   }
   int bad = 0;
+  double l = 0.0;                   // this row's multiplier of the step before
+  bool act = false;                 // and whether that step updates the row
   cluster.sync();                   // every CTA runs before any remote store
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
@@ -452,7 +473,7 @@ panel_getf2_cluster_kernel(int n, int j0, int nb, int rows_per_cta, double* __re
       const int kk = q * TPR + tt;
       if (kk >= nb) break;          // uniform over the cluster
       const int par = kk & 1;
-      // 1. this CTA's first max |a| in column kk (key 0: no candidate, NaN)
+      // 1. the CTA's first max |a| in column kk (key 0: none, NaN)
       unsigned long long key = 0;
       int idx = INT_MAX;
       if (has && t == tt && gi >= kk) {
@@ -460,80 +481,98 @@ panel_getf2_cluster_kernel(int n, int j0, int nb, int rows_per_cta, double* __re
         if (b >= 0) { key = (unsigned long long)b + 1; idx = gi; }
       }
       warp_first_max(key, idx);
-      if (lane == 0) { sm.wkey[warp] = key; sm.widx[warp] = idx; }
+      if (lane == 0) { sm.cand[par][warp].key = key; sm.cand[par][warp].idx = idx; }
+      if (has && t == tt && gi == idx) sm.cval[par][warp] = r[q];
       __syncthreads();
-      key = lane < nwarps ? sm.wkey[lane] : 0ull;
-      idx = lane < nwarps ? sm.widx[lane] : INT_MAX;
+      key = lane < nwarps ? sm.cand[par][lane].key : 0ull;
+      idx = lane < nwarps ? (int)sm.cand[par][lane].idx : INT_MAX;
+      const unsigned long long wk = key;
+      const int wi = idx;
       warp_first_max(key, idx);
-      // 2. its row, and row kk, staged and pushed to every CTA
+      if (warp == 0 && lane < ncta) {
+        PanelKey* dst = cluster.map_shared_rank(&sm.slot[par][rank], lane);
+        *reinterpret_cast<longlong2*>(dst) = make_longlong2((long long)key, (long long)idx);
+      }
+      // 2. meanwhile the rest of step kk - 1, and what the others will read
+      if (warp == nwarps - 1) {
+        const unsigned mask = __ballot_sync(0xffffffffu, wk == key && wi == idx);
+        const double rc = 1.0 / sm.cval[par][__ffs(mask) - 1];
+        if (lane == 0) sm.mine[par][kNB] = rc;
+      }
+      if (act) {
+#pragma unroll
+        for (int c = q + 1; c < Q; ++c) r[c] = fma(-l, sm.prow[par ^ 1][c * TPR + t], r[c]);
+      }
       if (has && gi == idx) {
 #pragma unroll
-        for (int c = 0; c < Q; ++c) sm.mine[c * TPR + t] = r[c];
+        for (int c = 0; c < Q; ++c) sm.mine[par][c * TPR + t] = r[c];
       }
-      const bool own_k = kk >= rank * R && kk < rank * R + R;
-      if (own_k && has && gi == kk) {
+      if (has && gi == kk) {
 #pragma unroll
-        for (int c = 0; c < Q; ++c) sm.minek[c * TPR + t] = r[c];
-      }
-      __syncthreads();
-      for (int e = tid; e < ncta * kNB; e += (int)blockDim.x) {
-        const int dst = e / kNB, c = e % kNB;
-        if (key != 0ull) cluster.map_shared_rank(&sm.row[par][rank][0], dst)[c] = sm.mine[c];
-        if (own_k) cluster.map_shared_rank(&sm.rowk[par][0], dst)[c] = sm.minek[c];
-        if (c == 0) {
-          *cluster.map_shared_rank(&sm.key[par][rank], dst) = key;
-          *cluster.map_shared_rank(&sm.idx[par][rank], dst) = idx;
-        }
+        for (int c = 0; c < Q; ++c) sm.minek[par][c * TPR + t] = r[c];
       }
       cluster.sync();               // the one cluster barrier of the column
       // 3. the winner, from local shared memory (the same in every CTA)
-      key = lane < ncta ? sm.key[par][lane] : 0ull;
-      idx = lane < ncta ? sm.idx[par][lane] : INT_MAX;
+      key = lane < ncta ? sm.slot[par][lane].key : 0ull;
+      idx = lane < ncta ? (int)sm.slot[par][lane].idx : INT_MAX;
       warp_first_max(key, idx);
       const bool none = key == 0ull;          // a column of NaNs: row kk stays
       const int p = none ? kk : idx;
-      const double* prow = none ? sm.rowk[par] : sm.row[par][p / R];
+      const int own_p = p / R, own_k = kk / R;
+      if (warp == nwarps - 1) {
+        if (lane <= kNB / 2) {      // the row and, behind it, the reciprocal
+          const double* src = cluster.map_shared_rank(none ? sm.minek[par] : sm.mine[par], own_p);
+          reinterpret_cast<double2*>(sm.prow[par])[lane] =
+              reinterpret_cast<const double2*>(src)[lane];
+        }
+      } else if (warp == 0 && own_p == rank) {
+        sm.rowk[lane] = cluster.map_shared_rank(sm.minek[par], own_k)[lane];
+      }
+      __syncthreads();
+      const double* prow = sm.prow[par];
       const double akk = prow[kk];
       const bool live = (__double_as_longlong(akk) << 1) != 0;  // akk != 0 (NaN included)
-      // the reciprocal once per CTA: a division is a long FP64 sequence
-      if (warp == 0) sm.rcp[par] = 1.0 / akk;
       if (live && p != kk && has) {
         if (gi == kk) {
 #pragma unroll
           for (int c = 0; c < Q; ++c) r[c] = prow[c * TPR + t];
         } else if (gi == p) {
 #pragma unroll
-          for (int c = 0; c < Q; ++c) r[c] = sm.rowk[par][c * TPR + t];
+          for (int c = 0; c < Q; ++c) r[c] = sm.rowk[c * TPR + t];
         }
       }
       if (rank == 0 && tid == 0) {
         piv[j0 + kk] = j0 + p;
         if (!live && bad == 0) bad = j0 + kk + 1;
       }
-      __syncthreads();
-      // 4. scale column kk and update the columns after it
-      const bool act = has && gi > kk;
-      double l = r[q];
+      // 4. column kk scaled; the update of column kk + 1 (with the rest of
+      // its register column), the others follow in the next step
+      act = has && gi > kk;
+      l = r[q];
       if (live && act && t == tt) {
-        l = scale_pivot(l, akk, sm.rcp[par], fabs(akk) >= DBL_MIN);
+        // |akk| >= DBL_MIN (false for NaN) from its bits: an FP64 comparison
+        // would take the FP64 pipe like a multiplication
+        const unsigned hi = (unsigned)__double2hiint(akk) & 0x7FFFFFFFu;
+        const bool use_recip = hi - 0x00100000u < 0x7FE00000u ||
+                               (hi == 0x7FF00000u && __double2loint(akk) == 0);
+        l = scale_pivot(l, akk, prow[kNB], use_recip);
         r[q] = l;
       }
       if (TPR > 1) l = __shfl_sync(0xffffffffu, l, (lane & ~(TPR - 1)) | tt);
-      if (act) {
-        if (t > tt) r[q] = fma(-l, prow[q * TPR + t], r[q]);
-#pragma unroll
-        for (int c = q + 1; c < Q; ++c) r[c] = fma(-l, prow[c * TPR + t], r[c]);
+      if (tt + 1 < TPR) {
+        if (act && t > tt) r[q] = fma(-l, prow[q * TPR + t], r[q]);
+      } else if (q + 1 < Q) {
+        if (act) r[q + 1 < Q ? q + 1 : q] = fma(-l, prow[(q + 1) * TPR + t], r[q + 1 < Q ? q + 1 : q]);
       }
     }
   }
-  pdl_trigger();
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const int c = q * TPR + t;
     if (has && c < nb) a[(int64_t)(j0 + gi) * n + j0 + c] = r[q];
   }
   if (rank == 0 && tid == 0 && bad != 0 && *info == 0) *info = bad;
-  cluster.sync();  // no CTA leaves while another may still store into its shared memory
+  cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // Whether a cluster of c CTAs of this kernel can be co-scheduled on the
@@ -549,11 +588,14 @@ static bool panel_clu_fits(int c) {
   auto it = known.find(key);
   if (it != known.end()) return it->second;
   bool ok = cudaFuncSetAttribute(panel_getf2_cluster_kernel<TPR>,
-                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            ensure_dynamic_smem(reinterpret_cast<const void*>(panel_getf2_cluster_kernel<TPR>),
+                                kPcluReserve) == cudaSuccess;
   if (ok) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)c);
     cfg.blockDim = dim3(kPcluThreads);
+    cfg.dynamicSmemBytes = kPcluReserve;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)c;
@@ -575,10 +617,10 @@ template <int TPR>
 static int launch_panel_clu(int c, int R, int n, int j0, int nb, double* a, int32_t* piv,
                             int32_t* info, cudaStream_t st) {
   if (!panel_clu_fits<TPR>(c)) return -1;
-  const int threads = (R * TPR + 31) / 32 * 32;
+  const int threads = (R * TPR + 31) / 32 * 32 + 32;
   const cudaError_t e =
-      launch_pdl(panel_getf2_cluster_kernel<TPR>, dim3((unsigned)c), dim3((unsigned)threads), 0, st,
-                 c, n, j0, nb, R, a, piv, info);
+      launch_pdl(panel_getf2_cluster_kernel<TPR>, dim3((unsigned)c), dim3((unsigned)threads),
+                 kPcluReserve, st, c, n, j0, nb, R, a, piv, info);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return -1;
@@ -599,8 +641,8 @@ static int launch_panel(int n, int j0, int nb, double* a, int32_t* piv, int32_t*
   if (c > kPcluMax) c = kPcluMax;
   const int R = (m + c - 1) / c;
   c = (m + R - 1) / R;              // no empty CTA
-  if (R <= kPcluThreads / 4) return launch_panel_clu<4>(c, R, n, j0, nb, a, piv, info, st);
-  if (R <= kPcluThreads / 2) return launch_panel_clu<2>(c, R, n, j0, nb, a, piv, info, st);
+  if (R <= kPcluRowThreads / 4) return launch_panel_clu<4>(c, R, n, j0, nb, a, piv, info, st);
+  if (R <= kPcluRowThreads / 2) return launch_panel_clu<2>(c, R, n, j0, nb, a, piv, info, st);
   return launch_panel_clu<1>(c, R, n, j0, nb, a, piv, info, st);
 }
 
@@ -680,34 +722,40 @@ swap_trsm_kernel(int n, int j0, int nb, double* __restrict__ a, const int32_t* _
 }
 
 // Trailing update A22 -= L21 U12 (k = j0..j0+nb-1), each element an FMA chain
-// from its stored value.  32x32 tile per CTA, 2x4 per thread: the FP64 pipe
-// bounds it at any tile size, so small tiles only shorten the last wave (n =
-// 1000: 27 us a panel against 45 us with 64x64 tiles; n = 2003: 79 against 95).
+// from its stored value, on the columns from c_lo on (c_lo a multiple of kGT
+// past the panel).  32x32 tile per CTA, 2x4 per thread: the FP64 pipe bounds
+// it at any tile size, so small tiles only shorten the last wave (n = 1000: 27
+// us a panel against 45 us with 64x64 tiles; n = 2003: 79 against 95).
+//
+// This is the part of the update that the next panel does not need: it is
+// launched behind that panel (a dependent launch, released as soon as the
+// panel's CTAs have started) and runs beside it.  It therefore reads at once
+// what kernels finished before the panel wrote (through L2: __ldcg), touches
+// none of the panel's columns, and waits for the panel only before it ends, so
+// that whatever follows it follows both.
 constexpr int kGT = 32;
 __global__ void __launch_bounds__(128)
-gemm_trailing_kernel(int n, int j0, int nb, double* __restrict__ a) {
+gemm_trailing_kernel(int n, int j0, int nb, int c_lo, double* a) {
   __shared__ double Ls[kGT][kNB + 1];
   __shared__ double Us[kNB][kGT + 2];
-  const int s = j0 + nb;
-  const int i0 = s + blockIdx.y * kGT;
-  const int c0 = s + blockIdx.x * kGT;
+  const int i0 = j0 + nb + blockIdx.y * kGT;
+  const int c0 = c_lo + blockIdx.x * kGT;
   const int tid = threadIdx.x;
   const int tx = tid & 7, ty = tid >> 3;
-  pdl_wait();
   double acc[2][4];
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int i = i0 + ty + 16 * r, j = c0 + tx + 8 * c;
-      acc[r][c] = (i < n && j < n) ? a[(int64_t)i * n + j] : 0.0;
+      acc[r][c] = (i < n && j < n) ? __ldcg(a + (int64_t)i * n + j) : 0.0;
     }
 #pragma unroll
   for (int e0 = 0; e0 < kGT * kNB; e0 += 128) {
     const int e = e0 + tid;
     const int r = e / kNB, k = e % kNB;
-    Ls[r][k] = (i0 + r < n && k < nb) ? a[(int64_t)(i0 + r) * n + j0 + k] : 0.0;
-    Us[r][k] = (c0 + k < n && r < nb) ? a[(int64_t)(j0 + r) * n + c0 + k] : 0.0;
+    Ls[r][k] = (i0 + r < n && k < nb) ? __ldcg(a + (int64_t)(i0 + r) * n + j0 + k) : 0.0;
+    Us[r][k] = (c0 + k < n && r < nb) ? __ldcg(a + (int64_t)(j0 + r) * n + c0 + k) : 0.0;
   }
   __syncthreads();
 #pragma unroll 8
@@ -722,7 +770,6 @@ gemm_trailing_kernel(int n, int j0, int nb, double* __restrict__ a) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[r][c] = fma(-l[r], u[c], acc[r][c]);
   }
-  pdl_trigger();
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
@@ -730,6 +777,52 @@ gemm_trailing_kernel(int n, int j0, int nb, double* __restrict__ a) {
       const int i = i0 + ty + 16 * r, j = c0 + tx + 8 * c;
       if (i < n && j < n) a[(int64_t)i * n + j] = acc[r][c];
     }
+  pdl_wait();
+}
+
+// The same update on the next panel's columns [j0+nb, j0+nb+32), ahead of the
+// rest.  8x32 tile per CTA: these few columns are on the critical path, and
+// only as many SMs work on them as there are tiles.
+constexpr int kNxRows = 8;
+__global__ void __launch_bounds__(128)
+gemm_next_panel_kernel(int n, int j0, int nb, double* __restrict__ a) {
+  __shared__ double Ls[kNxRows][kNB + 1];
+  __shared__ double Us[kNB][kNB];
+  const int s = j0 + nb;
+  const int i0 = s + (int)blockIdx.x * kNxRows;
+  const int tid = threadIdx.x;
+  const int tx = tid & 15, ty = tid >> 4;
+  const int i = i0 + ty;
+  pdl_wait();
+  double acc[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int j = s + tx + 16 * c;
+    acc[c] = (i < n && j < n) ? a[(int64_t)i * n + j] : 0.0;
+  }
+#pragma unroll
+  for (int e = tid; e < kNxRows * kNB; e += 128) {
+    const int r = e / kNB, k = e % kNB;
+    Ls[r][k] = (i0 + r < n && k < nb) ? a[(int64_t)(i0 + r) * n + j0 + k] : 0.0;
+  }
+#pragma unroll
+  for (int e = tid; e < kNB * kNB; e += 128) {
+    const int k = e / kNB, c = e % kNB;
+    Us[k][c] = (s + c < n && k < nb) ? a[(int64_t)(j0 + k) * n + s + c] : 0.0;
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int k = 0; k < nb; ++k) {
+    const double l = Ls[ty][k];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) acc[c] = fma(-l, Us[k][tx + 16 * c], acc[c]);
+  }
+  pdl_trigger();
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int j = s + tx + 16 * c;
+    if (i < n && j < n) a[(int64_t)i * n + j] = acc[c];
+  }
 }
 
 __global__ void zero_info_kernel(int32_t* info, int64_t count) {
@@ -737,12 +830,18 @@ __global__ void zero_info_kernel(int32_t* info, int64_t count) {
   if (i < count) info[i] = 0;
 }
 
+// Per panel: its interchanges and block row, the update of the next panel's
+// columns, the next panel, and beside that panel the rest of the update.
 int getrf_blocked(int n, double* a, int32_t* piv, int32_t* info, cudaStream_t st) {
   zero_info_kernel<<<1, 32, 0, st>>>(info, 1);
-  for (int j0 = 0; j0 < n; j0 += kNB) {
+  auto panel = [&](int j0) {
     const int nb = min(kNB, n - j0);
     if (launch_panel(n, j0, nb, a, piv, info, st) != 0)
       panel_getf2_kernel<<<1, kPanelThreads, 0, st>>>(n, j0, nb, a, piv, info);
+  };
+  panel(0);
+  for (int j0 = 0; j0 < n; j0 += kNB) {
+    const int nb = min(kNB, n - j0);
     const int rest = n - j0 - nb;
     const int strips = (j0 + kStCols - 1) / kStCols + (rest + kStCols - 1) / kStCols;
     if (strips > 0)
@@ -750,9 +849,18 @@ int getrf_blocked(int n, double* a, int32_t* piv, int32_t* info, cudaStream_t st
                                1, n, j0, nb, a, piv),
                     "getrf: swap_trsm launch");
     if (rest > 0) {
-      const unsigned g = (unsigned)((rest + kGT - 1) / kGT);
-      LXGB_CUDA_TRY(launch_pdl(gemm_trailing_kernel, dim3(g, g), dim3(128), 0, st, 1, n, j0, nb, a),
-                    "getrf: gemm launch");
+      LXGB_CUDA_TRY(launch_pdl(gemm_next_panel_kernel,
+                               dim3((unsigned)((rest + kNxRows - 1) / kNxRows)), dim3(128), 0, st,
+                               1, n, j0, nb, a),
+                    "getrf: next panel update launch");
+      panel(j0 + nb);
+      const int wide = rest - kNB;               // columns after the next panel's
+      if (wide > 0)
+        LXGB_CUDA_TRY(launch_pdl(gemm_trailing_kernel,
+                                 dim3((unsigned)((wide + kGT - 1) / kGT),
+                                      (unsigned)((rest + kGT - 1) / kGT)),
+                                 dim3(128), 0, st, 1, n, j0, nb, j0 + nb + kNB, a),
+                      "getrf: trailing update launch");
     }
   }
   return check_launch("getrf blocked");
