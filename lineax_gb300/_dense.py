@@ -72,18 +72,6 @@ def lu_solve(lu: torch.Tensor, piv: torch.Tensor, b: torch.Tensor, trans: int = 
 # -- Cholesky ---------------------------------------------------------------
 
 
-def _one_system_meta(n: int, nrhs: int, device):
-    meta = torch.tensor([n, nrhs], dtype=torch.int32)
-    offs = torch.zeros(2, dtype=torch.int64)
-    return (meta[0:1].to(device), meta[1:2].to(device), offs[0:1].to(device),
-            offs[1:2].to(device))
-
-
-# Largest order factored by the one-CTA kernel (in shared memory); larger
-# matrices use the multi-CTA lxgb_potrf_f64.
-POTRF_ONE_CTA_MAX = 160
-
-
 def gram(a: torch.Tensor, tall: bool) -> torch.Tensor:
     """AᵀA (tall) or AAᵀ (wide) of the row-major FP64 matrix a, full and
     symmetric (lxgb_syrk_f64)."""
@@ -104,13 +92,7 @@ def cho_factor(a: torch.Tensor, negate: bool = False) -> torch.Tensor:
         u.neg_()
     n = u.shape[0]
     info = torch.empty(1, dtype=torch.int32, device=u.device)
-    if n > POTRF_ONE_CTA_MAX:
-        # many CTAs (same bits as the one-CTA kernel)
-        _ffi.call("lxgb_potrf_f64", n, _ffi.ptr(u), n, _ffi.ptr(info), _stream(u))
-    else:
-        nvec, _, aoff, _ = _one_system_meta(n, 1, u.device)
-        _ffi.call("lxgb_potrf_ragged_f64", 1, n, _ffi.ptr(nvec), _ffi.ptr(aoff), _ffi.ptr(u),
-                  _ffi.ptr(info), _stream(u))
+    _ffi.call("lxgb_potrf_f64", n, _ffi.ptr(u), n, _ffi.ptr(info), _stream(u))
     # A failed factorisation is reported like jax: a NaN factor, which the
     # solve turns into RESULTS.singular.
     u.masked_fill_((info != 0).reshape(1, 1), float("nan"))

@@ -10,9 +10,9 @@
 // chain from its stored value in k order.
 //
 // lxgb_potrf_f64 factors one n×n SPD matrix (A = UᵀU, upper) right-looking
-// by 64-row block rows: the diagonal block by one CTA in shared memory, the
-// block row by a column-parallel substitution, the trailing matrix by the
-// SYRK update above.  Every element receives exactly the update chain of the
+// by 32-row block rows: the diagonal block and its block row in one sweep
+// (potrf_row_kernel), the update of the next block row, and beside that next
+// row the update of the rest.  Every element receives exactly the update chain of the
 // single-CTA factorisation (k ascending, scaling by the pivot reciprocal), so
 // both give the same bits.
 #include "common.cuh"
@@ -22,8 +22,15 @@ namespace lxgb {
 
 constexpr int kSyTile = 64;
 constexpr int kSyK = 16;
-constexpr int kPoNB = 64;       // block rows of the multi-CTA Cholesky
-constexpr int kPoCols = 128;    // columns per CTA of the block-row substitution
+constexpr int kPoNB = 32;       // block rows of the multi-CTA Cholesky
+// Columns per CTA of the block-row kernel: 32 G.  G = 2 above kPoWide trailing
+// columns, where the trailing update beside it wants the SMs (n = 1531: 24
+// instead of 48 of them); G = 1 below, where the block row's own time counts
+// (27 us against 31).  At n = 1531 both alone take 2.68 ms in all.
+constexpr int kPoWide = 1024;
+// Unused dynamic shared memory that a block-row CTA reserves, so that no CTA
+// of the trailing update running beside it (17 KB each) shares its SM.
+constexpr int kPoReserve = 190 * 1024;
 
 // Upper tile t (row-major over the triangle) of an nt×nt tile grid.
 __device__ __forceinline__ void upper_tile(int t, int nt, int& ti, int& tj) {
@@ -103,62 +110,206 @@ syrk_f64_kernel(int trans, int64_t n, int64_t k, const double* __restrict__ a, i
     }
 }
 
-// The diagonal block [j0, j0+nb)² factored by one CTA in shared memory.
-// info[0] records the first pivot that is not positive (global index + 1).
+// Block row [j0, j0+nb) of U: the diagonal block factored and U12 = U11⁻ᵀ A12
+// formed in the same sweep.  A CTA takes the diagonal block and 32 G columns
+// right of it; every CTA factors the block for itself.  Warp 0 runs the chain:
+// in step k it has row k of the block in registers, forms the pivot's square
+// root and reciprocal, scales the row, and after one barrier updates row k + 1
+// for itself.  Six other warps hold the remaining rows in registers (row i with
+// warp i mod 6, a lane per column of the block and one per column beside it),
+// scale row k of the CTA's columns and update their rows; the owners of rows
+// k + 1 and k + 2 pass on through shared memory what the next step reads.
+// (Warp 4 shares warp 0's sub-partition and stays out of its way.)  What
+// bounds it is warp 0's chain (square root, division, scaling, FMA: 1600
+// cycles a row).  Measured, n = 1531: 27 to 31 us a block row of 32; a block
+// row of 64 as a diagonal kernel (138 us) and a column-per-thread substitution
+// (149 us) before.  The whole factorisation 8.4 to 2.3 ms.
+// The operations on each element, and their order, are cta_potrf_upper's:
+// row k scaled by 1 / sqrt(a_kk), then one FMA per later row, k ascending.
+constexpr int kPoOwners = 6;
+constexpr int kPoRows = (kPoNB + kPoOwners - 1) / kPoOwners;
+
+template <int G>
 __global__ void __launch_bounds__(256)
-potrf_diag_kernel(int64_t n, double* __restrict__ a, int64_t lda, int64_t j0, int nb,
-                  int32_t* __restrict__ info) {
-  __shared__ double blk[kPoNB * (kPoNB + 1)];
-  const int ld = nb | 1;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    if (j >= i) blk[i * ld + j] = a[(j0 + i) * lda + j0 + j];
+potrf_row_kernel(int64_t n, double* __restrict__ a, int64_t lda, int64_t j0, int nb,
+                 int32_t* __restrict__ info) {
+  __shared__ double U[kPoNB][kPoNB + 1];   // finished rows of the block
+  __shared__ double D[2][kPoNB];           // row k of the block as warp 0 takes it, by parity
+  __shared__ double E[2][32 * G];          // row k beside it, not yet scaled
+  __shared__ double s_r[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t col = j0 + nb + (int64_t)blockIdx.x * (32 * G) + lane;  // and col + 32 h
+  const int uw = (warp < 4) ? warp - 1 : warp - 2;   // owner 0..5 (warp 0: -1)
+  const bool owner = warp != 0 && warp != 4;
+  pdl_wait();
+  // everything before is finished: the rest of the previous trailing update
+  // may start beside this kernel
+  pdl_trigger();
+  double g[kPoRows], e[kPoRows][G];        // rows uw + 6 q: block, columns beside it
+  double v = 0.0;
+  if (owner) {
+#pragma unroll
+    for (int q = 0; q < kPoRows; ++q) {
+      const int i = uw + kPoOwners * q;
+      g[q] = (i < nb && lane >= i && lane < nb) ? a[(j0 + i) * lda + j0 + lane] : 0.0;
+#pragma unroll
+      for (int h = 0; h < G; ++h)
+        e[q][h] = (i < nb && col + 32 * h < n) ? a[(j0 + i) * lda + col + 32 * h] : 0.0;
+    }
+    if (uw == 0) {
+#pragma unroll
+      for (int h = 0; h < G; ++h) E[0][lane + 32 * h] = e[0][h];
+    }
+    if (uw == 1) D[1][lane] = g[0];
+  } else if (warp == 0) {
+    v = (lane < nb) ? a[j0 * lda + j0 + lane] : 0.0;
   }
-  __syncthreads();
-  const int rc = cta_potrf_upper<double, 16>(blk, ld, nb);
-  __syncthreads();
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    if (j >= i) a[(j0 + i) * lda + j0 + j] = blk[i * ld + j];
+  int bad = 0;
+  for (int k = 0; k < nb; ++k) {
+    const int par = k & 1;
+    double u = 0.0;
+    if (warp == 0) {
+      const double akk = __shfl_sync(0xffffffffu, v, k);
+      if (!(akk > 0.0) && bad == 0) bad = k + 1;
+      const double d = sqrt(akk);
+      const double r = 1.0 / d;
+      u = (lane > k) ? v * r : (lane == k ? d : 0.0);
+      U[k][lane] = u;
+      if (lane == 0) s_r[par] = r;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const double uk1 = __shfl_sync(0xffffffffu, u, min(k + 1, kPoNB - 1));
+      v = fma(-uk1, u, D[par ^ 1][lane]);              // row k + 1
+    } else if (owner) {
+      const double ul = U[k][lane];
+      double x[G];
+#pragma unroll
+      for (int h = 0; h < G; ++h) {
+        x[h] = E[par][lane + 32 * h] * s_r[par];
+        if (uw == k % kPoOwners && col + 32 * h < n) a[(j0 + k) * lda + col + 32 * h] = x[h];
+      }
+#pragma unroll
+      for (int q = 0; q < kPoRows; ++q) {
+        const int i = uw + kPoOwners * q;
+        if (i > k && i < nb) {                         // uniform over the warp
+          const double ui = U[k][i];
+#pragma unroll
+          for (int h = 0; h < G; ++h) {
+            e[q][h] = fma(-ui, x[h], e[q][h]);
+            if (i == k + 1) E[par ^ 1][lane + 32 * h] = e[q][h];
+          }
+          if (i != k + 1) {
+            g[q] = fma(-ui, ul, g[q]);
+          }
+          if (i == k + 2) D[par][lane] = g[q];
+        }
+      }
+    }
   }
-  if (threadIdx.x == 0 && rc != 0 && info[0] == 0) info[0] = (int32_t)(j0 + rc);
+  if (blockIdx.x == 0) {
+    __syncthreads();
+    for (int t = tid; t < nb * nb; t += 256) {
+      const int i = t / nb, j = t % nb;
+      if (j >= i) a[(j0 + i) * lda + j0 + j] = U[i][j];
+    }
+    if (tid == 0 && bad != 0 && info[0] == 0) info[0] = (int32_t)(j0 + bad);
+  }
 }
 
-// Block row [j0, j0+nb) × columns [j1, n): U12 = U11⁻ᵀ A12 by substitution,
-// one column per thread, in the order of the single-CTA factorisation: row p
-// scaled by 1/U11[p][p], then rows q > p updated by an FMA.
-struct PoRowSmem {
-  double u[kPoNB][kPoNB + 1];
-  double rinv[kPoNB];
-  double x[kPoNB][kPoCols + 1];
-};
+// The next block row's share of the trailing update, ahead of the rest: rows
+// [s, s+32), s = j0 + nb, columns j >= i, a_ij -= sum_k u_ki u_kj.  32x8 tile
+// per CTA (the critical path: as many SMs as there are tiles).
+__global__ void __launch_bounds__(128)
+potrf_next_row_kernel(int64_t n, double* __restrict__ a, int64_t lda, int64_t j0, int nb) {
+  __shared__ double Ui[kPoNB][kPoNB + 1];
+  __shared__ double Uj[kPoNB][8];
+  const int64_t s = j0 + nb;
+  const int64_t c0 = s + (int64_t)blockIdx.x * 8;
+  const int tid = threadIdx.x;
+  const int tx = tid & 7, ty = tid >> 3;
+  const int64_t j = c0 + tx;
+  pdl_wait();
+  double acc[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int64_t i = s + ty + 16 * r;
+    acc[r] = (i < n && j < n && j >= i) ? a[i * lda + j] : 0.0;
+  }
+#pragma unroll
+  for (int e = tid; e < kPoNB * kPoNB; e += 128) {
+    const int k = e / kPoNB, i = e % kPoNB;
+    Ui[k][i] = (k < nb && s + i < n) ? a[(j0 + k) * lda + s + i] : 0.0;
+  }
+#pragma unroll
+  for (int e = tid; e < kPoNB * 8; e += 128) {
+    const int k = e / 8, c = e % 8;
+    Uj[k][c] = (k < nb && c0 + c < n) ? a[(j0 + k) * lda + c0 + c] : 0.0;
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int k = 0; k < nb; ++k) {
+    const double uj = Uj[k][tx];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) acc[r] = fma(-Ui[k][ty + 16 * r], uj, acc[r]);
+  }
+  pdl_trigger();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int64_t i = s + ty + 16 * r;
+    if (i < n && j < n && j >= i) a[i * lda + j] = acc[r];
+  }
+}
 
-__global__ void __launch_bounds__(kPoCols)
-potrf_blockrow_kernel(int64_t n, double* __restrict__ a, int64_t lda, int64_t j0, int nb,
-                      int64_t j1) {
-  extern __shared__ double po_smem[];
-  PoRowSmem& sm = *reinterpret_cast<PoRowSmem*>(po_smem);
-  auto& u = sm.u;
-  auto& rinv = sm.rinv;
-  auto& x = sm.x;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    u[i][j] = (j >= i) ? a[(j0 + i) * lda + j0 + j] : 0.0;
+// The rest of the trailing update: rows and columns from s = j0 + nb + 32 on,
+// upper 32x32 tiles, 2x4 outputs per thread.  Runs beside the next block row:
+// it reads at once what was finished before that kernel (through L2), touches
+// none of its elements, and waits for it only before it ends (as the LU's
+// trailing update does).
+__global__ void __launch_bounds__(128)
+potrf_trailing_kernel(int64_t n, double* a, int64_t lda, int64_t j0, int nb, int64_t s) {
+  __shared__ double Ui[kPoNB][kPoNB + 1];
+  __shared__ double Uj[kPoNB][kPoNB + 2];
+  const int nt = (int)((n - s + kPoNB - 1) / kPoNB);
+  int ti, tj;
+  upper_tile(blockIdx.x, nt, ti, tj);
+  const int64_t i0 = s + (int64_t)ti * kPoNB, c0 = s + (int64_t)tj * kPoNB;
+  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+  double acc[2][4];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t i = i0 + ty + 16 * r, j = c0 + tx + 8 * q;
+      acc[r][q] = (i < n && j < n && j >= i) ? __ldcg(a + i * lda + j) : 0.0;
+    }
+#pragma unroll
+  for (int e = tid; e < kPoNB * kPoNB; e += 128) {
+    const int k = e / kPoNB, i = e % kPoNB;
+    Ui[k][i] = (k < nb && i0 + i < n) ? __ldcg(a + (j0 + k) * lda + i0 + i) : 0.0;
+    Uj[k][i] = (k < nb && c0 + i < n) ? __ldcg(a + (j0 + k) * lda + c0 + i) : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x < nb) rinv[threadIdx.x] = 1.0 / u[threadIdx.x][threadIdx.x];
-  const int64_t col0 = j1 + (int64_t)blockIdx.x * kPoCols;
-  const int t = threadIdx.x;
-  const int64_t col = col0 + t;
-  for (int p = 0; p < nb; ++p) x[p][t] = (col < n) ? a[(j0 + p) * lda + col] : 0.0;
-  __syncthreads();
-  for (int p = 0; p < nb; ++p) {
-    const double xp = x[p][t] * rinv[p];
-    x[p][t] = xp;
-    for (int q = p + 1; q < nb; ++q) x[q][t] = fma(-u[p][q], xp, x[q][t]);
+#pragma unroll 8
+  for (int k = 0; k < nb; ++k) {
+    double ui[2], uj[4];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) ui[r] = Ui[k][ty + 16 * r];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) uj[q] = Uj[k][tx + 8 * q];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[r][q] = fma(-ui[r], uj[q], acc[r][q]);
   }
-  if (col < n)
-    for (int p = 0; p < nb; ++p) a[(j0 + p) * lda + col] = x[p][t];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t i = i0 + ty + 16 * r, j = c0 + tx + 8 * q;
+      if (i < n && j < n && j >= i) a[i * lda + j] = acc[r][q];
+    }
+  pdl_wait();
 }
 
 __global__ void zero_lower_kernel(int64_t n, double* __restrict__ a, int64_t lda) {
@@ -199,20 +350,33 @@ extern "C" int lxgb_potrf_f64(int64_t n, double* a, int64_t lda, int32_t* info, 
   set_info_kernel<<<1, 1, 0, st>>>(info);
   if (n == 0) return check_launch("potrf_f64");
   LXGB_REQUIRE(a && lda >= n, "potrf: null pointer or lda < n");
-  LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(potrf_blockrow_kernel),
-                                    (int)sizeof(PoRowSmem)),
-                "potrf: set smem");
+  for (const void* fn : {reinterpret_cast<const void*>(potrf_row_kernel<1>),
+                         reinterpret_cast<const void*>(potrf_row_kernel<2>)})
+    LXGB_CUDA_TRY(ensure_dynamic_smem(fn, kPoReserve), "potrf: set smem");
+  LXGB_REQUIRE(n < (1LL << 31) - 64, "potrf: n too large");
+  // per block row: the row itself, its update of the next row, and (beside the
+  // next row) of everything after that
   for (int64_t j0 = 0; j0 < n; j0 += kPoNB) {
     const int nb = (int)((n - j0 < kPoNB) ? (n - j0) : kPoNB);
-    const int64_t j1 = j0 + nb;
-    potrf_diag_kernel<<<1, 256, 0, st>>>(n, a, lda, j0, nb, info);
-    if (j1 < n) {
-      const int64_t cols = n - j1;
-      potrf_blockrow_kernel<<<(unsigned)((cols + kPoCols - 1) / kPoCols), kPoCols,
-                              sizeof(PoRowSmem), st>>>(n, a, lda, j0, nb, j1);
-      int rc = syrk_launch(0, cols, nb, a + j0 * lda + j1, lda, 1, a + j1 * lda + j1, lda, 0, st);
-      if (rc) return rc;
+    const int64_t rest = n - j0 - nb;
+    const int cols = rest > kPoWide ? 64 : 32;
+    const int64_t ctas = rest > 0 ? (rest + cols - 1) / cols : 1;
+    LXGB_CUDA_TRY(launch_pdl(cols == 64 ? potrf_row_kernel<2> : potrf_row_kernel<1>,
+                             dim3((unsigned)ctas), dim3(256), kPoReserve, st, 1, n, a, lda, j0, nb,
+                             info),
+                  "potrf: block row launch");
+    // the previous row's trailing update, released once this row's CTAs run
+    if (j0 > 0 && rest > 0) {
+      const int64_t nt = (rest + kPoNB - 1) / kPoNB;
+      LXGB_REQUIRE(nt * (nt + 1) / 2 < (1LL << 31), "potrf: n too large");
+      LXGB_CUDA_TRY(launch_pdl(potrf_trailing_kernel, dim3((unsigned)(nt * (nt + 1) / 2)),
+                               dim3(128), 0, st, 1, n, a, lda, j0 - kPoNB, (int)kPoNB, j0 + nb),
+                    "potrf: trailing update launch");
     }
+    if (rest > 0)
+      LXGB_CUDA_TRY(launch_pdl(potrf_next_row_kernel, dim3((unsigned)((rest + 7) / 8)), dim3(128),
+                               0, st, 1, n, a, lda, j0, nb),
+                    "potrf: next row update launch");
   }
   const int64_t g = (n < 4096) ? n : 4096;
   zero_lower_kernel<<<(unsigned)g, 256, 0, st>>>(n, a, lda);

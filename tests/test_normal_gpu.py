@@ -171,3 +171,19 @@ def test_normal_cg_with_preconditioner(dev):
         assert sol.result == lx.RESULTS.successful
         x_ls = np.linalg.lstsq(a, b, rcond=None)[0]
         np.testing.assert_allclose(sol.value.cpu().numpy(), x_ls, rtol=1e-7, atol=1e-9)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 65, 97, 1100, 1151])
+def test_potrf_block_edges(dev, n):
+    """Edges of the 32-row blocks and of both block-row widths: the bits of
+    the one-CTA factorisation, zeros below the diagonal."""
+    rng = np.random.default_rng(n)
+    a = spd(rng, n)
+    u = _dense.cho_factor(t(a, dev))
+    u_one = t(a, dev)
+    meta = torch.tensor([n], dtype=torch.int32, device=dev)
+    off = torch.zeros(1, dtype=torch.int64, device=dev)
+    info = torch.empty(1, dtype=torch.int32, device=dev)
+    _ffi.call("lxgb_potrf_ragged_f64", 1, n, _ffi.ptr(meta), _ffi.ptr(off), _ffi.ptr(u_one),
+              _ffi.ptr(info), _ffi.stream_handle(dev))
+    assert torch.equal(u, u_one)
