@@ -55,6 +55,12 @@ int sm_count();
 // calls cost microseconds of host time per launch).  Defined in status.cu.
 cudaError_t ensure_dynamic_smem(const void* fn, int bytes);
 
+// Whether a cluster of `c` CTAs of kernel `fn` (`threads` threads, `smem` bytes
+// of dynamic shared memory each) can be co-scheduled on the current device; the
+// kernel's limits are raised as needed.  Asked once per device and shape.
+// Defined in status.cu.
+bool cluster_fits(const void* fn, int c, int threads, size_t smem);
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -27,6 +27,7 @@
 #include <utility>
 
 #include "common.cuh"
+#include "qr64.cuh"
 #include "tc_gemm.cuh"
 
 namespace lxgb {
@@ -918,6 +919,8 @@ extern "C" int lxgb_geqrf_f64(int64_t m, int64_t n, const double* a, int32_t a_l
     copy_kernel<<<(unsigned)blocks, 256, 0, st>>>(cnt, a, h);
   }
   const int nn = (int)n;
+  const int rc = geqrf64_cluster(m, nn, h, tau, t, st);
+  if (rc >= 0) return rc;
   double* wbase = reinterpret_cast<double*>(reinterpret_cast<char*>(work) + 256);
   for (int j0 = 0; j0 < nn; j0 += kQrNB) {
     const int nb = min(kQrNB, nn - j0);
@@ -961,6 +964,8 @@ extern "C" int lxgb_ormqr_f64(int64_t m, int64_t n, const double* h, const doubl
     return LXGB_WORKSPACE_TOO_SMALL;
   }
   cudaStream_t st = as_stream(stream);
+  const int rc = ormqr64_cluster(m, (int)n, h, t, nrhs, c, trans, st);
+  if (rc >= 0) return rc;
   double* part = reinterpret_cast<double*>(reinterpret_cast<char*>(work) + 256);
   const int npan = (int)((n + kQrNB - 1) / kQrNB);
   for (int q = 0; q < npan; ++q) {

@@ -4,6 +4,7 @@
 
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 #include "common.cuh"
@@ -44,6 +45,38 @@ cudaError_t ensure_dynamic_smem(const void* fn, int bytes) {
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e == cudaSuccess) have = bytes;
   return e;
+}
+
+bool cluster_fits(const void* fn, int c, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, int, int, size_t>, bool> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(fn, dev, c, threads, smem);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                cudaSuccess &&
+            ensure_dynamic_smem(fn, (int)smem) == cudaSuccess;
+  if (ok) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)c);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int nclusters = 0;
+    ok = cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg) == cudaSuccess && nclusters >= 1;
+  }
+  if (!ok) cudaGetLastError();
+  known[key] = ok;
+  return ok;
 }
 
 }  // namespace lxgb

@@ -1,0 +1,53 @@
+"""GPU checks of the cluster Householder QR at the edges of its 16- and
+32-column blocks, its rows per CTA and the largest panel (8192 rows)."""
+
+import numpy as np
+import pytest
+import torch
+
+from lineax_gb300 import _dense
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+@pytest.mark.parametrize("m,n", [(2, 2), (16, 16), (17, 16), (33, 17), (64, 33), (200, 48),
+                                 (65, 65), (513, 49), (1025, 40), (2049, 33), (4100, 18),
+                                 (8192, 35), (8193, 18)])
+def test_q_transposed_a_is_r(dev, m, n):
+    """Qᵀ A = [R; 0] and Q (Qᵀ c) = c, with Q applied panel by panel: column
+    errors at most 20 n u ||a_j|| (n reflectors, each within a few u)."""
+    rng = np.random.default_rng(m + n)
+    a = torch.tensor(rng.standard_normal((m, n)), device=dev)
+    h, tau, t = _dense.geqrf(a)
+    qta = _dense.ormqr(h, tau, t, a.T.contiguous(), trans=True)      # rows: Qᵀ a_j
+    r = torch.triu(h[:, :n].T)                                       # R[i][j] = h[j][i]
+    want = torch.zeros(n, m, dtype=torch.float64, device=dev)
+    want[:, :n] = r.T
+    norms = a.norm(dim=0)
+    assert bool(((qta - want).norm(dim=1) <= 20 * n * U * norms).all())
+    c = torch.tensor(rng.standard_normal((3, m)), device=dev)
+    back = _dense.ormqr(h, tau, t, _dense.ormqr(h, tau, t, c, trans=True), trans=False)
+    assert bool(((back - c).norm(dim=1) <= 40 * n * U * c.norm(dim=1)).all())
+    # tau of unit-leading reflectors: tau ||v||² = 2
+    v = torch.tril(h.T, -1)
+    v[torch.arange(n), torch.arange(n)] = 1.0
+    live = tau != 0
+    assert bool(((tau * (v * v).sum(0) - 2).abs()[live] <= 100 * U).all())
+
+
+def test_qr_zero_columns_and_extreme_scales(dev):
+    """A zero column (tau = 0, nothing changed) and columns whose squares
+    overflow or underflow next to the others (the hypot path)."""
+    rng = np.random.default_rng(1)
+    a = rng.standard_normal((300, 40))
+    a[:, 7] = 0.0
+    scale = np.ones(40)
+    scale[20:] = 1e140
+    a = torch.tensor(a * scale, device=dev)
+    h, tau, t = _dense.geqrf(a)
+    assert bool(torch.isfinite(h).all())
+    qta = _dense.ormqr(h, tau, t, a.T.contiguous(), trans=True)
+    r = torch.triu(h[:, :40].T)
+    err = (qta[:, :40].T - r).abs().amax(0)
+    assert bool((err <= 20 * 40 * U * a.norm(dim=0)).all())
