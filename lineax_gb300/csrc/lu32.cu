@@ -219,43 +219,57 @@ panel_getf2_cluster_kernel(int n, int j0, int nb, int rows_per_cta, float* __res
   }
 }
 
-// The same panel factorisation with every panel row held in the registers
-// of one thread (a CTA owns up to 512 rows, a cluster up to 16 CTAs): the
-// rank-1 update of a column is 63 independent FMAs per thread instead of a
-// loop over shared memory.  Per column each CTA publishes, in a slot
-// double-buffered by column parity, its first max |a| together with that
-// row (and row kk, from its owner); after the column's single cluster
-// barrier every CTA reduces the candidates in the same order, copies the
-// winning row through distributed shared memory, and the owner of the pivot
-// row takes row kk.  The global first max is also its CTA's first max, so the
-// published row is the pivot row.  Same arithmetic and pivot choice (first
-// row of max |a|, NaN never chosen) as the shared-memory kernels.
+// The same panel factorisation with every panel row held in the registers of
+// one thread (a CTA owns up to 512 rows, a cluster up to 16 CTAs).
+//  * Rows never move: an interchange swaps the two rows' labels, and each
+//    thread writes its row where its label says at the end.
+//  * The columns left in a row are kept shifted: element 0 is the current
+//    column, and the rank-1 update stores r[j-1] = r[j] - l prow[j].  One loop
+//    body then serves all 64 columns (about 200 instructions; unrolled by
+//    column the panel ran 60 times as much code once and waited for it), the
+//    multipliers go to shared memory.
+//  * Per column: the CTA's first max |a| by integer reductions, (key, label)
+//    stored into every CTA's slots, the candidate's row laid out locally; one
+//    cluster barrier; every warp picks the same winner from its own slots and
+//    the winning row is read from the winner's CTA.  Slots and rows alternate
+//    with the column's parity.
+// Same arithmetic and pivot choice (first row of max |a|, NaN never chosen) as
+// the shared-memory kernels.  Measured at m = 8192: see launch_panel_cluster_reg.
 constexpr int kRegPanelThreads = 512;
+constexpr int kRegHistLd = kRegPanelThreads;
+constexpr size_t kRegPanelSmem = (size_t)kLu32NB * kRegHistLd * sizeof(float);
 
-// CLUSTER = false: a one-CTA panel (m <= 512) without the cluster barrier's
-// cluster-scope release/acquire; the exchange slots are then local.
+// CLUSTER = false: a one-CTA panel (m <= 512) without cluster barriers.
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kRegPanelThreads, 1)
 panel_getf2_cluster_reg_kernel(int n, int j0, int nb, int rows_per_cta, float* __restrict__ a,
                                int32_t* __restrict__ piv, int32_t* __restrict__ info) {
-  __shared__ float cand_v[2];
-  __shared__ int cand_i[2];
-  __shared__ __align__(16) float xbuf[2][2][kLu32NB];  // [parity][pivot row, row kk]
-  __shared__ __align__(16) float rowp[kLu32NB];
-  __shared__ float s_wv[kRegPanelThreads / 32];
-  __shared__ int s_wi[kRegPanelThreads / 32];
-  __shared__ int s_p;
+  extern __shared__ __align__(16) float hist[];  // [column][thread]: multipliers
+  __shared__ __align__(8) uint2 cand[2][kRegPanelThreads / 32];  // (key, label) by warp
+  __shared__ __align__(8) uint2 slot[2][kPanelCluMax];           // and by CTA
+  __shared__ __align__(16) float mine[2][kLu32NB];               // this CTA's candidate row
+  __shared__ __align__(16) float prow[2][kLu32NB];               // the pivot row
+  __shared__ int s_owner;
   cg::cluster_group cluster = cg::this_cluster();
   const int ncta = CLUSTER ? (int)cluster.num_blocks() : 1;
   const int rank = CLUSTER ? (int)cluster.block_rank() : 0;
+  auto barrier = [&]() {
+    if (CLUSTER) cluster.sync();
+    else __syncthreads();
+  };
   // shared memory of CTA `rk` of the cluster (this CTA's own without one)
   auto remote = [&](auto* ptr, int rk) { return CLUSTER ? cluster.map_shared_rank(ptr, rk) : ptr; };
   const int m = n - j0;
   const int R = rows_per_cta;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int gi = rank * R + tid;  // panel row held by this thread
+  constexpr int kWarps = kRegPanelThreads / 32;
+  int gi = rank * R + tid;             // label of this thread's row
   const bool has_row = tid < R && gi < m;
+  bool active = has_row;               // not yet a pivot row
+  int done_at = nb;                    // columns of this row that are multipliers
   float r[kLu32NB];
+#pragma unroll
+  for (int j = 0; j < kLu32NB; ++j) r[j] = 0.0f;
   if (has_row) {
     const float* src = a + (int64_t)(j0 + gi) * n + j0;
     if (nb == kLu32NB) {
@@ -271,101 +285,110 @@ panel_getf2_cluster_reg_kernel(int n, int j0, int nb, int rows_per_cta, float* _
 #pragma unroll
       for (int j = 0; j < kLu32NB; ++j) r[j] = (j < nb) ? src[j] : 0.0f;
     }
-  } else {
-#pragma unroll
-    for (int j = 0; j < kLu32NB; ++j) r[j] = 0.0f;
   }
-#pragma unroll
-  for (int kk = 0; kk < kLu32NB; ++kk) {
-    if (kk < nb) {  // uniform over the cluster
-      const int par = kk & 1;
-      // this CTA's first max |a| in column kk, and its row published with it
-      float v = -1.0f;
-      int idx = INT_MAX;
-      if (has_row && gi >= kk) {
-        const float x = fabsf(r[kk]);
-        if (x > v) { v = x; idx = gi; }
-      }
-      warp_argmax_first_f(v, idx);
-      if (lane == 0) { s_wv[warp] = v; s_wi[warp] = idx; }
-      __syncthreads();
-      if (warp == 0) {
-        v = lane < kRegPanelThreads / 32 ? s_wv[lane] : -1.0f;
-        idx = lane < kRegPanelThreads / 32 ? s_wi[lane] : INT_MAX;
-        warp_argmax_first_f(v, idx);
-        if (lane == 0) { cand_v[par] = v; cand_i[par] = idx; }
-      }
-      __syncthreads();
-      if (has_row && gi == cand_i[par]) {
-#pragma unroll
-        for (int j = 0; j < kLu32NB; ++j) xbuf[par][0][j] = r[j];
-      }
-      if (has_row && gi == kk) {
-#pragma unroll
-        for (int j = 0; j < kLu32NB; ++j) xbuf[par][1][j] = r[j];
-      }
-      if (CLUSTER) {
-        cluster.sync();  // the one cluster barrier of this column
-      } else {
-        __syncthreads();
-      }
-      if (warp == 0) {
-        float cv = -1.0f;
-        int ci = INT_MAX;
-        if (lane < ncta) {
-          cv = *remote(&cand_v[par], lane);
-          ci = *remote(&cand_i[par], lane);
-        }
-        warp_argmax_first_f(cv, ci);
-        if (lane == 0) s_p = ci;  // INT_MAX: no candidate (all NaN), keep row kk
-      }
-      __syncthreads();
-      const bool none = s_p == INT_MAX;
-      const int p = none ? kk : s_p;
-      const int own_p = p / R, own_k = kk / R;
-      // pivot row: the winning CTA's published row (row kk itself when none)
-      if (tid < kLu32NB)
-        rowp[tid] = remote(&xbuf[par][none ? 1 : 0][0], none ? own_k : own_p)[tid];
-      __syncthreads();
-      const float akk = rowp[kk];
-      if (akk != 0.0f && p != kk) {
-        if (has_row && gi == kk) {
-#pragma unroll
-          for (int j = 0; j < kLu32NB; ++j) r[j] = rowp[j];
-        } else if (has_row && gi == p) {
-          const float* rk = remote(&xbuf[par][1][0], own_k);
-#pragma unroll
-          for (int j = 0; j < kLu32NB; ++j) r[j] = rk[j];
-        }
-      }
-      if (rank == 0 && tid == 0) {
-        piv[j0 + kk] = j0 + p;
-        if (akk == 0.0f && *info == 0) *info = j0 + kk + 1;
-      }
-      if (has_row && gi > kk) {
-        float l = r[kk];
-        if (akk != 0.0f) {
-          l *= 1.0f / akk;
-          r[kk] = l;
-        }
-#pragma unroll
-        for (int j = kk + 1; j < kLu32NB; ++j) r[j] = fmaf(-l, rowp[j], r[j]);
-      }
-    }
-  }
-  if (has_row) {
-    float* dst = a + (int64_t)(j0 + gi) * n + j0;
-    if (nb == kLu32NB) {
+  int bad = 0;
+  if (CLUSTER) cluster.sync();         // every CTA runs before any remote store
+#pragma unroll 1
+  for (int kk = 0; kk < nb; ++kk) {
+    const int par = kk & 1;
+    // this CTA's first max |a| in column kk (key 0: no candidate)
+    const unsigned bits = __float_as_uint(r[0]) & 0x7FFFFFFFu;
+    unsigned key = (active && bits <= 0x7F800000u) ? bits + 1u : 0u;
+    unsigned mk = __reduce_max_sync(0xffffffffu, key);
+    unsigned ml = __reduce_min_sync(0xffffffffu, (key == mk && key != 0u) ? (unsigned)gi : ~0u);
+    if (lane == 0) cand[par][warp] = make_uint2(mk, ml);
+    __syncthreads();
+    const uint2 w = lane < kWarps ? cand[par][lane] : make_uint2(0u, ~0u);
+    mk = __reduce_max_sync(0xffffffffu, w.x);
+    ml = __reduce_min_sync(0xffffffffu, w.x == mk ? w.y : ~0u);
+    if (warp == 0 && lane < ncta) *remote(&slot[par][rank], lane) = make_uint2(mk, ml);
+    if (active && (unsigned)gi == ml) {
 #pragma unroll
       for (int q = 0; q < kLu32NB / 4; ++q)
-        reinterpret_cast<float4*>(dst)[q] =
+        reinterpret_cast<float4*>(mine[par])[q] =
             make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-    } else {
+    }
+    barrier();                         // the one cluster barrier of this column
+    const uint2 s = lane < ncta ? slot[par][lane] : make_uint2(0u, ~0u);
+    mk = __reduce_max_sync(0xffffffffu, s.x);
+    ml = __reduce_min_sync(0xffffffffu, s.x == mk ? s.y : ~0u);
+    const bool none = mk == 0u;        // a column of NaNs: row kk stays
+    const int p = none ? kk : (int)ml;
+    int own = __ffs(__ballot_sync(0xffffffffu, s.x == mk && s.y == ml)) - 1;
+    if (none) {                        // uniform over the cluster
+      if (active && gi == kk) {
 #pragma unroll
-      for (int j = 0; j < kLu32NB; ++j)
-        if (j < nb) dst[j] = r[j];
+        for (int j = 0; j < kLu32NB; ++j) mine[par][j] = r[j];
+        for (int c = 0; c < ncta; ++c) *remote(&s_owner, c) = rank;
+      }
+      barrier();
+      own = s_owner;
+    }
+    if (warp == 0 && lane < kLu32NB / 4)
+      reinterpret_cast<float4*>(prow[par])[lane] =
+          reinterpret_cast<const float4*>(remote(&mine[par][0], own))[lane];
+    __syncthreads();
+    const float akk = prow[par][0];
+    if (rank == 0 && tid == 0) {
+      piv[j0 + kk] = j0 + p;
+      if (akk == 0.0f && bad == 0) bad = j0 + kk + 1;
+    }
+    if (akk != 0.0f && p != kk) {      // the interchange: labels only
+      if (gi == kk) gi = p;
+      else if (gi == p) gi = kk;
+    }
+    if (active && gi == kk) {
+      // row kk of U (written below from the pivot row; a zero pivot leaves row
+      // kk where it is, and its thread writes its own row)
+      active = false;
+      done_at = kk;
+      if (akk == 0.0f)
+#pragma unroll
+        for (int j = 0; j < kLu32NB; ++j)
+          if (kk + j < nb) a[(int64_t)(j0 + kk) * n + j0 + kk + j] = r[j];
+    }
+    if (akk != 0.0f && rank == 0 && warp >= kWarps - 2) {
+      const int j = (warp - (kWarps - 2)) * 32 + lane;
+      if (kk + j < nb) a[(int64_t)(j0 + kk) * n + j0 + kk + j] = prow[par][j];
+    }
+    if (active) {
+      float l = r[0];
+      if (akk != 0.0f) l *= 1.0f / akk;
+      hist[kk * kRegHistLd + tid] = l;
+      const float4* pr = reinterpret_cast<const float4*>(prow[par]);
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        if (16 * g < nb - kk) {        // the columns left, 16 at a time
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 u = pr[4 * g + q];
+            const int j = 16 * g + 4 * q;
+            if (j > 0) r[j - 1] = fmaf(-l, u.x, r[j]);
+            r[j] = fmaf(-l, u.y, r[j + 1]);
+            r[j + 1] = fmaf(-l, u.z, r[j + 2]);
+            r[j + 2] = fmaf(-l, u.w, r[j + 3]);
+          }
+        }
+      }
     }
   }
+  if (rank == 0 && tid == 0 && bad != 0 && *info == 0) *info = bad;
+  if (has_row) {
+    float* dst = a + (int64_t)(j0 + gi) * n + j0;
+    for (int c = 0; c < done_at; c += 4) {
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = (c + q < done_at) ? hist[(c + q) * kRegHistLd + tid] : 0.0f;
+      if (c + 3 < done_at && (n & 3) == 0 && (j0 & 3) == 0) {
+        *reinterpret_cast<float4*>(dst + c) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (c + q < done_at) dst[c + q] = v[q];
+      }
+    }
+  }
+  if (CLUSTER) cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // Cluster geometry for an m-row panel: 0 when it does not fit (or the device
@@ -417,38 +440,6 @@ static bool panel_cluster_fits(int c, size_t smem) {
   return ok;
 }
 
-static bool reg_cluster_fits(int c) {
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, bool> known;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
-  std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_pair(dev, c);
-  auto it = known.find(key);
-  if (it != known.end()) return it->second;
-  bool ok = cudaFuncSetAttribute(panel_getf2_cluster_reg_kernel<true>,
-                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  if (ok) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)c);
-    cfg.blockDim = dim3(kRegPanelThreads);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)c;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    ok = cudaOccupancyMaxActiveClusters(&nclusters, panel_getf2_cluster_reg_kernel<true>, &cfg) ==
-             cudaSuccess &&
-         nclusters >= 1;
-  }
-  if (!ok) cudaGetLastError();
-  known[key] = ok;
-  return ok;
-}
-
 // Register-resident panel when every row fits one thread of a <=16-CTA
 // cluster; 0 on launch, -1 when the caller must use another kernel.
 static int launch_panel_cluster_reg(int n, int j0, int nb, float* a, int32_t* piv, int32_t* info,
@@ -459,14 +450,20 @@ static int launch_panel_cluster_reg(int n, int j0, int nb, float* a, int32_t* pi
   if (c > kPanelCluMax) return -1;
   const int r = (m + c - 1) / c;
   if (c == 1) {
-    panel_getf2_cluster_reg_kernel<false><<<1, kRegPanelThreads, 0, st>>>(n, j0, nb, r, a, piv,
-                                                                          info);
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(panel_getf2_cluster_reg_kernel<false>),
+                            (int)kRegPanelSmem) != cudaSuccess)
+      return -1;
+    panel_getf2_cluster_reg_kernel<false><<<1, kRegPanelThreads, kRegPanelSmem, st>>>(
+        n, j0, nb, r, a, piv, info);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
-  if (!reg_cluster_fits(c)) return -1;
+  if (!cluster_fits(reinterpret_cast<const void*>(panel_getf2_cluster_reg_kernel<true>), c,
+                    kRegPanelThreads, kRegPanelSmem))
+    return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)c);
   cfg.blockDim = dim3(kRegPanelThreads);
+  cfg.dynamicSmemBytes = kRegPanelSmem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
