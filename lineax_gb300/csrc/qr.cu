@@ -512,6 +512,236 @@ qr_panel_cluster_f32_kernel(int64_t mm, int j0, int pe, int64_t rows_per_cta,
   cluster.sync();  // CTA 0 has finished reading the others' shared memory
 }
 
+// FP32 panel with its rows in registers: R <= 1056 rows per CTA, RR per thread
+// (row x in slot x / rowthreads), 32 columns each.  The kernel above reads two
+// and writes one shared-memory value per multiply-add, which bounds it (189 us a
+// panel at m = 16384); here a column costs 64 FMAs per row and one exchange.
+// The columns are kept rotated: element 0 is the current column a_k, the update
+// of the later ones shifts them down by one place, and the finished reflector
+// joins at the end.  One loop body serves every column, and the dots of a_k
+// with all 32 elements give the norm, the update's dots and VᵀV for T at once.
+// The dots are reduced by a transposing butterfly (each exchange halves the
+// columns a lane keeps), over warps in shared memory and over the cluster by
+// the control warp, a warp without rows that also forms the reflector, the
+// update's coefficients and (while the others update) the next column of T.
+// V also goes out as rows (vrows, 32 × m) and columns (vcols, m × 32) for the
+// trailing update's two GEMMs, with its zeros and ones.
+// Eleven warps and the control warp: three per SM sub-partition, 168 registers
+// per thread, so up to three rows of 32 columns fit (more threads with fewer
+// rows each measured slower: 109 us a panel of 900 rows per CTA with 15 warps
+// of two rows, 83 us of 1024 rows with 11 warps of three).
+constexpr int kQpThreads = 352;          // threads that hold rows, at most
+
+struct QpSmem {
+  float part[2][kQpThreads / 32][kQrNB];  // per-warp dots, by column parity
+  float pub[2][kQrNB];                    // this CTA's dots
+  float rowk[2][kQrNB];                   // row k's elements (rank 0)
+  __align__(16) float coef[2][kQrNB];     // update coefficients (0: finished columns)
+  float sc[2];                            // scal by parity
+  float Rm[kQrNB][kQrNB + 1];             // finished rows of R (rank 0)
+  float T[kQrNB][kQrNB + 1];
+};
+
+template <int RR>
+__global__ void __launch_bounds__(kQpThreads + 32, 1)
+qr_panel_rot_f32_kernel(int64_t mm, int j0, int nb, int R, float* __restrict__ h,
+                        float* __restrict__ tau, float* __restrict__ t_out,
+                        float* __restrict__ vrows, float* __restrict__ vcols) {
+  __shared__ QpSmem sm;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ncta = (int)cluster.num_blocks();
+  const int rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nrow = (int)blockDim.x - 32;           // threads that hold rows
+  const int nwarps = nrow >> 5;
+  const bool holder = tid < nrow;
+  const int x0 = rank * R;                         // first row, relative to j0
+  float r[RR][kQrNB];
+  pdl_wait();
+#pragma unroll
+  for (int rr = 0; rr < RR; ++rr) {
+    const int x = rr * nrow + tid;
+    const bool ok = holder && x < R && j0 + (int64_t)x0 + x < mm;
+#pragma unroll
+    for (int c = 0; c < kQrNB; ++c)
+      r[rr][c] = (ok && c < nb) ? h[(int64_t)(j0 + c) * mm + j0 + x0 + x] : 0.0f;
+  }
+  if (!holder)
+    for (int e = lane; e < kQrNB * (kQrNB + 1); e += 32) (&sm.T[0][0])[e] = 0.0f;
+  cluster.sync();
+#pragma unroll 1
+  for (int kk = 0; kk < kQrNB; ++kk) {
+    if (kk >= nb) {  // uniform over the cluster: a short panel's rotation ends in place
+#pragma unroll
+      for (int rr = 0; rr < RR; ++rr) {
+        const float f = r[rr][0];
+#pragma unroll
+        for (int c = 0; c + 1 < kQrNB; ++c) r[rr][c] = r[rr][c + 1];
+        r[rr][kQrNB - 1] = f;
+      }
+      continue;
+    }
+    const int par = kk & 1;
+    float v[RR];
+    if (holder) {
+      float s[kQrNB];
+#pragma unroll
+      for (int rr = 0; rr < RR; ++rr) {
+        v[rr] = (x0 + rr * nrow + tid > kk) ? r[rr][0] : 0.0f;
+#pragma unroll
+        for (int c = 0; c < kQrNB; ++c)
+          s[c] = (rr == 0) ? v[0] * r[0][c] : fmaf(v[rr], r[rr][c], s[c]);
+      }
+      if (x0 + tid == kk) {
+#pragma unroll
+        for (int c = 0; c < kQrNB; ++c) sm.rowk[par][c] = r[0][c];
+      }
+      // transposing butterfly: lane L ends with the warp's dot of element L
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int c = 0; c < o; ++c) {
+          const float keep = up ? s[c + o] : s[c];
+          const float send = up ? s[c] : s[c + o];
+          s[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      }
+      sm.part[par][warp][lane] = s[0];
+    }
+    __syncthreads();
+    if (!holder) {
+      float p[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int w = 0; w < kQpThreads / 32; ++w)
+        if (w < nwarps) p[w & 3] += sm.part[par][w][lane];
+      sm.pub[par][lane] = (p[0] + p[1]) + (p[2] + p[3]);
+    }
+    cluster.sync();                                // the one cluster barrier of the column
+    float d = 0.0f, tk = 0.0f;
+    if (!holder) {
+      float pv[kQrCluMax];
+#pragma unroll
+      for (int c = 0; c < kQrCluMax; ++c)
+        pv[c] = (c < ncta) ? cluster.map_shared_rank(&sm.pub[par][0], c)[lane] : 0.0f;
+      const float rk = cluster.map_shared_rank(&sm.rowk[par][0], 0)[lane];
+#pragma unroll
+      for (int o = 1; o < kQrCluMax; o *= 2)
+#pragma unroll
+        for (int c = 0; c + o < kQrCluMax; c += 2 * o) pv[c] += pv[c + o];
+      d = pv[0];
+      const float xn2 = __shfl_sync(0xffffffffu, d, 0);
+      const float alpha = __shfl_sync(0xffffffffu, rk, 0);
+      const float xnorm = sqrtf(xn2);
+      float scal = 1.0f, beta = alpha;
+      if (xnorm != 0.0f) {
+        beta = -copysignf(hypotf(alpha, xnorm), alpha);
+        tk = (beta - alpha) / beta;
+        scal = 1.0f / (alpha - beta);
+      }
+      // v_kᵀ a_c = a_c[k] + scal d_c (v_k[k] = 1); of a finished column: v_cᵀ v_k
+      d = fmaf(scal, d, rk);
+      const bool later = lane > 0 && lane < kQrNB - kk;   // element of column kk + lane
+      const float tw = tk * d;
+      sm.coef[par][lane] = later ? tw * scal : 0.0f;
+      if (rank == 0 && lane < kQrNB - kk)
+        sm.Rm[kk][kk + lane] = (lane == 0) ? beta : rk - tw;
+      if (lane == 0) {
+        sm.sc[par] = scal;
+        if (rank == 0) tau[j0 + kk] = tk;
+      }
+    }
+    __syncthreads();
+    if (!holder) {
+      // T[0:k, k] = -tau T[0:k, 0:k] (V[:, 0:k]ᵀ v_k), T[k][k] = tau; v_pᵀ v_k sits in
+      // lane 32 - kk + p
+      float acc = 0.0f;
+      for (int p = 0; p < kk; ++p) {
+        const float g = __shfl_sync(0xffffffffu, d, kQrNB - kk + p);
+        acc = fmaf(sm.T[lane][p], g, acc);
+      }
+      if (lane < kk) sm.T[lane][kk] = -tk * acc;
+      if (lane == kk) sm.T[kk][kk] = tk;
+      __syncwarp();
+    } else {
+      const float scal = sm.sc[par];
+      float first[RR];
+#pragma unroll
+      for (int rr = 0; rr < RR; ++rr) first[rr] = r[rr][0];
+#pragma unroll
+      for (int q = 0; q < kQrNB / 4; ++q) {
+        const float4 w = reinterpret_cast<const float4*>(sm.coef[par])[q];
+#pragma unroll
+        for (int rr = 0; rr < RR; ++rr) {
+          if (q > 0) r[rr][4 * q - 1] = fmaf(-w.x, v[rr], r[rr][4 * q]);
+          r[rr][4 * q + 0] = fmaf(-w.y, v[rr], r[rr][4 * q + 1]);
+          r[rr][4 * q + 1] = fmaf(-w.z, v[rr], r[rr][4 * q + 2]);
+          r[rr][4 * q + 2] = fmaf(-w.w, v[rr], r[rr][4 * q + 3]);
+        }
+      }
+#pragma unroll
+      for (int rr = 0; rr < RR; ++rr)
+        r[rr][kQrNB - 1] = (x0 + rr * nrow + tid > kk) ? v[rr] * scal : first[rr];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int rr = 0; rr < RR; ++rr) {
+    const int x = rr * nrow + tid;
+    const int gx = x0 + x;                         // row relative to j0
+    if (!(holder && x < R && j0 + (int64_t)gx < mm)) continue;
+    if (gx < kQrNB) {                              // rank 0: rows of R and of the unit triangle
+#pragma unroll
+      for (int c = 0; c < kQrNB; ++c) {
+        const float val = (gx <= c) ? sm.Rm[gx][c] : r[rr][c];
+        if (c < nb && (gx > c || gx < nb)) h[(int64_t)(j0 + c) * mm + j0 + gx] = val;
+        r[rr][c] = (gx < c) ? 0.0f : (gx == c ? (c < nb ? 1.0f : 0.0f) : r[rr][c]);
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < kQrNB; ++c)
+        if (c < nb) h[(int64_t)(j0 + c) * mm + j0 + gx] = r[rr][c];
+    }
+#pragma unroll
+    for (int c = 0; c < kQrNB; ++c) vrows[(int64_t)c * mm + j0 + gx] = (c < nb) ? r[rr][c] : 0.0f;
+    float4* vc = reinterpret_cast<float4*>(vcols + (int64_t)(j0 + gx) * kQrNB);
+#pragma unroll
+    for (int q = 0; q < kQrNB / 4; ++q)
+      vc[q] = make_float4(4 * q < nb ? r[rr][4 * q] : 0.0f, 4 * q + 1 < nb ? r[rr][4 * q + 1] : 0.0f,
+                          4 * q + 2 < nb ? r[rr][4 * q + 2] : 0.0f,
+                          4 * q + 3 < nb ? r[rr][4 * q + 3] : 0.0f);
+  }
+  if (rank == 0)
+    for (int e = tid; e < kQrNB * kQrNB; e += (int)blockDim.x)
+      t_out[e] = sm.T[e / kQrNB][e % kQrNB];
+  cluster.sync();  // no CTA leaves while another may still read its shared memory
+}
+
+// The panel at j0 on qr_panel_rot_f32_kernel: about 128 rows per CTA, at most
+// 16 CTAs (up to 16896 rows).  0 when launched, -1 when the panel is taller or
+// the cluster cannot be scheduled.
+static int launch_qr_panel_rot(int64_t mm, int j0, int nb, float* h, float* tau, float* t_out,
+                               float* vrows, float* vcols, cudaStream_t st) {
+  const int64_t rows = mm - j0;
+  int c = (int)((rows + 127) / 128 < kQrCluMax ? (rows + 127) / 128 : kQrCluMax);
+  int64_t R = (rows + c - 1) / c;
+  if (R > 3 * kQpThreads) return -1;
+  if (R < kQrNB) R = kQrNB;          // rank 0 owns the panel's triangle
+  c = (int)((rows + R - 1) / R);
+  const int slots = R > 2 * kQpThreads ? 3 : (R > kQpThreads ? 2 : 1);
+  const int threads = (int)(((R + slots - 1) / slots + 31) / 32 * 32) + 32;
+  auto fn = slots == 3 ? qr_panel_rot_f32_kernel<3>
+                       : (slots == 2 ? qr_panel_rot_f32_kernel<2> : qr_panel_rot_f32_kernel<1>);
+  if (!cluster_fits(reinterpret_cast<const void*>(fn), c, threads, 0)) return -1;
+  const cudaError_t e = launch_pdl(fn, dim3((unsigned)c), dim3((unsigned)threads), 0, st, c, mm,
+                                   j0, nb, (int)R, h, tau, t_out, vrows, vcols);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  return 0;
+}
+
 // The panel kernel a launch uses: the FP32 single-barrier variant (FUSED,
 // rows in shared memory), or qr_panel_cluster_kernel<T, SM>.
 template <typename T, bool SM, bool FUSED>
@@ -1121,15 +1351,17 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
   for (int j0 = 0; j0 < nn; j0 += kQrNB) {
     const int nb = min(kQrNB, nn - j0);
     float* Tp = t + (int64_t)(j0 / kQrNB) * kQrNB * kQrNB;
-    if (launch_qr_panel_cluster<float>(m, j0, j0 + nb, h, tau, Tp, st) != 0) {
-      set_last_error("%s: the panel's thread-block cluster cannot be scheduled", who);
-      return LXGB_NOT_SUPPORTED;
-    }
     const int n2 = nn - (j0 + nb);
+    if (launch_qr_panel_rot(m, j0, nb, h, tau, Tp, vrows, vcols, st) != 0) {
+      if (launch_qr_panel_cluster<float>(m, j0, j0 + nb, h, tau, Tp, st) != 0) {
+        set_last_error("%s: the panel's thread-block cluster cannot be scheduled", who);
+        return LXGB_NOT_SUPPORTED;
+      }
+      const int64_t tot = (int64_t)kQrNB * m;
+      qr32_make_v_kernel<<<(unsigned)((tot + 255) / 256 < 4096 ? (tot + 255) / 256 : 4096), 256,
+                           0, st>>>(m, j0, nb, h, vrows, vcols);
+    }
     if (n2 <= 0 && !q) continue;
-    const int64_t tot = (int64_t)kQrNB * m;
-    qr32_make_v_kernel<<<(unsigned)((tot + 255) / 256 < 4096 ? (tot + 255) / 256 : 4096), 256, 0,
-                         st>>>(m, j0, nb, h, vrows, vcols);
     if (n2 > 0) {
       int rc = apply(h + (int64_t)(j0 + nb) * m, n2, j0, nb, Tp);  // trailing rows of h
       if (rc) return rc;
