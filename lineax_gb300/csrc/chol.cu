@@ -156,41 +156,6 @@ struct MxSmem {
 };
 
 
-// Split W FP64 values, given as their two 32-bit words (x = low, y = high),
-// with one warp vote (see split_f64).  Only 32-bit integer operations run on
-// the common path.
-template <int W>
-__device__ __forceinline__ void splitw(const uint2 (&a)[W], float (&hi)[W], float (&lo)[W]) {
-  bool slow = false;
-#pragma unroll
-  for (int u = 0; u < W; ++u) {
-    const unsigned wl = a[u].x, wh = a[u].y;
-    const unsigned e = (wh >> 20) & 0x7FFu;
-    const unsigned sign = wh & 0x80000000u;
-    const unsigned mh = ((wh & 0xFFFFFu) << 3) | (wl >> 29);
-    const unsigned rem = wl & 0x1FFFFFFFu;
-    const int sh = __clz(rem | 1u) - 8;
-    const unsigned m = (sh >= 0) ? (rem << sh) : (rem >> (-sh));
-    const int ex = (int)e - 1052 - sh + 127;
-    const bool zero = ((wh << 1) | wl) == 0u;
-    hi[u] = zero ? __uint_as_float(sign) : __uint_as_float(sign | (((e - 1023u + 127u) & 0xFFu) << 23) | mh);
-    lo[u] = (rem == 0u) ? 0.0f : __uint_as_float(sign | (((unsigned)ex & 0xFFu) << 23) | (m & 0x7FFFFFu));
-    slow |= !zero && ((e < 949u) || (e > 1150u));
-  }
-  if (__any_sync(__activemask(), slow)) {
-#pragma unroll
-    for (int u = 0; u < W; ++u) {
-      const unsigned wl = a[u].x, wh = a[u].y;
-      const unsigned e = (wh >> 20) & 0x7FFu;
-      if (((wh << 1) | wl) != 0u && ((e < 949u) || (e > 1150u))) {
-        const double d = __hiloint2double((int)wh, (int)wl);
-        hi[u] = __double2float_rz(d);
-        lo[u] = __double2float_rn(d - (double)hi[u]);
-      }
-    }
-  }
-}
-
 // FP32 copy (the hi part of split_f64) of the upper triangle of the row-major
 // n×n FP64 matrix A into F (row stride ld).  A warp walks 256-column chunks of
 // its rows (j >= i); the next chunk's eight loads per lane are issued before
