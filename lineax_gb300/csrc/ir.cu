@@ -13,15 +13,16 @@
 //     product and residual of the refinement at a fraction of the FP64-pipe
 //     cost.
 //
-// The products share one kernel: a CTA owns 16 rows and 16 right-hand sides;
-// its eight warps each keep 4 rows x 8 right-hand sides of accumulators while
-// the lanes walk the columns, then reduce across lanes.  No cross-CTA
-// reduction: results are bitwise reproducible.
+// Sums are formed in a fixed order: results are bitwise reproducible.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "df.cuh"
 #include "tc_gemm.cuh"
 
 namespace lxgb {
+
+namespace cg = cooperative_groups;
 
 constexpr int kInvNB = 64;     // diagonal block size of the inversion
 constexpr int kInvCols = 128;  // columns per CTA in the diagonal-block solves
@@ -184,33 +185,17 @@ inv_diag_kernel(int n, int j0, int nb, const float* __restrict__ lu, float* __re
 }
 
 // ---------------------------------------------------------------------------
-// Products.  MODE 0: FP32 products and sums (x rounded to FP32, no lo parts).
-// MODE 1: double-float, exact FP32 matrix.  MODE 2: double-float, matrix
-// hi + lo.  TRI 0 full; 1 lower (columns < the row block's end: the matrix
-// holds zeros above its diagonal); 2 upper (columns from the row block's
-// start).  OUT 0: (yh, yl) pair; 1: y64 = value; 2: y64 = b64 - value.
+// FP32 products (x rounded to FP32).  TRI 0 full; 1 lower (columns < the row
+// block's end: the matrix holds zeros above its diagonal); 2 upper (columns from
+// the row block's start).  OUT 0: yh; 1: y64 = value; 2: y64 = b64 - value.
+// A CTA owns 16 rows and 16 right-hand sides; its eight warps each keep 4 rows x
+// 8 right-hand sides of accumulators while the lanes walk the columns, then
+// reduce across lanes.
 // ---------------------------------------------------------------------------
-template <int MODE>
-__device__ __forceinline__ void acc_step(float& sh, float& sl, float m, float ml, float xh,
-                                         float xl) {
-  if (MODE == 0) {
-    sh = fmaf(m, xh, sh);
-  } else {
-    const float p = m * xh;
-    float e = fmaf(m, xh, -p);  // exact: m xh = p + e
-    e = fmaf(m, xl, e);
-    if (MODE == 2) e = fmaf(ml, xh, e);
-    float err;
-    two_sum(sh, p, err);
-    sl += err + e;
-  }
-}
-
-template <int MODE, int TRI, int OUT>
-__global__ void __launch_bounds__(256, MODE == 0 ? 2 : 1)
-gemv16_kernel(int m, int ncol, const float* __restrict__ Mh, const float* __restrict__ Ml,
-              int64_t ldm, int k, const float* __restrict__ xh, const float* __restrict__ xl,
-              int64_t ldx, float* __restrict__ yh, float* __restrict__ yl,
+template <int TRI, int OUT>
+__global__ void __launch_bounds__(256, 2)
+gemv16_kernel(int m, int ncol, const float* __restrict__ Mh, int64_t ldm, int k,
+              const float* __restrict__ xh, int64_t ldx, float* __restrict__ yh,
               double* __restrict__ y64, const double* __restrict__ b64, int64_t ldy) {
   const int nblk = (m + kGvRows - 1) / kGvRows;
   // Lower triangles: the heaviest row blocks (last) start first.
@@ -227,95 +212,299 @@ gemv16_kernel(int m, int ncol, const float* __restrict__ Mh, const float* __rest
   const float* mr[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) mr[r] = Mh + (int64_t)min(row0 + r, m - 1) * ldm;
-  const int64_t mlo = (MODE == 2) ? (Ml - Mh) : 0;  // lo matrix at the same offsets
   int xo[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) xo[q] = min(rhs0 + q, k - 1) * (int)ldx;
-  const int64_t xlo = (MODE >= 1) ? (xl - xh) : 0;
-  float ah[4][8], al[4][8];
+  float ah[4][8];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int q = 0; q < 8; ++q) ah[r][q] = al[r][q] = 0.0f;
-
-  // Double-float products are FP32-pipe bound with one CTA per SM: the next
-  // column's operands are loaded while the current one is multiplied.
-  float mv[4], mlv[4], xv[8], xlv[8];
-  auto load = [&](int c, float (&m_)[4], float (&ml_)[4], float (&x_)[8], float (&xl_)[8]) {
-    const bool ok = c < c_hi;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      m_[r] = ok ? __ldg(mr[r] + c) : 0.0f;
-      ml_[r] = (MODE == 2 && ok) ? __ldg(mr[r] + mlo + c) : 0.0f;
-    }
-    const float* xc = xh + c;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      x_[q] = ok ? __ldg(xc + xo[q]) : 0.0f;
-      xl_[q] = (MODE >= 1 && ok) ? __ldg(xc + xlo + xo[q]) : 0.0f;
-    }
-  };
-  load(c_lo + lane, mv, mlv, xv, xlv);
+    for (int q = 0; q < 8; ++q) ah[r][q] = 0.0f;
   for (int c = c_lo + lane; c < c_hi; c += 32) {
-    float nm[4], nml[4], nx[8], nxl[8];
-    if (MODE != 0) load(c + 32, nm, nml, nx, nxl);
+    float mv[4], xv[8];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) mv[r] = __ldg(mr[r] + c);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) xv[q] = __ldg(xh + c + xo[q]);
 #pragma unroll
     for (int q = 0; q < 8; ++q)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) acc_step<MODE>(ah[r][q], al[r][q], mv[r], mlv[r], xv[q], xlv[q]);
-    if (MODE != 0) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) { mv[r] = nm[r]; mlv[r] = nml[r]; }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { xv[q] = nx[q]; xlv[q] = nxl[q]; }
-    } else {
-      load(c + 32, mv, mlv, xv, xlv);
-    }
+      for (int r = 0; r < 4; ++r) ah[r][q] = fmaf(mv[r], xv[q], ah[r][q]);
   }
-
   // Butterfly reduction across the lanes (every lane ends with every sum).
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
+  for (int off = 16; off > 0; off >>= 1)
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float oh = __shfl_xor_sync(0xffffffffu, ah[r][q], off);
-        if (MODE == 0) {
-          ah[r][q] += oh;
-        } else {
-          const float ol = __shfl_xor_sync(0xffffffffu, al[r][q], off);
-          float err;
-          two_sum(ah[r][q], oh, err);
-          al[r][q] += ol + err;
-        }
-      }
-  }
+      for (int q = 0; q < 8; ++q) ah[r][q] += __shfl_xor_sync(0xffffffffu, ah[r][q], off);
   // Lane r*8 + q writes (row0 + r, rhs0 + q).
-  float oh = 0.0f, ol = 0.0f;
+  float oh = 0.0f;
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int q = 0; q < 8; ++q)
-      if (lane == r * 8 + q) {
-        oh = ah[r][q];
-        ol = al[r][q];
-      }
+      if (lane == r * 8 + q) oh = ah[r][q];
   const int row = row0 + (lane >> 3), rhs = rhs0 + (lane & 7);
   if (row >= m || rhs >= k) return;
   const int64_t o = (int64_t)rhs * ldy + row;
-  if (MODE >= 1) {
-    float e;
-    fast_two_sum(oh, ol, e);
-    ol = e;
-  }
   if (OUT == 0) {
     yh[o] = oh;
-    if (MODE >= 1) yl[o] = ol;
   } else {
-    const double v = (MODE >= 1) ? (double)oh + (double)ol : (double)oh;
+    const double v = (double)oh;
     y64[o] = (OUT == 2) ? b64[o] - v : v;
   }
+}
+
+// ---------------------------------------------------------------------------
+// Double-float products Y = T X, T exact FP32 or a hi + lo pair (LO), X a pair:
+// a CTA owns 32 rows x NR right-hand sides, a cluster of CTAs splits the columns.
+//
+// What bounds it is the FP32 pipe.  A multiply-add takes 10 operations (9
+// without lo): p = fl(a x), r = fl(s + p), and as in TwoSum z = r - s,
+// t = r - z, whose exact parts give s + p - r = (s - t) + (p - z); the
+// product's own rounding error joins the second part, (p - z) + (a x - p) =
+// a x - z, in one FMA.  (TwoProd and TwoSum apart take 12.)  The FMA's rounding
+// is 2^-24 of a term that is itself at most an ulp; measured against 128 bits,
+// the sums' errors are those of the 12-operation form.  The low-order terms
+// join by FMAs before the one addition to the second accumulator.
+// A thread keeps 4 rows x NR/4 right-hand sides; the operands are staged by
+// asynchronous copies, 64 columns at a time, and the eight warps take the
+// columns of a stage in pairs (8-byte loads from shared memory).  The warps' and
+// then the cluster's partial sums are added in a fixed order.
+// Measured, n = 8192, 16 right-hand sides: hi + lo matrix 396 us (one CTA of 16
+// rows per SM, loads and sums one column at a time: 877 us), triangles 186 us
+// (329): 57 % of the FP32 pipe's rate.
+// ---------------------------------------------------------------------------
+constexpr int kDfRows = 32;     // rows per CTA
+constexpr int kDfK = 64;        // columns per stage
+constexpr int kDfLd = kDfK + 4; // padded row: 16-byte aligned, conflict-free over 8 rows
+constexpr int kDfThreads = 256;
+
+template <bool LO>
+__device__ __forceinline__ void df_mac(float& s, float& sl, float a, float al, float x, float xl) {
+  const float r = __fadd_rn(s, __fmul_rn(a, x));  // not to be contracted to an FMA
+  const float z = r - s;
+  const float t = r - z;
+  float e = (s - t) + fmaf(a, x, -z);
+  e = fmaf(a, xl, e);
+  if (LO) e = fmaf(al, x, e);
+  s = r;
+  sl += e;
+}
+
+// `bytes` of the 4 VEC bytes at src (the rest zero) into shared memory.
+template <int VEC>
+__device__ __forceinline__ void df_copy(float* dst, const float* src, int bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (VEC == 4)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes)
+                 : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes)
+                 : "memory");
+}
+
+template <int NR, bool LO>
+constexpr size_t df_stage_floats() {
+  return (size_t)((LO ? 2 : 1) * kDfRows + 2 * NR) * kDfLd;
+}
+template <int NR, bool LO>
+constexpr size_t df_smem() {
+  return 2 * df_stage_floats<NR, LO>() * sizeof(float);
+}
+
+template <int NR, bool LO, int TRI, int OUT, int VEC>
+__global__ void __launch_bounds__(kDfThreads, 2)
+gemm_df_kernel(int m, int ncol, const float* __restrict__ Mh, const float* __restrict__ Ml,
+               int64_t ldm, int k, const float* __restrict__ xh, const float* __restrict__ xl,
+               int64_t ldx, float* __restrict__ yh, float* __restrict__ yl,
+               double* __restrict__ y64, const double* __restrict__ b64, int64_t ldy) {
+  constexpr int J = NR / 4;                 // right-hand sides per thread
+  constexpr int kOut = kDfRows * NR;
+  extern __shared__ __align__(16) float df_dyn[];
+  __shared__ float2 pub[kOut];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int parts = (int)cluster.num_blocks();
+  const int part = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = lane & 7, cgp = lane >> 3;
+  const int nblk = (m + kDfRows - 1) / kDfRows;
+  const int bx = (int)(blockIdx.x / parts);
+  // lower triangles: the heaviest row blocks (last) start first
+  const int rb = (TRI == 1) ? (nblk - 1 - bx) : bx;
+  const int row0 = rb * kDfRows;
+  const int rhs0 = (int)blockIdx.y * NR;
+  int c_lo = 0, c_hi = ncol;
+  if (TRI == 1) c_hi = min(ncol, row0 + kDfRows);
+  if (TRI == 2) c_lo = row0;                // a multiple of 32: stages start aligned
+  const int chunks = (c_hi - c_lo + kDfK - 1) / kDfK;
+  const int ch0 = (int)((int64_t)chunks * part / parts);
+  const int ch1 = (int)((int64_t)chunks * (part + 1) / parts);
+  auto stage = [&](int buf) { return df_dyn + buf * df_stage_floats<NR, LO>(); };
+  auto load = [&](int ch, int buf) {
+    float* A = stage(buf);
+    float* X = A + (LO ? 2 : 1) * kDfRows * kDfLd;
+    constexpr int kPer = kDfK / VEC;        // copies per row
+    const int cb = c_lo + ch * kDfK;
+#pragma unroll
+    for (int e0 = 0; e0 < kDfRows * kPer; e0 += kDfThreads) {
+      const int e = e0 + tid;
+      const int r = e / kPer, c = (e % kPer) * VEC;
+      const int left = (row0 + r < m) ? min(VEC, max(0, c_hi - cb - c)) * 4 : 0;
+      const int64_t o = left ? (int64_t)(row0 + r) * ldm + cb + c : 0;
+      df_copy<VEC>(A + r * kDfLd + c, Mh + o, left);
+      if (LO) df_copy<VEC>(A + (kDfRows + r) * kDfLd + c, Ml + o, left);
+    }
+    for (int e = tid; e < NR * kPer; e += kDfThreads) {
+      const int r = e / kPer, c = (e % kPer) * VEC;
+      const int left = (rhs0 + r < k) ? min(VEC, max(0, c_hi - cb - c)) * 4 : 0;
+      const int64_t o = left ? (int64_t)(rhs0 + r) * ldx + cb + c : 0;
+      df_copy<VEC>(X + r * kDfLd + c, xh + o, left);
+      df_copy<VEC>(X + (NR + r) * kDfLd + c, xl + o, left);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float s[4][J], sl[4][J];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < J; ++j) s[i][j] = sl[i][j] = 0.0f;
+  if (ch0 < ch1) load(ch0, 0);
+  for (int ch = ch0; ch < ch1; ++ch) {
+    const int buf = (ch - ch0) & 1;
+    if (ch + 1 < ch1) {
+      load(ch + 1, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const float* A = stage(buf);
+    const float* X = A + (LO ? 2 : 1) * kDfRows * kDfLd;
+#pragma unroll
+    for (int u = 0; u < kDfK / 16; ++u) {
+      const int c = 2 * (warp + 8 * u);
+      float2 a[4], al[4], x[J], x2[J];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[i] = *reinterpret_cast<const float2*>(A + (8 * i + rg) * kDfLd + c);
+        al[i] = LO ? *reinterpret_cast<const float2*>(A + (kDfRows + 8 * i + rg) * kDfLd + c)
+                   : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        x[j] = *reinterpret_cast<const float2*>(X + (4 * j + cgp) * kDfLd + c);
+        x2[j] = *reinterpret_cast<const float2*>(X + (NR + 4 * j + cgp) * kDfLd + c);
+      }
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) df_mac<LO>(s[i][j], sl[i][j], a[i].x, al[i].x, x[j].x, x2[j].x);
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) df_mac<LO>(s[i][j], sl[i][j], a[i].y, al[i].y, x[j].y, x2[j].y);
+    }
+    __syncthreads();
+  }
+  // warps: output o = rhs * 32 + row (the staging buffers are free now)
+  float2* red = reinterpret_cast<float2*>(df_dyn);  // [8][kOut]
+  static_assert(8 * kOut * sizeof(float2) <= df_smem<NR, LO>(), "reduction fits the stages");
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+      red[warp * kOut + (4 * j + cgp) * kDfRows + 8 * i + rg] = make_float2(s[i][j], sl[i][j]);
+  __syncthreads();
+  for (int o = tid; o < kOut; o += kDfThreads) {
+    float2 v = red[o];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) {
+      const float2 u = red[w * kOut + o];
+      float err;
+      two_sum(v.x, u.x, err);
+      v.y += u.y + err;
+    }
+    pub[o] = v;
+  }
+  cluster.sync();
+  // the cluster: CTA `part` finishes its share of the outputs
+  const int share = kOut / parts;
+  for (int q = tid; q < share; q += kDfThreads) {
+    const int o = part * share + q;
+    float2 v = cluster.map_shared_rank(pub, 0)[o];
+    for (int c = 1; c < parts; ++c) {
+      const float2 u = cluster.map_shared_rank(pub, c)[o];
+      float err;
+      two_sum(v.x, u.x, err);
+      v.y += u.y + err;
+    }
+    const int row = row0 + o % kDfRows, rhs = rhs0 + o / kDfRows;
+    if (row < m && rhs < k) {
+      float e;
+      fast_two_sum(v.x, v.y, e);
+      const int64_t at = (int64_t)rhs * ldy + row;
+      if (OUT == 0) {
+        yh[at] = v.x;
+        yl[at] = e;
+      } else {
+        const double d = (double)v.x + (double)e;
+        y64[at] = (OUT == 2) ? b64[at] - d : d;
+      }
+    }
+  }
+  cluster.sync();  // no CTA leaves while another may still read its sums
+}
+
+template <int NR, bool LO, int TRI, int OUT, int VEC>
+static int launch_df_nr(int m, int ncol, const float* Mh, const float* Ml, int64_t ldm, int k,
+                        const float* xh, const float* xl, int64_t ldx, float* yh, float* yl,
+                        double* y64, const double* b64, int64_t ldy, cudaStream_t st) {
+  auto fn = gemm_df_kernel<NR, LO, TRI, OUT, VEC>;
+  const int nblk = (m + kDfRows - 1) / kDfRows;
+  // columns split so that about 1000 CTAs share the SMs evenly (256 row blocks
+  // alone would leave 48 SMs with two and 104 with one at a time)
+  const int parts = nblk <= 128 ? 8 : (nblk <= 256 ? 4 : 2);
+  constexpr size_t smem = df_smem<NR, LO>();
+  LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(fn), (int)smem), "gemm_df: smem");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(nblk * parts), (unsigned)((k + NR - 1) / NR));
+  cfg.blockDim = dim3(kDfThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)parts;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  LXGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, m, ncol, Mh, Ml, ldm, k, xh, xl, ldx, yh, yl, y64,
+                                   b64, ldy),
+                "gemm_df: launch");
+  return check_launch("gemm_df");
+}
+
+// 4, 8 or 16 right-hand sides per CTA; 16-byte copies when every row of the
+// operands starts on a 16-byte boundary.
+template <bool LO, int TRI, int OUT>
+static int launch_df(int m, int ncol, const float* Mh, const float* Ml, int64_t ldm, int k,
+                     const float* xh, const float* xl, int64_t ldx, float* yh, float* yl,
+                     double* y64, const double* b64, int64_t ldy, cudaStream_t st) {
+  if (m <= 0 || k <= 0) return LXGB_SUCCESSFUL;
+  const bool vec = (((uintptr_t)Mh | (uintptr_t)(LO ? Ml : Mh) | (uintptr_t)xh | (uintptr_t)xl) &
+                    15) == 0 &&
+                   (ldm & 3) == 0 && (ldx & 3) == 0;
+#define LXGB_DF(NR)                                                                              \
+  return vec ? launch_df_nr<NR, LO, TRI, OUT, 4>(m, ncol, Mh, Ml, ldm, k, xh, xl, ldx, yh, yl,   \
+                                                 y64, b64, ldy, st)                              \
+             : launch_df_nr<NR, LO, TRI, OUT, 1>(m, ncol, Mh, Ml, ldm, k, xh, xl, ldx, yh, yl,   \
+                                                 y64, b64, ldy, st)
+  if (k <= 4) LXGB_DF(4);
+  if (k <= 8) LXGB_DF(8);
+  LXGB_DF(16);
+#undef LXGB_DF
 }
 
 // Few right-hand sides (k <= 4): one warp per matrix row, lanes along the
@@ -458,14 +647,13 @@ split_matrix_kernel(int64_t rows, int64_t cols, const double* __restrict__ a, in
   }
 }
 
-template <int MODE, int TRI, int OUT>
-int launch_gemv16(int m, int ncol, const float* Mh, const float* Ml, int64_t ldm, int k,
-                  const float* xh, const float* xl, int64_t ldx, float* yh, float* yl,
-                  double* y64, const double* b64, int64_t ldy, cudaStream_t st) {
+template <int TRI, int OUT>
+int launch_gemv16(int m, int ncol, const float* Mh, int64_t ldm, int k, const float* xh,
+                  int64_t ldx, float* yh, double* y64, const double* b64, int64_t ldy,
+                  cudaStream_t st) {
   LXGB_REQUIRE((int64_t)k * ldx < ((int64_t)1 << 31), "gemv16: right-hand-side block above 2^31 entries");
   dim3 grid((unsigned)((m + kGvRows - 1) / kGvRows), (unsigned)((k + kGvRhs - 1) / kGvRhs));
-  gemv16_kernel<MODE, TRI, OUT><<<grid, 256, 0, st>>>(m, ncol, Mh, Ml, ldm, k, xh, xl, ldx, yh,
-                                                      yl, y64, b64, ldy);
+  gemv16_kernel<TRI, OUT><<<grid, 256, 0, st>>>(m, ncol, Mh, ldm, k, xh, ldx, yh, y64, b64, ldy);
   return check_launch("gemv16");
 }
 
@@ -605,16 +793,13 @@ extern "C" int lxgb_lu32_apply(int32_t n, int32_t nrhs, const float* linv, const
   split_rows_kernel<<<g, 256, 0, st>>>(nrhs, n, x, n, perm, zh, mode ? zl : nullptr, n);
   int rc;
   if (mode == 0) {
-    rc = launch_gemv16<0, 1, 0>(n, n, linv, nullptr, n, nrhs, zh, nullptr, n, th, nullptr, nullptr,
-                                nullptr, n, st);
-    if (!rc)
-      rc = launch_gemv16<0, 2, 1>(n, n, uinv, nullptr, n, nrhs, th, nullptr, n, nullptr, nullptr,
-                                  y, nullptr, n, st);
+    rc = launch_gemv16<1, 0>(n, n, linv, n, nrhs, zh, n, th, nullptr, nullptr, n, st);
+    if (!rc) rc = launch_gemv16<2, 1>(n, n, uinv, n, nrhs, th, n, nullptr, y, nullptr, n, st);
   } else {
-    rc = launch_gemv16<1, 1, 0>(n, n, linv, nullptr, n, nrhs, zh, zl, n, th, tl, nullptr, nullptr,
+    rc = launch_df<false, 1, 0>(n, n, linv, nullptr, n, nrhs, zh, zl, n, th, tl, nullptr, nullptr,
                                 n, st);
     if (!rc)
-      rc = launch_gemv16<1, 2, 1>(n, n, uinv, nullptr, n, nrhs, th, tl, n, nullptr, nullptr, y,
+      rc = launch_df<false, 2, 1>(n, n, uinv, nullptr, n, nrhs, th, tl, n, nullptr, nullptr, y,
                                   nullptr, n, st);
   }
   return rc;
@@ -647,16 +832,13 @@ extern "C" int lxgb_qr32_apply(int32_t n, int32_t nrhs, const float* qt, const f
   split_rows_kernel<<<g, 256, 0, st>>>(nrhs, n, x, n, nullptr, zh, mode ? zl : nullptr, n);
   int rc;
   if (mode == 0) {
-    rc = launch_gemv16<0, 0, 0>(n, n, qt, nullptr, n, nrhs, zh, nullptr, n, th, nullptr, nullptr,
-                                nullptr, n, st);
-    if (!rc)
-      rc = launch_gemv16<0, 2, 1>(n, n, rinv, nullptr, n, nrhs, th, nullptr, n, nullptr, nullptr,
-                                  y, nullptr, n, st);
+    rc = launch_gemv16<0, 0>(n, n, qt, n, nrhs, zh, n, th, nullptr, nullptr, n, st);
+    if (!rc) rc = launch_gemv16<2, 1>(n, n, rinv, n, nrhs, th, n, nullptr, y, nullptr, n, st);
   } else {
-    rc = launch_gemv16<1, 0, 0>(n, n, qt, nullptr, n, nrhs, zh, zl, n, th, tl, nullptr, nullptr,
+    rc = launch_df<false, 0, 0>(n, n, qt, nullptr, n, nrhs, zh, zl, n, th, tl, nullptr, nullptr,
                                 n, st);
     if (!rc)
-      rc = launch_gemv16<1, 2, 1>(n, n, rinv, nullptr, n, nrhs, th, tl, n, nullptr, nullptr, y,
+      rc = launch_df<false, 2, 1>(n, n, rinv, nullptr, n, nrhs, th, tl, n, nullptr, nullptr, y,
                                   nullptr, n, st);
   }
   return rc;
@@ -721,17 +903,15 @@ extern "C" int lxgb_gemv_df(int32_t m, int32_t n, const float* a_hi, const float
     return check_launch("gemv_df");
   }
   if (mode == 0)
-    return res ? launch_gemv16<0, 0, 2>(m, n, a_hi, nullptr, lda, nrhs, xh, nullptr, nn, nullptr,
-                                        nullptr, y, b, ldy, st)
-               : launch_gemv16<0, 0, 1>(m, n, a_hi, nullptr, lda, nrhs, xh, nullptr, nn, nullptr,
-                                        nullptr, y, nullptr, ldy, st);
+    return res ? launch_gemv16<0, 2>(m, n, a_hi, lda, nrhs, xh, nn, nullptr, y, b, ldy, st)
+               : launch_gemv16<0, 1>(m, n, a_hi, lda, nrhs, xh, nn, nullptr, y, nullptr, ldy, st);
   if (a_lo)
-    return res ? launch_gemv16<2, 0, 2>(m, n, a_hi, a_lo, lda, nrhs, xh, xl, nn, nullptr, nullptr,
-                                        y, b, ldy, st)
-               : launch_gemv16<2, 0, 1>(m, n, a_hi, a_lo, lda, nrhs, xh, xl, nn, nullptr, nullptr,
-                                        y, nullptr, ldy, st);
-  return res ? launch_gemv16<1, 0, 2>(m, n, a_hi, nullptr, lda, nrhs, xh, xl, nn, nullptr, nullptr,
+    return res ? launch_df<true, 0, 2>(m, n, a_hi, a_lo, lda, nrhs, xh, xl, nn, nullptr, nullptr,
+                                       y, b, ldy, st)
+               : launch_df<true, 0, 1>(m, n, a_hi, a_lo, lda, nrhs, xh, xl, nn, nullptr, nullptr,
+                                       y, nullptr, ldy, st);
+  return res ? launch_df<false, 0, 2>(m, n, a_hi, nullptr, lda, nrhs, xh, xl, nn, nullptr, nullptr,
                                       y, b, ldy, st)
-             : launch_gemv16<1, 0, 1>(m, n, a_hi, nullptr, lda, nrhs, xh, xl, nn, nullptr, nullptr,
+             : launch_df<false, 0, 1>(m, n, a_hi, nullptr, lda, nrhs, xh, xl, nn, nullptr, nullptr,
                                       y, nullptr, ldy, st);
 }
