@@ -15,6 +15,7 @@
 //
 // Sums are formed in a fixed order: results are bitwise reproducible.
 #include <cooperative_groups.h>
+#include <cuda_bf16.h>
 
 #include "common.cuh"
 #include "df.cuh"
@@ -25,7 +26,6 @@ namespace lxgb {
 namespace cg = cooperative_groups;
 
 constexpr int kInvNB = 64;     // diagonal block size of the inversion
-constexpr int kInvCols = 128;  // columns per CTA in the diagonal-block solves
 constexpr int kGvRows = 16;    // rows per CTA of the products
 constexpr int kGvRhs = 16;     // right-hand sides per CTA of the products
 constexpr int kPermMaxN = 25600;
@@ -111,77 +111,241 @@ __global__ void set_identity_f32_kernel(int n, float* __restrict__ w) {
     for (int c = threadIdx.x; c < n; c += blockDim.x) w[(int64_t)r * n + c] = (r == c) ? 1.0f : 0.0f;
 }
 
-// X = T_jj^{-1} W_j on rows [j0, j0+nb) of w and columns [c_begin, c_end):
-// T_jj the unit-lower (LOWER) or upper diagonal block of the factor.  X goes
-// back into w and, transposed (column c - c_begin, 64 entries, zero padded),
-// into xt: the K-major operand of the following tensor-core update.
-template <bool LOWER>
-__global__ void __launch_bounds__(kInvCols)
-inv_diag_kernel(int n, int j0, int nb, const float* __restrict__ lu, float* __restrict__ w,
-                int c_begin, int c_end, float* __restrict__ xt) {
-  // Tt[k][i] = T[i][k]: for a fixed k the multipliers of all rows i are
-  // contiguous (16-byte broadcast loads).  Padding rows/columns past nb hold
-  // the identity, so the fully unrolled substitution needs no bounds.
-  __shared__ __align__(16) float Tt[kInvNB][kInvNB + 4];
-  __shared__ float X[kInvNB][kInvCols + 1];
-#pragma unroll 16
-  for (int u = 0; u < kInvNB * kInvNB / kInvCols; ++u) {
-    const int e = threadIdx.x + u * kInvCols;
-    const int i = e / kInvNB, k = e % kInvNB;
-    Tt[k][i] = (i < nb && k < nb) ? lu[(int64_t)(j0 + i) * n + j0 + k] : (i == k ? 1.0f : 0.0f);
-  }
-  const int t = threadIdx.x;
-  const int cbase = c_begin + blockIdx.x * kInvCols;
-  const int c = cbase + t;
-  // Each thread substitutes its own column, held in registers.
-  float x[kInvNB];
-#pragma unroll
-  for (int i = 0; i < kInvNB; ++i)
-    x[i] = (i < nb && c < c_end) ? w[(int64_t)(j0 + i) * n + c] : 0.0f;
-  __syncthreads();
-  if (LOWER) {
-#pragma unroll
-    for (int k = 0; k < kInvNB; ++k) {
-      const float xk = x[k];
-#pragma unroll
-      for (int i4 = (k + 1) / 4; i4 < kInvNB / 4; ++i4) {
-        const float4 tq = *reinterpret_cast<const float4*>(&Tt[k][4 * i4]);
-        if (4 * i4 + 0 > k) x[4 * i4 + 0] = fmaf(-tq.x, xk, x[4 * i4 + 0]);
-        if (4 * i4 + 1 > k) x[4 * i4 + 1] = fmaf(-tq.y, xk, x[4 * i4 + 1]);
-        if (4 * i4 + 2 > k) x[4 * i4 + 2] = fmaf(-tq.z, xk, x[4 * i4 + 2]);
-        if (4 * i4 + 3 > k) x[4 * i4 + 3] = fmaf(-tq.w, xk, x[4 * i4 + 3]);
-      }
-    }
+// One block row of the LU or of a triangular inversion, everything between the
+// panel (or the previous update) and the tensor-core update in one launch:
+//  * strips of 64 columns: the panel's row interchanges (KIND 0), then
+//    X = T_jj^{-1} W_j on rows [j0, j0+nb) of w — T_jj the unit-lower (KIND 0,
+//    1) or upper (KIND 2) diagonal block of the factor, one column per thread in
+//    registers — written back in place and, transposed (64 entries per column,
+//    zero padded), as the K-major operand of the update: FP32 (PREC 0), its
+//    TF32-exact hi and lo parts (PREC 1) or BF16 (PREC 2).  KIND 0 also has
+//    strips left of the panel, which only take the interchanges;
+//  * further CTAs: the other operand (the panel's columns, na rows of `a_src`)
+//    split or converted the same way (PREC 1 and 2), 64 rows each.
+// The rows that the interchanges touch (the panel's 64 and up to 64 others) are
+// loaded at once into shared memory and swapped there.  Bound by latency: two
+// waits for device memory, 64 dependent swaps and 64 dependent substitution
+// steps.  Measured per panel at n = 8192: 15 us (LU), 10 and 19 (lower and upper
+// inversion, the latter with 64 divisions in its chain); as separate launches —
+// one thread per column swapping in global memory, the substitution, two splits
+// — 37 + 19 + 8 (LU) and 19 + 8 (inversions).
+constexpr int kBrCols = 64;
+constexpr int kBrThreads = 128;
+constexpr int kBrT = 16;
+constexpr int kBrLoads = kInvNB * kInvNB / kBrThreads;
+constexpr int kBrLd = kBrCols + 1;
+
+struct BlockRowArgs {
+  int n, j0, nb;
+  const float* lu;      // holds T_jj at (j0, j0)
+  float* w;             // target matrix (row stride n)
+  const int32_t* piv;   // KIND 0
+  int c_begin, c_end;   // columns solved
+  int strips, left;     // strips in all; of these left of the panel (KIND 0)
+  void *b0, *b1;        // operand from X: FP32 / hi, lo / BF16
+  const float* a_src;   // the other operand, row stride n
+  int na;
+  void *a0, *a1;
+};
+
+template <int PREC>
+__device__ __forceinline__ void br_store(void* p0, void* p1, int64_t at, float v) {
+  if (PREC == 0) {
+    reinterpret_cast<float*>(p0)[at] = v;
+  } else if (PREC == 1) {
+    const float h = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
+    reinterpret_cast<float*>(p0)[at] = h;
+    reinterpret_cast<float*>(p1)[at] = v - h;
   } else {
+    reinterpret_cast<__nv_bfloat16*>(p0)[at] = __float2bfloat16_rn(v);
+  }
+}
+
+template <int KIND, int PREC>
+__global__ void __launch_bounds__(kBrThreads)
+block_row_kernel(BlockRowArgs g) {
+  constexpr int kRows = KIND == 0 ? 2 * kInvNB : kInvNB;
+  // Tt[k][i] = T[i][k]: for a fixed k the multipliers of all rows i are
+  // contiguous (16-byte broadcast loads).  Padding rows/columns past nb hold the
+  // identity, so the fully unrolled substitution needs no bounds.
+  extern __shared__ __align__(16) float br_smem[];
+  float (*Tt)[kInvNB + 4] = reinterpret_cast<float (*)[kInvNB + 4]>(br_smem);
+  float (*X)[kBrLd] = reinterpret_cast<float (*)[kBrLd]>(br_smem + kInvNB * (kInvNB + 4));
+  __shared__ int s_piv[kInvNB], s_slot[kInvNB], s_row[kRows];
+  const int tid = threadIdx.x;
+  const int n = g.n, j0 = g.j0, nb = g.nb;
+  pdl_wait();
+  if ((int)blockIdx.x >= g.strips) {               // the other operand
+    if (PREC != 0) {
+      const int r0 = ((int)blockIdx.x - g.strips) * kInvNB;
+      float v[kBrLoads];
 #pragma unroll
-    for (int k = kInvNB - 1; k >= 0; --k) {
-      const float xk = x[k] / Tt[k][k];
-      x[k] = xk;
+      for (int u = 0; u < kBrLoads; ++u) {
+        const int e = tid + u * kBrThreads, r = r0 + e / kInvNB, c = e % kInvNB;
+        v[u] = (r < g.na && c < nb) ? __ldcg(g.a_src + (int64_t)r * n + c) : 0.0f;
+      }
 #pragma unroll
-      for (int i4 = 0; i4 < (k + 3) / 4; ++i4) {
-        const float4 tq = *reinterpret_cast<const float4*>(&Tt[k][4 * i4]);
-        if (4 * i4 + 0 < k) x[4 * i4 + 0] = fmaf(-tq.x, xk, x[4 * i4 + 0]);
-        if (4 * i4 + 1 < k) x[4 * i4 + 1] = fmaf(-tq.y, xk, x[4 * i4 + 1]);
-        if (4 * i4 + 2 < k) x[4 * i4 + 2] = fmaf(-tq.z, xk, x[4 * i4 + 2]);
-        if (4 * i4 + 3 < k) x[4 * i4 + 3] = fmaf(-tq.w, xk, x[4 * i4 + 3]);
+      for (int u = 0; u < kBrLoads; ++u) {
+        const int e = tid + u * kBrThreads, r = r0 + e / kInvNB, c = e % kInvNB;
+        if (r < g.na) br_store<PREC>(g.a0, g.a1, (int64_t)r * kInvNB + c, v[u]);
       }
     }
+    return;
   }
-  if (c < c_end) {
-#pragma unroll
-    for (int i = 0; i < kInvNB; ++i)
-      if (i < nb) w[(int64_t)(j0 + i) * n + c] = x[i];
+  const bool solve = KIND != 0 || (int)blockIdx.x >= g.left;
+  float t[kBrLoads];
+  const int c0 = solve ? g.c_begin + ((int)blockIdx.x - (KIND == 0 ? g.left : 0)) * kBrCols
+                       : (int)blockIdx.x * kBrCols;
+  const int cend = solve ? g.c_end : j0;
+  if (KIND == 0) {
+    if (tid < kInvNB) s_piv[tid] = (tid < nb) ? g.piv[j0 + tid] : j0 + tid;
+    __syncthreads();
+    if (tid < kInvNB) {
+      // slot of interchange k's partner: a panel row, or 64 + the first
+      // interchange that names the same outside row
+      const int p = s_piv[tid];
+      int first = tid;
+#pragma unroll 16
+      for (int k = kInvNB - 1; k >= 0; --k)
+        if (k < tid && s_piv[k] == p) first = k;
+      const bool inside = p < j0 + kInvNB;
+      s_slot[tid] = inside ? p - j0 : kInvNB + first;
+      s_row[tid] = (tid < nb) ? j0 + tid : -1;
+      s_row[kInvNB + tid] = (!inside && first == tid) ? p : -1;
+    }
+  } else if (tid < kInvNB) {
+    s_row[tid] = (tid < nb) ? j0 + tid : -1;
   }
+  if (solve) {
 #pragma unroll
-  for (int i = 0; i < kInvNB; ++i) X[i][t] = x[i];
+    for (int u = 0; u < kBrLoads; ++u) {
+      const int e = tid + u * kBrThreads;
+      const int i = e / kInvNB, k = e % kInvNB;
+      t[u] = (i < nb && k < nb) ? __ldcg(g.lu + (int64_t)(j0 + i) * n + j0 + k)
+                                : (i == k ? 1.0f : 0.0f);
+    }
+  }
   __syncthreads();
-  // Transposed copy, coalesced along the 64 entries of each column.
-  const int ncols = min(kInvCols, c_end - cbase);
-#pragma unroll 8
-  for (int e = threadIdx.x; e < ncols * kInvNB; e += kInvCols) {
-    const int col = e / kInvNB, i = e % kInvNB;
-    xt[(int64_t)(cbase - c_begin + col) * kInvNB + i] = X[i][col];
+  // all loads of a batch are issued before the first value is stored
+#pragma unroll
+  for (int h = 0; h < kRows / kInvNB; ++h) {
+    float v[kBrLoads];
+#pragma unroll
+    for (int u = 0; u < kBrLoads; ++u) {
+      const int e = tid + u * kBrThreads, i = h * kInvNB + e / kBrCols, c = e % kBrCols;
+      const int row = s_row[i];
+      v[u] = (row >= 0 && c0 + c < cend) ? __ldcg(g.w + (int64_t)row * n + c0 + c) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kBrLoads; ++u) {
+      const int e = tid + u * kBrThreads;
+      X[h * kInvNB + e / kBrCols][e % kBrCols] = v[u];
+    }
   }
+  if (solve) {
+#pragma unroll
+    for (int u = 0; u < kBrLoads; ++u) {
+      const int e = tid + u * kBrThreads;
+      Tt[e % kInvNB][e / kInvNB] = t[u];
+    }
+  }
+  __syncthreads();
+  if (KIND == 0) {
+    if (tid < kBrCols) {
+#pragma unroll 8
+      for (int k = 0; k < nb; ++k) {
+        const int sl = s_slot[k];
+        const float u = X[k][tid], v = X[sl][tid];
+        X[k][tid] = v;
+        X[sl][tid] = u;
+      }
+    }
+    __syncthreads();
+  }
+  if (solve && tid < kBrCols) {
+    // Each thread substitutes its own column, 16 rows at a time in registers:
+    // one body for the product with a 16 x 16 block and one for the triangle.
+#pragma unroll 1
+    for (int bi = 0; bi < kInvNB / kBrT; ++bi) {
+      const int i0 = (KIND != 2) ? bi * kBrT : kInvNB - kBrT - bi * kBrT;
+      float x[kBrT];
+#pragma unroll
+      for (int i = 0; i < kBrT; ++i) x[i] = X[i0 + i][tid];
+#pragma unroll 1
+      for (int bk = 0; bk < bi; ++bk) {
+        const int k0 = (KIND != 2) ? bk * kBrT : kInvNB - kBrT - bk * kBrT;
+        float xk[kBrT];
+#pragma unroll
+        for (int k = 0; k < kBrT; ++k) xk[k] = X[k0 + k][tid];
+#pragma unroll
+        for (int kk = 0; kk < kBrT; ++kk) {
+          const int k = (KIND != 2) ? kk : kBrT - 1 - kk;
+#pragma unroll
+          for (int i4 = 0; i4 < kBrT / 4; ++i4) {
+            const float4 tq = *reinterpret_cast<const float4*>(&Tt[k0 + k][i0 + 4 * i4]);
+            x[4 * i4 + 0] = fmaf(-tq.x, xk[k], x[4 * i4 + 0]);
+            x[4 * i4 + 1] = fmaf(-tq.y, xk[k], x[4 * i4 + 1]);
+            x[4 * i4 + 2] = fmaf(-tq.z, xk[k], x[4 * i4 + 2]);
+            x[4 * i4 + 3] = fmaf(-tq.w, xk[k], x[4 * i4 + 3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < kBrT; ++kk) {
+        const int k = (KIND != 2) ? kk : kBrT - 1 - kk;
+        if (KIND == 2) x[k] = x[k] / Tt[i0 + k][i0 + k];
+        const float xk = x[k];
+#pragma unroll
+        for (int i4 = 0; i4 < kBrT / 4; ++i4) {
+          if ((KIND != 2) ? (4 * i4 + 3 <= k) : (4 * i4 >= k)) continue;
+          const float4 tq = *reinterpret_cast<const float4*>(&Tt[i0 + k][i0 + 4 * i4]);
+          const float t4[4] = {tq.x, tq.y, tq.z, tq.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if ((KIND != 2) ? (4 * i4 + q > k) : (4 * i4 + q < k))
+              x[4 * i4 + q] = fmaf(-t4[q], xk, x[4 * i4 + q]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kBrT; ++i) X[i0 + i][tid] = x[i];
+    }
+  }
+  __syncthreads();
+#pragma unroll 16
+  for (int u = 0; u < kRows * kBrCols / kBrThreads; ++u) {
+    const int e = tid + u * kBrThreads, i = e / kBrCols, c = e % kBrCols;
+    const int row = s_row[i];
+    if (row >= 0 && c0 + c < cend) g.w[(int64_t)row * n + c0 + c] = X[i][c];
+  }
+  if (solve) {
+    // transposed copy, coalesced along the 64 entries of each column
+#pragma unroll 16
+    for (int u = 0; u < kInvNB * kBrCols / kBrThreads; ++u) {
+      const int e = tid + u * kBrThreads, c = e / kInvNB, i = e % kInvNB;
+      if (c0 + c < cend)
+        br_store<PREC>(g.b0, g.b1, (int64_t)(c0 + c - g.c_begin) * kInvNB + i, X[i][c]);
+    }
+  }
+}
+
+template <int KIND>
+static int launch_block_row(int prec, BlockRowArgs g, cudaStream_t st) {
+  const int cols = g.c_end - g.c_begin;
+  g.left = KIND == 0 ? (g.j0 + kBrCols - 1) / kBrCols : 0;
+  g.strips = g.left + (cols + kBrCols - 1) / kBrCols;
+  const int others = prec != 0 ? (g.na + kInvNB - 1) / kInvNB : 0;
+  if (g.strips + others == 0) return LXGB_SUCCESSFUL;
+  // (the inversions have no BF16 form)
+  auto fn = prec == 0 ? block_row_kernel<KIND, 0>
+                      : (KIND != 0 || prec == 1 ? block_row_kernel<KIND, 1>
+                                                : block_row_kernel<KIND, KIND == 0 ? 2 : 1>);
+  const int rows = KIND == 0 ? 2 * kInvNB : kInvNB;
+  const int smem = (kInvNB * (kInvNB + 4) + rows * kBrLd) * (int)sizeof(float);
+  LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(fn), smem), "block_row: set smem");
+  LXGB_CUDA_TRY(launch_pdl(fn, dim3((unsigned)(g.strips + others)), dim3(kBrThreads), (size_t)smem,
+                           st, 1, g),
+                "block_row: launch");
+  return check_launch("block_row");
 }
 
 // ---------------------------------------------------------------------------
@@ -657,12 +821,24 @@ int launch_gemv16(int m, int ncol, const float* Mh, int64_t ldm, int k, const fl
   return check_launch("gemv16");
 }
 
-int launch_inv_diag_lower(int n, int j0, int nb, const float* lu, float* w, int c_begin,
-                          int c_end, float* xt, cudaStream_t st) {
-  if (c_end <= c_begin) return LXGB_SUCCESSFUL;
-  inv_diag_kernel<true><<<(unsigned)((c_end - c_begin + kInvCols - 1) / kInvCols), kInvCols, 0,
-                          st>>>(n, j0, nb, lu, w, c_begin, c_end, xt);
-  return check_launch("inv_diag_lower");
+int lu32_block_row(int precision, int n, int j0, int nb, float* lu, const int32_t* piv, void* a0,
+                   void* a1, void* b0, void* b1, cudaStream_t st) {
+  BlockRowArgs g = {};
+  g.n = n;
+  g.j0 = j0;
+  g.nb = nb;
+  g.lu = lu;
+  g.w = lu;
+  g.piv = piv;
+  g.c_begin = j0 + nb;
+  g.c_end = n;
+  g.b0 = b0;
+  g.b1 = b1;
+  g.a_src = lu + (int64_t)(j0 + nb) * n + j0;
+  g.na = n - j0 - nb;
+  g.a0 = a0;
+  g.a1 = a1;
+  return launch_block_row<0>(precision, g, st);
 }
 
 static int64_t blk_bytes(int n) {
@@ -714,54 +890,49 @@ extern "C" int lxgb_lu32_inverse(int32_t n, const float* lu, const int32_t* piv,
   float* bh = reinterpret_cast<float*>(wb + 3 * blk);
   float* bl = reinterpret_cast<float*>(wb + 4 * blk);
   const bool split = precision == 1;
+  auto block = [&](float* w, int j0, int nb, int c_begin, int c_end, const float* a_src, int na) {
+    BlockRowArgs g = {};
+    g.n = n;
+    g.j0 = j0;
+    g.nb = nb;
+    g.lu = lu;
+    g.w = w;
+    g.c_begin = c_begin;
+    g.c_end = c_end;
+    g.b0 = split ? bh : xt;
+    g.b1 = bl;
+    g.a_src = a_src;
+    g.na = na;
+    g.a0 = ah;
+    g.a1 = al;
+    return g;
+  };
+  auto update = [&](int rows, int cols, int nb, const float* a_src, float* c) {
+    if (split)
+      return gemm_tf32_nt_split(rows, cols, nb, ah, al, kInvNB, bh, bl, kInvNB, c, n, -1.0f, 1.0f,
+                                err, st);
+    return gemm_tf32_nt(rows, cols, nb, a_src, n, xt, kInvNB, c, n, -1.0f, 1.0f, err, st);
+  };
   // L^{-1}: top to bottom.  Row block j of W = L^{-1} has nonzeros in
   // columns < j0 + nb only.  (Skipped when linv is NULL: the square QR needs
   // only R^{-1}.)
   for (int j0 = 0; linv && j0 < n; j0 += kInvNB) {
     const int nb = min(kInvNB, n - j0);
-    const int ncols = j0 + nb;
-    inv_diag_kernel<true><<<(unsigned)((ncols + kInvCols - 1) / kInvCols), kInvCols, 0, st>>>(
-        n, j0, nb, lu, linv, 0, ncols, xt);
-    const int m2 = n - ncols;
-    if (m2 > 0) {
-      const float* a21 = lu + (int64_t)ncols * n + j0;
-      float* c = linv + (int64_t)ncols * n;
-      int rc;
-      if (split) {
-        rc = tf32_split(m2, nb, a21, n, ah, al, kInvNB, st);
-        if (!rc) rc = tf32_split(ncols, kInvNB, xt, kInvNB, bh, bl, kInvNB, st);
-        if (!rc)
-          rc = gemm_tf32_nt_split(m2, ncols, nb, ah, al, kInvNB, bh, bl, kInvNB, c, n, -1.0f, 1.0f,
-                                  err, st);
-      } else {
-        rc = gemm_tf32_nt(m2, ncols, nb, a21, n, xt, kInvNB, c, n, -1.0f, 1.0f, err, st);
-      }
-      if (rc) return rc;
-    }
+    const int ncols = j0 + nb, m2 = n - ncols;
+    const float* a21 = lu + (int64_t)ncols * n + j0;
+    int rc = launch_block_row<1>(precision, block(linv, j0, nb, 0, ncols, a21, m2), st);
+    if (!rc && m2 > 0) rc = update(m2, ncols, nb, a21, linv + (int64_t)ncols * n);
+    if (rc) return rc;
   }
   // U^{-1}: bottom to top.  Row block j of W = U^{-1} has nonzeros in
   // columns >= j0 only.  (Skipped when uinv is NULL: a Cholesky factor forms
   // it from L^{-1} with lxgb_chol32_uinv.)
   for (int j0 = ((n - 1) / kInvNB) * kInvNB; uinv && j0 >= 0; j0 -= kInvNB) {
     const int nb = min(kInvNB, n - j0);
-    const int ncols = n - j0;
-    inv_diag_kernel<false><<<(unsigned)((ncols + kInvCols - 1) / kInvCols), kInvCols, 0, st>>>(
-        n, j0, nb, lu, uinv, j0, n, xt);
-    if (j0 > 0) {
-      const float* a01 = lu + j0;  // rows [0, j0), columns [j0, j0 + nb)
-      float* c = uinv + j0;
-      int rc;
-      if (split) {
-        rc = tf32_split(j0, nb, a01, n, ah, al, kInvNB, st);
-        if (!rc) rc = tf32_split(ncols, kInvNB, xt, kInvNB, bh, bl, kInvNB, st);
-        if (!rc)
-          rc = gemm_tf32_nt_split(j0, ncols, nb, ah, al, kInvNB, bh, bl, kInvNB, c, n, -1.0f, 1.0f,
-                                  err, st);
-      } else {
-        rc = gemm_tf32_nt(j0, ncols, nb, a01, n, xt, kInvNB, c, n, -1.0f, 1.0f, err, st);
-      }
-      if (rc) return rc;
-    }
+    const float* a01 = lu + j0;  // rows [0, j0), columns [j0, j0 + nb)
+    int rc = launch_block_row<2>(precision, block(uinv, j0, nb, j0, n, a01, j0), st);
+    if (!rc && j0 > 0) rc = update(j0, n - j0, nb, a01, uinv + j0);
+    if (rc) return rc;
   }
   return check_launch("lu32_inverse");
 }

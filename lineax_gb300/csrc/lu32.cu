@@ -12,9 +12,9 @@
 //                            shared memory (taller panels); and
 //                            panel_getf2_f32_kernel (one CTA, panel in global
 //                            memory) for panels too tall for either.
-//   laswp_f32_kernel       — the panel's row interchanges on the other columns
-//   launch_inv_diag_lower  — U12 = L11^{-1} A12 in place, and U12ᵀ into a
-//                            K-major buffer for the GEMM (ir.cu)
+//   lu32_block_row         — the panel's row interchanges on the other columns,
+//                            U12 = L11^{-1} A12 in place, and the operands of
+//                            the update as K-major buffers (ir.cu)
 //   gemm_tf32_nt           — A22 -= L21 U12 on the tensor cores
 #include <cooperative_groups.h>
 #include <float.h>
@@ -234,7 +234,8 @@ panel_getf2_cluster_kernel(int n, int j0, int nb, int rows_per_cta, float* __res
 //    the winning row is read from the winner's CTA.  Slots and rows alternate
 //    with the column's parity.
 // Same arithmetic and pivot choice (first row of max |a|, NaN never chosen) as
-// the shared-memory kernels.  Measured at m = 8192: see launch_panel_cluster_reg.
+// the shared-memory kernels.  Measured at m = 8192, 64 columns: 89 us (226 us with
+// the columns unrolled and rows exchanged between threads).
 constexpr int kRegPanelThreads = 512;
 constexpr int kRegHistLd = kRegPanelThreads;
 constexpr size_t kRegPanelSmem = (size_t)kLu32NB * kRegHistLd * sizeof(float);
@@ -508,22 +509,6 @@ static int launch_panel_cluster(int n, int j0, int nb, float* a, int32_t* piv, i
   return 0;
 }
 
-__global__ void laswp_f32_kernel(int n, int j0, int nb, float* __restrict__ a,
-                                 const int32_t* __restrict__ piv) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const int outside = n - nb;
-  if (c >= outside) return;
-  const int j = (c < j0) ? c : c + nb;
-  for (int k = j0; k < j0 + nb; ++k) {
-    const int p = piv[k];
-    if (p != k) {
-      const float t = a[(int64_t)k * n + j];
-      a[(int64_t)k * n + j] = a[(int64_t)p * n + j];
-      a[(int64_t)p * n + j] = t;
-    }
-  }
-}
-
 __global__ void cvt_f64_to_f32_kernel(int64_t count, const double* __restrict__ src,
                                       float* __restrict__ dst) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
@@ -603,32 +588,21 @@ extern "C" int lxgb_getrf_f32_tc(int32_t n, const double* a64, float* lu, int32_
     const int nb = min(kLu32NB, n - j0);
     if (launch_panel_cluster(n, j0, nb, lu, piv, info, st) != 0)
       panel_getf2_f32_kernel<<<1, kLu32PanelThreads, 0, st>>>(n, j0, nb, lu, piv, info);
-    const int outside = n - nb;
-    if (outside > 0) laswp_f32_kernel<<<(outside + 127) / 128, 128, 0, st>>>(n, j0, nb, lu, piv);
+    // interchanges, U12 in place and the operands of the update
+    int rc = lu32_block_row(precision, n, j0, nb, lu, piv, ah, al, precision == 0 ? bt : bh, bl, st);
+    if (rc) return rc;
     const int n2 = n - j0 - nb;
     if (n2 > 0) {
-      // U12 = L11^{-1} A12 in place, and U12ᵀ (K-major) into bt for the GEMM
-      int rc0 = launch_inv_diag_lower(n, j0, nb, lu, lu, j0 + nb, n, bt, st);
-      if (rc0) return rc0;
-      // A22 -= L21 U12   (A = L21: n2×nb at lu[(j0+nb)*n + j0], B = U12ᵀ: n2×nb)
+      // A22 -= L21 U12
       float* c22 = lu + (int64_t)(j0 + nb) * n + j0 + nb;
-      const float* l21 = lu + (int64_t)(j0 + nb) * n + j0;
-      int rc;
-      if (precision == 1) {
-        rc = tf32_split(n2, nb, l21, n, ah, al, kLu32NB, st);
-        if (!rc) rc = tf32_split(n2, nb, bt, kLu32NB, bh, bl, kLu32NB, st);
-        if (!rc)
-          rc = gemm_tf32_nt_split(n2, n2, nb, ah, al, kLu32NB, bh, bl, kLu32NB, c22, n, -1.0f, 1.0f,
-                                  err, st);
-      } else if (precision == 2) {
-        // BF16 operands (8-bit significands), FP32 accumulation in tensor memory
-        rc = bf16_convert(n2, nb, l21, n, ah, kLu32NB, st);
-        if (!rc) rc = bf16_convert(n2, nb, bt, kLu32NB, bh, kLu32NB, st);
-        if (!rc)
-          rc = gemm_bf16_nt(n2, n2, nb, ah, kLu32NB, bh, kLu32NB, c22, n, -1.0f, 1.0f, err, st);
-      } else {
-        rc = gemm_tf32_nt(n2, n2, nb, l21, n, bt, kLu32NB, c22, n, -1.0f, 1.0f, err, st);
-      }
+      if (precision == 1)
+        rc = gemm_tf32_nt_split(n2, n2, nb, ah, al, kLu32NB, bh, bl, kLu32NB, c22, n, -1.0f, 1.0f,
+                                err, st);
+      else if (precision == 2)  // BF16 operands (8-bit significands), FP32 accumulation
+        rc = gemm_bf16_nt(n2, n2, nb, ah, kLu32NB, bh, kLu32NB, c22, n, -1.0f, 1.0f, err, st);
+      else
+        rc = gemm_tf32_nt(n2, n2, nb, lu + (int64_t)(j0 + nb) * n + j0, n, bt, kLu32NB, c22, n,
+                          -1.0f, 1.0f, err, st);
       if (rc) return rc;
     }
   }

@@ -15,13 +15,13 @@ int gemm_tf32_nt_split(int M, int N, int K, const float* A, const float* Al, int
 // 3xTF32 when Al is given; the full product when tiles cannot be skipped.
 int gemm_tf32_nt_split_lower(int M, int K, const float* A, const float* Al, int64_t lda, float* C,
                              int64_t ldc, float alpha, float beta, int* err, cudaStream_t st);
-// X = L_jj^{-1} W on rows [j0, j0+nb) of w, columns [c_begin, c_end), L_jj
-// the unit-lower 64-block of lu at (j0, j0) (row stride n; lu and w may be
-// the same array when the columns are disjoint from the block).  X goes back
-// into w and, transposed and zero padded to 64 entries per column, into xt
-// (ir.cu).
-int launch_inv_diag_lower(int n, int j0, int nb, const float* lu, float* w, int c_begin,
-                          int c_end, float* xt, cudaStream_t st);
+// One block row of the FP32 LU between its panel and the trailing update
+// (ir.cu): the panel's interchanges on the other columns, U12 = L11^{-1} A12 in
+// place, and the update's operands with 64 entries per row or column: U12ᵀ in
+// b0 (FP32, precision 0; BF16, precision 2) or b0, b1 (hi, lo; precision 1),
+// L21 likewise in a0, a1 (precision 1 and 2).
+int lu32_block_row(int precision, int n, int j0, int nb, float* lu, const int32_t* piv, void* a0,
+                   void* a1, void* b0, void* b1, cudaStream_t st);
 // Split-K products C_s = A[:, K_s] B[:, K_s]ᵀ (K_s: splits ranges of chunk
 // elements, chunk % 32 == 0), C_s at C + s * M * ldc, in one launch.
 int gemm_tf32_nt_splitk(int M, int N, int K, const float* A, int64_t lda, const float* B,
