@@ -621,7 +621,8 @@ int lxgb_gemv_df(int32_t m, int32_t n, const float* a_hi, const float* a_lo,
 
 /* Mixed-precision CG for the 5-point Poisson operator (the matrix-free
  * FunctionLinearOperator of lxgb_poisson5_f64 with scale 1) on an nx×ny grid,
- * k right-hand sides: FP32 iteration vectors p, r, Ap and correction x_lo;
+ * k right-hand sides: FP32 iteration vectors p, r, correction x_lo and a
+ * scratch vector ap (the other buffer of p: A p itself is not stored);
  * FP64 solution x and right-hand side b (k vectors of nx*ny back to back).
  * lxgb_cg32_refresh folds x_lo into x, replaces r by the FP64 true residual
  * and applies lineax's max-norm stopping test to it (the solve of
