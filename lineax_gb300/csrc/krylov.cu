@@ -9,12 +9,16 @@
 // host may run iterations past convergence and only checks the flags now and
 // then.  Reductions are two-stage (per-CTA partials, then one CTA per vector
 // combining them in index order), so results do not depend on timing.
+#include <cooperative_groups.h>
 #include <math.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
 #include "krylov.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace lxgb {
 
@@ -522,45 +526,173 @@ __global__ void gm_cycle_reset_kernel(int64_t n, int k, GmWork w, int cur,
   }
 }
 
-// Arnoldi step kk for right-hand sides live and not broken down:
-//   partial dots proj[j] = <V[j], w>, j <= kk, and ||w||^2   (gmres.py:355-363)
+// Arnoldi step kk for right-hand sides live and not broken down, n up to
+// kGmClusterMaxN: the whole step (gmres.py:355-398) in one launch, one cluster of
+// CTAs per right-hand side, each with n / clusterDim rows of w in shared memory.
+// Three reductions' worth of latency bound it: the dots of w with V[0..kk] and
+// ||w||^2 by warps (one vector each), summed over the CTAs through shared memory
+// that every CTA writes into every other; w -= sum_j proj[j] V[j]; ||w|| the same
+// way; V[kk+1] = w / ||w||.  on[c] is whether the right-hand side took part.
+// Measured per step against the five kernels of the general path, whose launches
+// and partial sums in memory it saves: see gm_cluster_size.
+constexpr int kGmClusterThreads = 512;
+constexpr int kGmClusterRows = 1024;
+constexpr int kGmClusterMax = 16;
+constexpr int64_t kGmClusterMaxN = (int64_t)kGmClusterRows * kGmClusterMax;
+
+__global__ void __launch_bounds__(kGmClusterThreads)
+gm_step_cluster_kernel(int n, GmWork w, int cur, int kk, double* __restrict__ wv,
+                       int* __restrict__ on) {
+  constexpr int kWarps = kGmClusterThreads / 32;
+  __shared__ double sw[kGmClusterRows];
+  __shared__ double loc[kGmMaxRestart + 2], pj[kGmMaxRestart + 2];
+  __shared__ double sp[kGmClusterMax][kGmMaxRestart + 2], sq[kGmClusterMax], red[kWarps];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int c = blockIdx.x / C, R = w.R;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool live = gm_live(w, c, cur) && !w.fl[c * 8 + 2];
+  if (rank == 0 && tid == 0) on[c] = live;
+  if (!live) return;  // uniform over the cluster: the flags change after its first barrier
+  const int per = (n + C - 1) / C, i0 = rank * per, m = max(0, min(per, n - i0));
+  double* V = w.V + (int64_t)c * (R + 1) * n + i0;
+  double* wc = wv + (int64_t)c * n + i0;
+  for (int i = tid; i < m; i += kGmClusterThreads) sw[i] = wc[i];
+  __syncthreads();
+  const double only = sw[0];  // ||w|| of a single row
+  for (int j = warp; j <= kk + 1; j += kWarps) {
+    const double* v = V + (int64_t)j * n;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = lane; i < m; i += 32 * 8) {
+      double a[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        a[u] = (i + 32 * u < m) ? (j <= kk ? v[i + 32 * u] : sw[i + 32 * u]) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (i + 32 * u < m) acc[u & 3] = fma(a[u], sw[i + 32 * u], acc[u & 3]);
+    }
+    const double t = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+    if (lane == 0) loc[j] = t;
+  }
+  __syncthreads();
+  for (int e = tid; e < C * (kk + 2); e += kGmClusterThreads) {
+    const int dst = e / (kk + 2), j = e - dst * (kk + 2);
+    *cluster.map_shared_rank(&sp[rank][j], dst) = loc[j];
+  }
+  cluster.sync();
+  for (int j = tid; j <= kk + 1; j += kGmClusterThreads) {
+    double t = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < C; ++q) t += sp[q][j];
+    pj[j] = t;
+  }
+  __syncthreads();
+  double acc = 0.0;
+  for (int i = tid; i < m; i += kGmClusterThreads) {
+    double t = 0.0;
+    for (int j0 = 0; j0 <= kk; j0 += 8) {
+      double a[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) a[u] = (j0 + u <= kk) ? V[(int64_t)(j0 + u) * n + i] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (j0 + u <= kk) t = fma(a[u], pj[j0 + u], t);
+    }
+    const double x = sw[i] - t;
+    sw[i] = x;
+    wc[i] = x;
+    acc = fma(x, x, acc);
+  }
+  acc = warp_sum(acc);
+  if (lane == 0) red[warp] = acc;
+  __syncthreads();
+  if (warp == 0) {
+    const double t = warp_sum(lane < kWarps ? red[lane] : 0.0);
+    if (lane < C) *cluster.map_shared_rank(&sq[rank], lane) = t;
+  }
+  cluster.sync();
+  const double ss = warp_sum(lane < C ? sq[lane] : 0.0);
+  const double nrm = two_norm_from(ss, sw[0], n);
+  const double before = two_norm_from(pj[kk + 1], only, n);
+  const bool bd = nrm < before * 2.220446049250313e-16;
+  const double d = bd ? INFINITY : nrm;
+  for (int i = tid; i < m; i += kGmClusterThreads) V[(int64_t)(kk + 1) * n + i] = sw[i] / d;
+  if (rank == 0) {
+    double* row = w.coeff + (int64_t)c * R * (R + 1) + (int64_t)kk * (R + 1);
+    for (int j = tid; j <= R; j += kGmClusterThreads)
+      row[j] = (j == kk + 1) ? nrm : (j <= kk ? pj[j] : 0.0);
+    if (tid == 0) {
+      w.sc[c * 8 + 1] = before;
+      w.sc[c * 8 + 3] = nrm;
+      w.sc[c * 8 + 4] = d;
+      w.fl[c * 8 + 2] = bd;
+    }
+  }
+}
+
+// CTAs per right-hand side of the one-launch step, 0 where the general path is
+// taken: n above what the clusters hold in shared memory, or no such cluster on
+// the device.  Above the CTAs that n needs, 128 rows per CTA before another is
+// added while the clusters of all right-hand sides leave an SM to every CTA.
+// Measured, us per step of a cycle of 20, here and on the general path:
+//   n      rhs  here  general      n      rhs  here  general
+//   200      1  11.9    15.1       8192     1  16.8    25.4
+//   2000     1  12.9    25.8       8192    16  34.9    35.8
+//   2000    16  20.3    29.8       8192    64  76.9    83.1
+//   2000   200  52.1    71.5       16384   16  50.4    51.1
+// (both with a copy of w, 3 to 10 us, in front of each step; the general path's
+// dots one after the other in one CTA took 47.5 at 2000 and 48.3 at 8192 x 16).
+static int gm_cluster_size(int64_t n, int k) {
+  if (n > kGmClusterMaxN) return 0;
+  int c = 1;
+  while ((int64_t)c * kGmClusterRows < n) c *= 2;
+  while (c < kGmClusterMax && (int64_t)c * 128 < n && 2LL * c * k <= sm_count()) c *= 2;
+  return cluster_fits(reinterpret_cast<const void*>(gm_step_cluster_kernel), c, kGmClusterThreads, 0)
+             ? c
+             : 0;
+}
+
+// The general path: partial dots proj[j] = <V[j], w>, j <= kk, and ||w||^2
+// (gmres.py:355-363), one j per blockIdx.z.
 __global__ void __launch_bounds__(kKThreads)
 gm_proj_partial_kernel(int64_t n, int k, GmWork w, int cur, int kk,
                        const double* __restrict__ wv) {
   __shared__ double sm[kKThreads / 32];
-  const int c = blockIdx.y;
+  const int c = blockIdx.y, j = blockIdx.z;
   const int R = w.R;
   const bool on = gm_live(w, c, cur) && !w.fl[c * 8 + 2];
   const double* V = w.V + (int64_t)c * (R + 1) * n;
   const double* wc = wv + (int64_t)c * n;
   double* part = w.part + (int64_t)c * w.parts * (R + 2);
-  for (int j = 0; j <= kk + 1; ++j) {
-    double acc = 0.0;
-    if (on) {
-      for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-           i += (int64_t)gridDim.x * blockDim.x) {
-        const double x = wc[i];
-        acc = (j <= kk) ? fma(V[(int64_t)j * n + i], x, acc) : fma(x, x, acc);
-      }
+  double acc = 0.0;
+  if (on) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+      const double x = wc[i];
+      acc = (j <= kk) ? fma(V[(int64_t)j * n + i], x, acc) : fma(x, x, acc);
     }
-    const double s = block_reduce<false>(acc, sm);
-    if (threadIdx.x == 0) part[(int64_t)(j <= kk ? j : R + 1) * w.parts + blockIdx.x] = s;
   }
+  const double s = block_reduce<false>(acc, sm);
+  if (threadIdx.x == 0) part[(int64_t)(j <= kk ? j : R + 1) * w.parts + blockIdx.x] = s;
 }
 
+// One warp per j.
 __global__ void gm_proj_final_kernel(int k, int64_t n, GmWork w, int cur, int kk,
                                      const double* __restrict__ wv) {
   const int c = blockIdx.x;
   const int R = w.R;
   if (!(gm_live(w, c, cur) && !w.fl[c * 8 + 2])) return;
   const double* part = w.part + (int64_t)c * w.parts * (R + 2);
-  for (int j = 0; j <= R; ++j) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int j = threadIdx.x >> 5; j <= R + 1; j += nw) {
     double v = 0.0;
-    if (j <= kk) v = combine(part + (int64_t)j * w.parts, w.parts, false);
-    if (threadIdx.x == 0) w.proj[c * (R + 1) + j] = v;
+    if (j <= kk || j == R + 1) v = combine(part + (int64_t)j * w.parts, w.parts, false);
+    if (lane == 0) {
+      if (j <= R) w.proj[c * (R + 1) + j] = v;
+      else w.sc[c * 8 + 1] = two_norm_from(v, wv[(int64_t)c * n], n);
+    }
   }
-  const double ss = combine(part + (int64_t)(R + 1) * w.parts, w.parts, false);
-  if (threadIdx.x == 0) w.sc[c * 8 + 1] = two_norm_from(ss, wv[(int64_t)c * n], n);
 }
 
 // w -= sum_{j<=kk} proj[j] V[j]; partial ||w||^2 (gmres.py:364-366).
@@ -578,6 +710,7 @@ gm_orth_kernel(int64_t n, int k, GmWork w, int cur, int kk, double* __restrict__
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
       double s = 0.0;
+#pragma unroll 8
       for (int j = 0; j <= kk; ++j) s = fma(V[(int64_t)j * n + i], pj[j], s);
       const double x = wc[i] - s;
       wc[i] = x;
@@ -626,72 +759,51 @@ __global__ void gm_snapshot_kernel(int k, GmWork w, int cur, int* on) {
 }
 
 // Least squares min ||H z - r_norm e1|| with H = coeffᵀ ((R+1)×R) by
-// Householder QR in shared memory, one CTA per right-hand side (the
-// linear_solve(..., QR()) of gmres.py:301-303).
-__global__ void __launch_bounds__(64)
+// Householder QR in shared memory, one warp per right-hand side (the
+// linear_solve(..., QR()) of gmres.py:301-303).  H is upper Hessenberg (row kk of
+// coeff ends at kk + 1), so each reflection has two rows; a lane takes every 32nd
+// column.  A chain of R reflections and R back-substitution steps bounds it:
+// 44 us for R = 20 (116 with full columns and one thread's sums).
+__global__ void __launch_bounds__(32)
 gm_lstsq_kernel(int k, GmWork w, int cur) {
   extern __shared__ double smem_h[];  // (R+1)×(R+1) matrix, then rhs
-  __shared__ double s_tau, s_beta, s_scal;
-  const int c = blockIdx.x;
+  const int c = blockIdx.x, lane = threadIdx.x;
   if (!gm_live(w, c, cur)) return;
   const int R = w.R, m = R + 1;
   const int ldh = R + 1;
   double* rhs = smem_h + (int64_t)ldh * m;
 #define H(i, j) smem_h[(i) * ldh + (j)]
   const double* cm = w.coeff + (int64_t)c * R * (R + 1);
-  for (int e = threadIdx.x; e < m * R; e += blockDim.x) {
-    const int i = e / R, j = e % R;
-    H(i, j) = cm[(int64_t)j * (R + 1) + i];  // H = coeffᵀ
-  }
-  for (int i = threadIdx.x; i < m; i += blockDim.x) rhs[i] = (i == 0) ? w.sc[c * 8 + 0] : 0.0;
-  __syncthreads();
+  for (int e = lane; e < m * R; e += 32) H(e % m, e / m) = cm[e];  // H = coeffᵀ
+  for (int i = lane; i < m; i += 32) rhs[i] = (i == 0) ? w.sc[c * 8 + 0] : 0.0;
+  __syncwarp();
   for (int j = 0; j < R; ++j) {
-    if (threadIdx.x == 0) {
-      double ss = 0.0;
-      for (int i = j + 1; i < m; ++i) ss = fma(H(i, j), H(i, j), ss);
-      const double alpha = H(j, j);
-      const double xn = sqrt(ss);
-      if (xn == 0.0) {
-        s_tau = 0.0;
-        s_scal = 1.0;
-        s_beta = alpha;
-      } else {
-        const double beta = -copysign(hypot(alpha, xn), alpha);
-        s_tau = (beta - alpha) / beta;
-        s_scal = 1.0 / (alpha - beta);
-        s_beta = beta;
-      }
+    // every lane forms the reflection of rows j and j + 1
+    const double alpha = H(j, j), below = H(j + 1, j);
+    double tau = 0.0, v = below, beta = alpha;
+    if (below != 0.0) {  // (NaN included)
+      beta = -copysign(hypot(alpha, below), alpha);
+      tau = (beta - alpha) / beta;
+      v = below / (alpha - beta);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int i = j + 1; i < m; ++i) H(i, j) *= s_scal;
-      H(j, j) = s_beta;
+    for (int q = j + 1 + lane; q <= R; q += 32) {  // q = R: the right-hand side
+      double* top = (q == R) ? rhs + j : &H(j, q);
+      double* bot = (q == R) ? rhs + j + 1 : &H(j + 1, q);
+      const double wq = fma(v, *bot, *top) * tau;
+      *top -= wq;
+      *bot = fma(-wq, v, *bot);
     }
-    __syncthreads();
-    const double tj = s_tau;
-    // apply H_j to the columns > j and to rhs (column index R)
-    for (int q = j + 1 + threadIdx.x; q <= R; q += blockDim.x) {
-      double* col_rhs = (q == R) ? rhs : nullptr;
-      double wq = (q == R) ? rhs[j] : H(j, q);
-      for (int i = j + 1; i < m; ++i) wq = fma(H(i, j), col_rhs ? rhs[i] : H(i, q), wq);
-      wq *= tj;
-      if (col_rhs) {
-        rhs[j] -= wq;
-        for (int i = j + 1; i < m; ++i) rhs[i] = fma(-wq, H(i, j), rhs[i]);
-      } else {
-        H(j, q) -= wq;
-        for (int i = j + 1; i < m; ++i) H(i, q) = fma(-wq, H(i, j), H(i, q));
-      }
-    }
-    __syncthreads();
+    __syncwarp();
+    if (lane == 0) H(j, j) = beta;
+    __syncwarp();
   }
-  if (threadIdx.x == 0) {
-    double* zc = w.z + (int64_t)c * R;
-    for (int i = R - 1; i >= 0; --i) {
-      double s = rhs[i];
-      for (int j = i + 1; j < R; ++j) s = fma(-H(i, j), zc[j], s);
-      zc[i] = s / H(i, i);
-    }
+  double* zc = w.z + (int64_t)c * R;
+  for (int i = R - 1; i >= 0; --i) {
+    const double zi = rhs[i] / H(i, i);
+    __syncwarp();
+    if (lane == 0) zc[i] = zi;
+    for (int q = lane; q < i; q += 32) rhs[q] = fma(-H(q, i), zi, rhs[q]);
+    __syncwarp();
   }
 #undef H
 }
@@ -711,6 +823,7 @@ __global__ void gm_update_kernel(int64_t n, int k, GmWork w, int cur, int first,
       diff[o + i] = INFINITY;
     } else {
       double s = 0.0;
+#pragma unroll 8
       for (int j = 0; j < R; ++j) s = fma(V[(int64_t)j * n + i], zc[j], s);
       diff[o + i] = s;
       y[o + i] += s;
@@ -859,10 +972,26 @@ extern "C" int lxgb_gmres_arnoldi(int32_t k, int64_t n, int32_t restart, int32_t
   cudaStream_t st = as_stream(stream);
   GmWork w = gm_carve(work, k, n, restart);
   const int cur = parity & 1;
+  if (const int c = gm_cluster_size(n, k)) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(c * k));
+    cfg.blockDim = dim3(kGmClusterThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LXGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, gm_step_cluster_kernel, (int)n, w, cur, kk, wv, (int*)on),
+                  "gmres_arnoldi: launch");
+    return check_launch("gmres_arnoldi");
+  }
   dim3 g(w.parts, k);
   gm_snapshot_kernel<<<(k + 127) / 128, 128, 0, st>>>(k, w, cur, on);
-  gm_proj_partial_kernel<<<g, kKThreads, 0, st>>>(n, k, w, cur, kk, wv);
-  gm_proj_final_kernel<<<k, 32, 0, st>>>(k, n, w, cur, kk, wv);
+  gm_proj_partial_kernel<<<dim3(w.parts, k, kk + 2), kKThreads, 0, st>>>(n, k, w, cur, kk, wv);
+  gm_proj_final_kernel<<<k, 32 * std::min(32, restart + 2), 0, st>>>(k, n, w, cur, kk, wv);
   gm_orth_kernel<<<g, kKThreads, 0, st>>>(n, k, w, cur, kk, wv);
   gm_norm_final_kernel<<<k, 32, 0, st>>>(k, n, w, cur, kk, wv);
   gm_store_basis_kernel<<<g, kKThreads, 0, st>>>(n, k, w, cur, kk, wv, on);
@@ -883,7 +1012,7 @@ extern "C" int lxgb_gmres_cycle_end(int32_t k, int64_t n, int32_t restart, int32
     const size_t smem = (size_t)(restart + 1) * (restart + 2) * sizeof(double);
     LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(gm_lstsq_kernel), (int)smem),
                   "gmres: set smem");
-    gm_lstsq_kernel<<<k, 64, smem, st>>>(k, w, cur);
+    gm_lstsq_kernel<<<k, 32, smem, st>>>(k, w, cur);
   }
   dim3 g(w.parts, k);
   gm_update_kernel<<<g, kKThreads, 0, st>>>(n, k, w, cur, first, y, diff);
@@ -977,6 +1106,25 @@ __global__ void cg_result_kernel(int k, CgWork w, int64_t max_steps, int max_giv
     res = (s == max_steps) ? LXGB_MAX_STEPS_REACHED : LXGB_SUCCESSFUL;
   steps[c] = s;
   results[c] = res;
+}
+
+// After an outer iteration of parity 1: its flags back to parity 1, and another
+// round while any right-hand side goes on.
+__global__ void __launch_bounds__(256)
+gm_next_cycle_kernel(cudaGraphConditionalHandle h, GmWork w, int k, int* __restrict__ counter,
+                     int max_rounds) {
+  int any = 0;
+  for (int c = threadIdx.x; c < k; c += blockDim.x) {
+    const int go = w.fl[c * 8];
+    w.fl[c * 8 + 1] = go;
+    any |= go;
+  }
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) {
+    const int rounds = *counter + 1;
+    *counter = rounds;
+    cudaGraphSetConditional(h, (any && rounds < max_rounds) ? 1u : 0u);
+  }
 }
 
 __global__ void gm_result_kernel(int k, GmWork w, int64_t max_steps, int max_given,
@@ -1393,27 +1541,25 @@ static int gmres_enqueue(Capture& cap, cudaStream_t st, const GmresCall& c, cons
   int rc = lxgb_gmres_init(k, n, R, gmws, gmb, st);
   if (!rc) rc = outer(0, 1, st);
   if (rc) return rc;
-  // rounds of two outer iterations (parities 1, 0); the flags of parity 1
-  // are the loop condition after each round
-  const int64_t rounds64 = (c.max_s + 1) / 2 + 2;
-  const int max_rounds = (int)(rounds64 < (1LL << 30) ? rounds64 : (1LL << 30));
+  // one outer iteration per round, always of parity 1: gm_next_cycle_kernel
+  // moves the flags it leaves in parity 0 back, and they are the loop condition
+  const int max_rounds = (int)(c.max_s < (1LL << 30) ? c.max_s + 4 : (1LL << 30));
   cudaGraphConditionalHandle h;
   if ((rc = cap.handle(st, &h, who))) return rc;
   loop_cond_kernel<<<1, 32, 0, st>>>(h, w.fl + 1, k, 8, counter, max_rounds, 1);
   cudaStream_t sb;
   if ((rc = cap.cond(st, h, cudaGraphCondTypeWhile, 1, &sb, who))) return rc;
-  rc = outer(1, 0, sb);
-  if (!rc) rc = outer(0, 0, sb);
-  if (rc) return rc;
-  loop_cond_kernel<<<1, 32, 0, sb>>>(h, w.fl + 1, k, 8, counter, max_rounds, 0);
+  if ((rc = outer(1, 0, sb))) return rc;
+  gm_next_cycle_kernel<<<1, 256, 0, sb>>>(h, w, k, counter, max_rounds);
   if ((rc = cap.end_body(sb, who))) return rc;
   gm_result_kernel<<<(k + 127) / 128, 128, 0, st>>>(k, w, c.max_s, c.max_given, has_scale,
                                                      c.stagnation_iters, c.steps, c.results);
   return check_launch(who);
 }
 
-static int gmres_prepare(int R, const char* who) {
-  // the least-squares kernel's shared memory is raised outside any capture
+static int gmres_prepare(int64_t n, int k, int R, const char* who) {
+  // kernel attributes are set outside any capture
+  gm_cluster_size(n, k);
   const size_t smem = (size_t)(R + 1) * (R + 2) * sizeof(double);
   LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(gm_lstsq_kernel), (int)smem),
                 who);
@@ -1446,7 +1592,7 @@ extern "C" int lxgb_gmres_run(int32_t k, int64_t n, const lxgb_linear_operator* 
     set_last_error("gmres_run: workspace too small");
     return LXGB_WORKSPACE_TOO_SMALL;
   }
-  if ((rc = gmres_prepare(R, who))) return rc;
+  if ((rc = gmres_prepare(n, k, R, who))) return rc;
   const bool max_given = max_steps >= 0;
   GmresCall c{k, n, R, op, precond, b, y, rtol, atol, max_given ? max_steps : 10 * n,
               max_given ? 1 : 0, stagnation_iters, work, steps, results};
@@ -1601,7 +1747,7 @@ extern "C" int lxgb_gmres_ir_run(int32_t k, int64_t n, const lxgb_linear_operato
     set_last_error("gmres_ir_run: workspace too small");
     return LXGB_WORKSPACE_TOO_SMALL;
   }
-  if ((rc = gmres_prepare(R, who))) return rc;
+  if ((rc = gmres_prepare(n, k, R, who))) return rc;
   char* wb = reinterpret_cast<char*>(work);
   double* rr = reinterpret_cast<double*>(wb + L.rr);
   double* rhat = reinterpret_cast<double*>(wb + L.rhat);
