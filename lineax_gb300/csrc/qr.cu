@@ -558,6 +558,7 @@ qr_panel_rot_f32_kernel(int64_t mm, int j0, int nb, int R, float* __restrict__ h
   const int x0 = rank * R;                         // first row, relative to j0
   float r[RR][kQrNB];
   pdl_wait();
+  pdl_trigger();  // the wide update of the panel before runs beside this one
 #pragma unroll
   for (int rr = 0; rr < RR; ++rr) {
     const int x = rr * nrow + tid;
@@ -1293,7 +1294,7 @@ extern "C" int64_t lxgb_geqrf_f32_tc_workspace_size(int64_t m, int64_t n) {
   const int64_t v = qr32_align((int64_t)kQrNB * m * 4);
   const int64_t wp = qr32_align((int64_t)kQr32Split * (n > 0 ? n : 1) * kQrNB * 4);
   const int64_t w2 = qr32_align((int64_t)(n > 0 ? n : 1) * kQrNB * 4);
-  return 256 + 2 * v + wp + w2;
+  return 256 + 3 * v + wp + w2;
 }
 
 namespace lxgb {
@@ -1331,12 +1332,21 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
   const int64_t wpb = qr32_align((int64_t)kQr32Split * rows_w * kQrNB * 4);
   char* wb = reinterpret_cast<char*>(work) + 256;
   float* vrows = reinterpret_cast<float*>(wb);
-  float* vcols = reinterpret_cast<float*>(wb + vb);
-  float* wpart = reinterpret_cast<float*>(wb + 2 * vb);
-  float* w2 = reinterpret_cast<float*>(wb + 2 * vb + wpb);
+  // the reflectors by columns, two in turn: a panel writes its own while the
+  // update beside it still reads those of the panel before
+  float* vcols2[2] = {reinterpret_cast<float*>(wb + vb), reinterpret_cast<float*>(wb + 2 * vb)};
+  float* wpart = reinterpret_cast<float*>(wb + 3 * vb);
+  float* w2 = reinterpret_cast<float*>(wb + 3 * vb + wpb);
   const int nn = (int)n;
-  // C -= (C Vᵀ) T' V on the rows c[0..rows) (each a column being transformed)
-  auto apply = [&](float* c, int rows, int j0, int nb, const float* Tp) -> int {
+  // C -= W' V on `rows` rows from c, W' from w2's row w0 on
+  auto update = [&](float* c, int w0, int rows, int j0, int nb, bool beside) -> int {
+    return gemm_tf32_nt(rows, (int)(m - j0), nb, w2 + (int64_t)w0 * kQrNB, kQrNB,
+                        vcols2[(j0 / kQrNB) & 1] + (int64_t)j0 * kQrNB, kQrNB, c + j0, m, -1.0f,
+                        1.0f, err, st, beside);
+  };
+  // W' = (C Vᵀ) T' of the rows c[0..rows) (each a column being transformed),
+  // then the update of the first `now` of them
+  auto apply = [&](float* c, int rows, int now, int j0, int nb, const float* Tp) -> int {
     const int64_t klen = m - j0;
     const int64_t chunk = ((klen + kQr32Split - 1) / kQr32Split + 31) / 32 * 32;
     const int used = (int)((klen + chunk - 1) / chunk);
@@ -1345,13 +1355,14 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
                                   (int)chunk, used, err, st);
     if (rc0) return rc0;
     qr32_wt_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(rows, nb, used, wpart, Tp, w2);
-    return gemm_tf32_nt(rows, (int)klen, nb, w2, kQrNB, vcols + (int64_t)j0 * kQrNB, kQrNB,
-                        c + j0, m, -1.0f, 1.0f, err, st);
+    return update(c, 0, now, j0, nb, false);
   };
+  const bool ahead = q == nullptr;  // (w2 is one workspace: with q it is taken at once)
   for (int j0 = 0; j0 < nn; j0 += kQrNB) {
     const int nb = min(kQrNB, nn - j0);
     float* Tp = t + (int64_t)(j0 / kQrNB) * kQrNB * kQrNB;
     const int n2 = nn - (j0 + nb);
+    float* vcols = vcols2[(j0 / kQrNB) & 1];
     if (launch_qr_panel_rot(m, j0, nb, h, tau, Tp, vrows, vcols, st) != 0) {
       if (launch_qr_panel_cluster<float>(m, j0, j0 + nb, h, tau, Tp, st) != 0) {
         set_last_error("%s: the panel's thread-block cluster cannot be scheduled", who);
@@ -1361,15 +1372,16 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
       qr32_make_v_kernel<<<(unsigned)((tot + 255) / 256 < 4096 ? (tot + 255) / 256 : 4096), 256,
                            0, st>>>(m, j0, nb, h, vrows, vcols);
     }
-    if (n2 <= 0 && !q) continue;
-    if (n2 > 0) {
-      int rc = apply(h + (int64_t)(j0 + nb) * m, n2, j0, nb, Tp);  // trailing rows of h
-      if (rc) return rc;
-    }
-    if (q) {
-      int rc = apply(q, (int)m, j0, nb, Tp);
-      if (rc) return rc;
-    }
+    // the rows of h after this panel take the panel before beside it (16384 x
+    // 2048: 64 updates of 40 us and 64 panels of 86, least squares 13.4 -> 11.5 ms)
+    int rc = 0;
+    if (ahead && j0 > 0 && n2 > 0)
+      rc = update(h + (int64_t)(j0 + nb) * m, kQrNB, n2, j0 - kQrNB, kQrNB, true);
+    // trailing rows of h: with `ahead` the next panel's now, the others beside it
+    if (!rc && n2 > 0)
+      rc = apply(h + (int64_t)(j0 + nb) * m, n2, ahead ? min(kQrNB, n2) : n2, j0, nb, Tp);
+    if (!rc && q) rc = apply(q, (int)m, (int)m, j0, nb, Tp);
+    if (rc) return rc;
   }
   return check_launch(who);
 }

@@ -21,6 +21,7 @@
 #include <cudaTypedefs.h>
 
 #include "common.cuh"
+#include "tc_gemm.cuh"
 #include "tcgen05.cuh"
 
 #include <cuda_bf16.h>
@@ -355,7 +356,7 @@ gemm_nt_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                           const __grid_constant__ CUtensorMap map_al,
                           const __grid_constant__ CUtensorMap map_bl,
                           const __grid_constant__ CUtensorMap map_c, int M, int N, int K,
-                          float alpha, float beta, int* err, int lower) {
+                          float alpha, float beta, int* err, int lower, int beside) {
   constexpr bool SPLIT = Cfg::SPLIT;
   constexpr bool BF = MODE == 2;
   constexpr int BN = Cfg::BN, S = Cfg::S;
@@ -598,6 +599,7 @@ gemm_nt_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                  "r"(Cfg::TMEM_COLS)
                  : "memory");
   }
+  if (beside) pdl_wait();  // so that this kernel's end is also the panel's
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no libcuda link).
@@ -649,13 +651,17 @@ __global__ void scale_c_kernel(int M, int N, float* C, int64_t ldc, float beta) 
 // can be addressed by a tensor map; 0: one CTA per 128×128 tile.
 static int g_gemm_persistent = 1;
 
+// SMs left to the panel kernel by a product launched beside it: the largest
+// cluster a panel takes.
+constexpr int kBesideSms = 16;
+
 // Persistent launch; returns -1 when C cannot be addressed by a tensor map
 // (the caller then uses the one-tile-per-CTA kernel).
 template <int MODE, class Cfg>
 static int gemm_persistent_cfg(int M, int N, int K, const void* A, const void* Al, int64_t lda,
                                const void* B, const void* Bl, int64_t ldb, float* C, int64_t ldc,
                                float alpha, float beta, int* err, cudaStream_t st,
-                               int lower = 0) {
+                               int lower = 0, bool beside = false) {
   constexpr bool BF = MODE == 2;
   if (!g_gemm_persistent) return -1;
   if ((((uintptr_t)C) & 15) != 0 || (ldc % 4) != 0) return -1;
@@ -677,12 +683,19 @@ static int gemm_persistent_cfg(int M, int N, int K, const void* A, const void* A
     if (rc) return rc;
   }
   const int64_t tiles = (int64_t)((M + kTcM - 1) / kTcM) * ((N + Cfg::BN - 1) / Cfg::BN);
-  const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+  const int ctas = sm_count() - (beside ? kBesideSms : 0);
+  const int grid = (int)(tiles < ctas ? tiles : ctas);
   auto kern = gemm_nt_persistent_kernel<MODE, Cfg>;
   LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg::SMEM),
                 "gemm persistent: set smem");
+  if (beside) {
+    LXGB_CUDA_TRY(launch_pdl(kern, dim3((unsigned)grid), dim3(kPThreads), Cfg::SMEM, st, 1, ma, mb,
+                             mal, mbl, mc, M, N, K, alpha, beta, err, lower, 1),
+                  "gemm persistent: launch");
+    return check_launch("gemm persistent");
+  }
   kern<<<grid, kPThreads, Cfg::SMEM, st>>>(ma, mb, mal, mbl, mc, M, N, K, alpha, beta, err,
-                                           lower);
+                                           lower, 0);
   return check_launch("gemm persistent");
 }
 
@@ -690,30 +703,31 @@ static int gemm_persistent_cfg(int M, int N, int K, const void* A, const void* A
 template <int MODE>
 static int gemm_persistent(int M, int N, int K, const void* A, const void* Al, int64_t lda,
                            const void* B, const void* Bl, int64_t ldb, float* C, int64_t ldc,
-                           float alpha, float beta, int* err, cudaStream_t st) {
+                           float alpha, float beta, int* err, cudaStream_t st,
+                           bool beside = false) {
   const int kstage = MODE == 2 ? 2 * kTcK : kTcK;
   const bool short_k = beta != 0.0f && K <= 2 * kstage;
   if constexpr (MODE == 0) {
     if (short_k)
       return gemm_persistent_cfg<0, PCfgTf32ShortK>(M, N, K, A, Al, lda, B, Bl, ldb, C, ldc,
-                                                    alpha, beta, err, st);
+                                                    alpha, beta, err, st, 0, beside);
     return gemm_persistent_cfg<0, PCfgTf32>(M, N, K, A, Al, lda, B, Bl, ldb, C, ldc, alpha, beta,
-                                            err, st);
+                                            err, st, 0, beside);
   } else if constexpr (MODE == 2) {
     if (short_k)
       return gemm_persistent_cfg<2, PCfgBf16ShortK>(M, N, K, A, Al, lda, B, Bl, ldb, C, ldc,
-                                                    alpha, beta, err, st);
+                                                    alpha, beta, err, st, 0, beside);
     return gemm_persistent_cfg<2, PCfgBf16>(M, N, K, A, Al, lda, B, Bl, ldb, C, ldc, alpha, beta,
-                                            err, st);
+                                            err, st, 0, beside);
   } else {
     return gemm_persistent_cfg<1, PCfgSplit>(M, N, K, A, Al, lda, B, Bl, ldb, C, ldc, alpha, beta,
-                                             err, st);
+                                             err, st, 0, beside);
   }
 }
 
 int gemm_tf32_nt_split(int M, int N, int K, const float* A, const float* Al, int64_t lda,
                        const float* B, const float* Bl, int64_t ldb, float* C, int64_t ldc,
-                       float alpha, float beta, int* err, cudaStream_t st) {
+                       float alpha, float beta, int* err, cudaStream_t st, bool beside) {
   if (M <= 0 || N <= 0) return LXGB_SUCCESSFUL;
   if (K == 0) {  // C = beta * C
     const int64_t total = (int64_t)M * N;
@@ -723,9 +737,9 @@ int gemm_tf32_nt_split(int M, int N, int K, const float* A, const float* Al, int
   const bool split = (Al != nullptr) && (Bl != nullptr);
   {
     const int prc = split ? gemm_persistent<1>(M, N, K, A, Al, lda, B, Bl, ldb, C, ldc, alpha,
-                                               beta, err, st)
+                                               beta, err, st, beside)
                           : gemm_persistent<0>(M, N, K, A, nullptr, lda, B, nullptr, ldb, C, ldc,
-                                               alpha, beta, err, st);
+                                               alpha, beta, err, st, beside);
     if (prc >= 0) return prc;
   }
   CUtensorMap ma, mb, mal, mbl;
@@ -790,9 +804,10 @@ int gemm_tf32_nt_split_lower(int M, int K, const float* A, const float* Al, int6
 }
 
 int gemm_tf32_nt(int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb,
-                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st) {
+                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
+                 bool beside) {
   return gemm_tf32_nt_split(M, N, K, A, nullptr, lda, B, nullptr, ldb, C, ldc, alpha, beta, err,
-                            st);
+                            st, beside);
 }
 
 // Split-K: C_s = A[:, K_s] B[:, K_s]ᵀ for s < splits, K_s the s-th range of
@@ -822,7 +837,8 @@ int gemm_tf32_nt_splitk(int M, int N, int K, const float* A, int64_t lda, const 
 // C = alpha A Bᵀ + beta C with BF16 operands (A m×k, B n×k, K-major, row
 // strides multiples of 8 elements, 16-byte aligned), FP32 C.
 int gemm_bf16_nt(int M, int N, int K, const void* A, int64_t lda, const void* B, int64_t ldb,
-                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st) {
+                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
+                 bool beside) {
   if (M <= 0 || N <= 0) return LXGB_SUCCESSFUL;
   if (K == 0) {
     const int64_t total = (int64_t)M * N;
@@ -831,7 +847,7 @@ int gemm_bf16_nt(int M, int N, int K, const void* A, int64_t lda, const void* B,
   }
   {
     const int prc = gemm_persistent<2>(M, N, K, A, nullptr, lda, B, nullptr, ldb, C, ldc, alpha,
-                                       beta, err, st);
+                                       beta, err, st, beside);
     if (prc >= 0) return prc;
   }
   CUtensorMap ma, mb;

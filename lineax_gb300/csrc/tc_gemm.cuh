@@ -5,12 +5,17 @@
 #include "common.cuh"
 
 namespace lxgb {
+// beside: the kernel before it on the stream is a panel that lets its successor
+// start at once and touches nothing of this product; the product then runs on
+// the SMs the panel leaves and ends no earlier than the panel.  (Without the
+// persistent kernel it runs after the panel.)
 int gemm_tf32_nt(int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb,
-                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st);
+                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
+                 bool beside = false);
 // 3xTF32 when Al and Bl (the lo parts) are given, plain TF32 otherwise.
 int gemm_tf32_nt_split(int M, int N, int K, const float* A, const float* Al, int64_t lda,
                        const float* B, const float* Bl, int64_t ldb, float* C, int64_t ldc,
-                       float alpha, float beta, int* err, cudaStream_t st);
+                       float alpha, float beta, int* err, cudaStream_t st, bool beside = false);
 // C = alpha A Aᵀ + beta C on the tiles holding C's lower triangle (M×M),
 // 3xTF32 when Al is given; the full product when tiles cannot be skipped.
 int gemm_tf32_nt_split_lower(int M, int K, const float* A, const float* Al, int64_t lda, float* C,
@@ -29,7 +34,8 @@ int gemm_tf32_nt_splitk(int M, int N, int K, const float* A, int64_t lda, const 
                         cudaStream_t st);
 // BF16 operands (kind::f16, FP32 accumulation); A and B hold __nv_bfloat16.
 int gemm_bf16_nt(int M, int N, int K, const void* A, int64_t lda, const void* B, int64_t ldb,
-                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st);
+                 float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
+                 bool beside = false);
 // dst = src rounded to BF16 (rows × cols; row strides in elements).
 int bf16_convert(int64_t rows, int64_t cols, const float* src, int64_t lds, void* dst, int64_t ldd,
                  cudaStream_t st);
