@@ -32,6 +32,8 @@ namespace lxgb {
 
 constexpr int kSmallMax = 168;   // 168*169*8 B = 227 KB of shared memory
 constexpr int kSmallThreads = 256;
+constexpr int kSmallMaxThreads = 512;
+constexpr int kSmallBlocks = (kSmallMax + 31) / 32;
 constexpr int kNB = 32;          // panel width of the blocked path
 constexpr int kPanelThreads = 1024;
 
@@ -42,118 +44,186 @@ __device__ __forceinline__ double scale_pivot(double v, double akk, double r, bo
 // ---------------------------------------------------------------------------
 // n <= kSmallMax: one CTA per matrix, matrix in shared memory (row stride ld,
 // odd so that column walks hit distinct banks).
+//
+// Warp 0 carries the chain of pivots with the current column in its registers
+// (row 32 m + lane in register m): while the other warps apply step k to columns
+// >= k + 2 it applies it to column k + 1, finds that column's first maximum by
+// integer reductions, forms the reciprocal and writes the multipliers.  The
+// others exchange rows k and p as they go: they read u from row p and leave row
+// k's update there.  One barrier per column for the CTA, one among the others.
+// Bound by the chain up to n of about 64 — an FMA, the reductions, a division, a
+// product and a barrier per column, its FP64 instructions in turn with those of
+// the update — and by the FP64 pipe of one SM above (n = 128: 217 us of FMAs).
+// Measured (one matrix): 47 us at n = 48, 289 at 128, 566 at 168, against 64, 328
+// and 660 with the exchange and the scaling between two barriers.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kSmallThreads)
+// Step k on columns k + 2 .. n - 1, exactly NC chunks of 16, a half warp per row:
+// rows i0, i0 + 1, i0 + step, ... > k.  Row p (the pivot, still in its place; p = k
+// without an interchange) gives u; where i = p the old row k takes the step and
+// goes there, and u goes to row k.  The number of chunks is a template argument
+// because a chunk that is only predicated off still costs its FP64 instruction.
+// `threads`: those that run this.
+template <int NC>
+__device__ __forceinline__ void small_update(double* A, int ld, int n, int k, int p, int i0,
+                                             int step, int lane, int threads) {
+  const int j = k + 2 + (lane & 15);
+  const bool last = j + 16 * (NC - 1) < n;   // the other chunks are full
+  double u[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) u[c] = (c + 1 < NC || last) ? A[p * ld + j + 16 * c] : 0.0;
+  // every u is read before row p is written
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+  for (int ib = i0; ib < n; ib += step) {
+    const int i = ib + (lane >> 4);
+    const bool in = i < n;
+    double* y = A + (in ? i : k) * ld;
+    const double* src = (i == p) ? A + k * ld : y;
+    const double l = y[k];
+    double v[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = (c + 1 < NC || last) ? src[j + 16 * c] : 0.0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = fma(-l, u[c], v[c]);
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      if (in && (c + 1 < NC || last)) y[j + 16 * c] = v[c];
+    if (i == p) {
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (c + 1 < NC || last) A[k * ld + j + 16 * c] = u[c];
+    }
+  }
+}
+
+template <int MAX>
+__device__ __forceinline__ void small_update_n(int nc, double* A, int ld, int n, int k, int p,
+                                               int i0, int step, int lane, int threads) {
+  if constexpr (MAX > 0) {
+    if (nc == MAX) small_update<MAX>(A, ld, n, k, p, i0, step, lane, threads);
+    else small_update_n<MAX - 1>(nc, A, ld, n, k, p, i0, step, lane, threads);
+  }
+}
+
+template <int MB>
+__global__ void __launch_bounds__(kSmallMaxThreads)
 getrf_small_kernel(int n, double* __restrict__ a, int64_t stride_a, int32_t* __restrict__ piv,
                    int64_t stride_piv, int32_t* __restrict__ info) {
   extern __shared__ double smem_lu[];
-  // pivot of step k in slot k & 1: row, |a| test for the reciprocal, a(p,k),
-  // the old a(k,k), 1/a(p,k)
-  __shared__ int s_p[2], s_recip[2];
-  __shared__ double s_akk[2], s_old[2], s_rcp[2];
+  __shared__ int s_p[2];               // pivot row of the step (k: no interchange), by parity
   const int ld = n | 1;
   double* A = smem_lu;
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nwarps = blockDim.x >> 5;
   const int b = blockIdx.x;
   double* g = a + (int64_t)b * stride_a;
   int32_t* gp = piv + (int64_t)b * stride_piv;
-  for (int e = tid; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e - i * n;
-    A[i * ld + j] = g[e];
-  }
-  int my_info = 0;
-  const int tx = tid & 31, ty = tid >> 5;
-  constexpr int kUpdWarps = (kSmallThreads >> 5) - 1;   // warps 1.. update columns >= k + 2
-  // Warp 0: pivot of column k (rows >= k) into slot k & 1; `upd` first
-  // applies step k - 1 to that column (the lookahead: the pivot search of
-  // step k overlaps the other warps' update of step k - 1).
-  auto pivot_warp = [&](int k, bool upd) {
-    long long v = -1;
-    int idx = INT_MAX;
-    const double uk = upd ? A[(k - 1) * ld + k] : 0.0;
-    for (int i = k + lane; i < n; i += 32) {
-      double x = A[i * ld + k];
-      if (upd) {
-        x = fma(-A[i * ld + k - 1], uk, x);
-        A[i * ld + k] = x;
-      }
-      const long long key = pivot_key(x);
-      if (key > v) { v = key; idx = i; }
+  constexpr int kLoads = 8;
+  for (int e0 = tid; e0 < n * n; e0 += kLoads * (int)blockDim.x) {
+    double v[kLoads];
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      const int e = e0 + q * (int)blockDim.x;
+      v[q] = e < n * n ? g[e] : 0.0;
     }
-    warp_argmax_first_key(v, idx);
-    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      const int e = e0 + q * (int)blockDim.x;
+      if (e < n * n) A[(e / n) * ld + e % n] = v[q];
+    }
+  }
+  __syncthreads();
+  int my_info = 0;
+  double x[MB];                        // warp 0: the multipliers of column k
+  // Warp 0: x holds column k, rows > k - 1 after step k - 1.  Finds its pivot,
+  // exchanges rows k and p, scales, and writes the column.
+  auto pivot = [&](int k) {
+    unsigned long long key = 0;        // 1 + |x|'s order, 0: no candidate
+    int p = INT_MAX;
+    double best = 0.0, at_k = 0.0;
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+      const int i = 32 * m + lane;
+      const long long kx = (i >= k && i < n) ? pivot_key(x[m]) : -1;
+      if (kx >= 0 && (unsigned long long)kx + 1 > key) {
+        key = (unsigned long long)kx + 1;
+        p = i;
+        best = x[m];
+      }
+      if (m == (k >> 5)) at_k = x[m];
+    }
+    warp_first_max(key, p);
+    const double old = __shfl_sync(0xffffffffu, at_k, k & 31);
+    const bool found = p != INT_MAX;
+    const double akk = __shfl_sync(0xffffffffu, found ? best : at_k, found ? p & 31 : k & 31);
+    if (!found) p = k;                 // column of NaNs: keep the row
+    const uint32_t hi = (uint32_t)__double2hiint(akk) & 0x7FFFFFFFu;
+    const uint32_t lo = (uint32_t)__double2loint(akk);
+    const bool nz = (hi | lo) != 0;    // NaN included
+    // |akk| >= DBL_MIN (false for NaN)
+    const bool use_recip = hi >= 0x00100000u && (hi < 0x7FF00000u || (hi == 0x7FF00000u && lo == 0));
     if (lane == 0) {
-      if (idx == INT_MAX) idx = k;  // column of NaNs: keep the row
-      const int sl = k & 1;
-      const double akk = A[idx * ld + k];
-      s_p[sl] = idx;
-      s_akk[sl] = akk;
-      s_old[sl] = A[k * ld + k];
-      // the reciprocal once per column (a division is a long FP64 sequence)
-      s_recip[sl] = fabs(akk) >= DBL_MIN;
-      s_rcp[sl] = 1.0 / akk;
-      gp[k] = idx;
+      s_p[k & 1] = nz ? p : k;
+      gp[k] = p;
+    }
+    if (nz) {
+      const double r = 1.0 / akk;
+#pragma unroll
+      for (int m = 0; m < MB; ++m) {
+        if (32 * m + 31 < k || 32 * m >= n) continue;  // uniform
+        const int i = 32 * m + lane;
+        if (i == p) x[m] = old;
+        if (i > k) x[m] = scale_pivot(x[m], akk, r, use_recip);
+        if (i == k) x[m] = akk;
+      }
+    } else if (my_info == 0) {
+      my_info = k + 1;
+    }
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+      const int i = 32 * m + lane;
+      if (i >= k && i < n) A[i * ld + k] = x[m];
     }
   };
-  __syncthreads();
-  if (tid < 32) pivot_warp(0, false);
-  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int m = 0; m < MB; ++m) x[m] = (32 * m + lane < n) ? A[(32 * m + lane) * ld] : 0.0;
+    pivot(0);
+  }
   for (int k = 0; k < n; ++k) {
-    const int sl = k & 1;
-    const int p = s_p[sl];
-    const double akk = s_akk[sl];
-    if ((__double_as_longlong(akk) << 1) != 0) {   // akk != 0 (NaN included), integer test
-      if (p != k) {
-        for (int j = tid; j < n; j += blockDim.x) {
-          if (j == k) continue;
+    __syncthreads();
+    const int p = s_p[k & 1];
+    if (warp == 0) {
+      if (k + 1 < n) {
+        const double uk = A[p * ld + k + 1], ok = A[k * ld + k + 1];
+#pragma unroll
+        for (int m = 0; m < MB; ++m) {
+          if (32 * m + 31 <= k || 32 * m >= n) continue;  // uniform
+          const int i = 32 * m + lane;
+          if (i > k && i < n) x[m] = fma(-x[m], uk, i == p ? ok : A[i * ld + k + 1]);
+        }
+        __syncwarp();
+        if (lane == 0) A[k * ld + k + 1] = uk;
+        pivot(k + 1);
+      }
+    } else {
+      if (p != k) {                    // the multipliers of the columns before
+        for (int j = tid - 32; j < k; j += (int)blockDim.x - 32) {
           const double t = A[k * ld + j];
           A[k * ld + j] = A[p * ld + j];
           A[p * ld + j] = t;
         }
       }
-      const bool use_recip = s_recip[sl] != 0;
-      const double r = s_rcp[sl];
-      if (tid == 0) A[k * ld + k] = akk;
-      for (int i = k + 1 + tid; i < n; i += blockDim.x) {
-        const double v = (i == p) ? s_old[sl] : A[i * ld + k];
-        A[i * ld + k] = scale_pivot(v, akk, r, use_recip);
-      }
-    } else if (my_info == 0) {
-      my_info = k + 1;
+      small_update_n<2 * MB>((n - k - 2 + 15) >> 4, A, ld, n, k, p, k + 2 * warp - 1,
+                             2 * (nwarps - 1), lane, (int)blockDim.x - 32);
     }
-    __syncthreads();
-    if (ty == 0) {
-      // column k + 1 updated and its pivot found while the others update
-      if (k + 1 < n) pivot_warp(k + 1, true);
-    } else {
-      // rank-1 update of columns >= k + 2; u(k,j) cached in registers.  Only
-      // the 32-column chunks that hold trailing columns are visited (a
-      // warp-uniform break): a predicated-off FP64 instruction still occupies
-      // GB300's narrow FP64 pipe.
-      const int nchunk = (n - k - 2 + 31) >> 5;
-      double u[(kSmallMax + 31) / 32];
-#pragma unroll
-      for (int c = 0; c < (kSmallMax + 31) / 32; ++c) {
-        if (c >= nchunk) break;
-        const int j = k + 2 + tx + 32 * c;
-        u[c] = (j < n) ? A[k * ld + j] : 0.0;
-      }
-      for (int i = k + 1 + (ty - 1); i < n; i += kUpdWarps) {
-        const double l = A[i * ld + k];
-#pragma unroll
-        for (int c = 0; c < (kSmallMax + 31) / 32; ++c) {
-          if (c >= nchunk) break;
-          const int j = k + 2 + tx + 32 * c;
-          if (j < n) A[i * ld + j] = fma(-l, u[c], A[i * ld + j]);
-        }
-      }
-    }
-    __syncthreads();
   }
-  for (int e = tid; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e - i * n;
-    g[e] = A[i * ld + j];
+  __syncthreads();
+  for (int e0 = tid; e0 < n * n; e0 += kLoads * (int)blockDim.x) {
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      const int e = e0 + q * (int)blockDim.x;
+      if (e < n * n) g[e] = A[(e / n) * ld + e % n];
+    }
   }
   if (tid == 0) info[b] = my_info;
 }
@@ -870,7 +940,6 @@ int getrf_blocked(int n, double* a, int32_t* piv, int32_t* info, cudaStream_t st
 // getrs for n > kSmallMax: the row interchanges as one gather or scatter per
 // vector, then two multi-CTA triangular solves (trisolve.cu).
 // ---------------------------------------------------------------------------
-constexpr int kSolveThreads = 256;
 constexpr int kPermThreads = 1024;
 constexpr int kPermMaxN = 11000;   // 20 bytes of shared memory per row
 
@@ -968,136 +1037,131 @@ static int getrs_perm(int64_t batch, int n, int nrhs, const int32_t* piv, int64_
 
 // ---------------------------------------------------------------------------
 // getrs for n <= kSmallMax: one CTA per system, the factors staged in shared
-// memory, one warp per right-hand side with x held in registers (lane l owns
-// rows l, l + 32, ...).  Each substitution step broadcasts the finished
-// unknown with a shuffle and updates the later rows with one FMA per lane, so
-// the dependent chain per step is a shuffle and an FMA; the diagonal of U is
-// inverted up front, off that chain (x_t * (1 / u_tt) instead of x_t / u_tt:
-// within one rounding of the quotient).  The row interchanges are composed
-// once into a gather index.
+// memory, one warp per right-hand side and 32 unknowns (lane l of warp m owns
+// row 32 m + l).  A sweep goes by half blocks of 16 unknowns: their warp
+// substitutes (a shuffle and an FMA per unknown; with U also x_t * (1 / u_tt),
+// within one rounding of the quotient, the inverses formed up front), then the
+// other warps subtract them from their rows while it goes on with its second
+// half.  The dependent chain of a step is what bounds it: one warp with all the
+// rows of a right-hand side issues its FMAs for every 32 rows one after the
+// other on GB300's narrow FP64 pipe.  Interchanges: every thread follows one
+// element through the n swaps, all in parallel.
+// Measured (one right-hand side): 16.6 us at n = 48, 37 at 128, 53 at 168, against
+// 29, 72 and 98 with one warp per right-hand side.
 // ---------------------------------------------------------------------------
-constexpr int kSmallRegs = (kSmallMax + 31) / 32;
+constexpr int kSmallRhs = 4;           // right-hand sides at a time
+constexpr int kSmallSolveThreads = 32 * kSmallBlocks * kSmallRhs;
+constexpr int kSmallHalf = 16;
 
-__global__ void __launch_bounds__(kSolveThreads)
-getrs_small_kernel(int n, int nrhs, const double* __restrict__ lu, int64_t stride_a,
+// One sweep over op(T), ascending (FWD) or descending, on the x of this thread
+// (row 32 m + lane, rinv the inverse of its diagonal); op(T)[i][t] is T[t][i]
+// with TR.  xs: the unknowns of two half blocks in turn.
+template <bool FWD, bool UNIT, bool TR>
+__device__ __forceinline__ void small_sweep(int n, int ld, const double* T, double rinv,
+                                            double* xs, int nblk, int m, int lane, bool active,
+                                            double& x) {
+  constexpr int kH = kSmallHalf;
+  const int i = 32 * m + lane;
+  for (int q = 0; q < 2 * nblk; ++q) {
+    const int hb = FWD ? q : 2 * nblk - 1 - q;      // half block: unknowns 16 hb ..
+    const int t0 = kH * hb;
+    if (active && m == (hb >> 1)) {
+      double tv[kH];
+#pragma unroll
+      for (int u = 0; u < kH; ++u) {
+        const int t = FWD ? t0 + u : t0 + kH - 1 - u;
+        const bool use = t < n && i < n && (FWD ? i > t : i < t);
+        tv[u] = use ? (TR ? T[t * ld + i] : T[i * ld + t]) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kH; ++u) {
+        const int t = FWD ? t0 + u : t0 + kH - 1 - u;
+        if (t < n) {
+          if (!UNIT && i == t) x *= rinv;
+          const double xt = __shfl_sync(0xffffffffu, x, t & 31);
+          if (i < n && (FWD ? i > t : i < t)) x = fma(-tv[u], xt, x);
+        }
+      }
+      if ((i >> 4) == hb) xs[kH * (q & 1) + (i & (kH - 1))] = x;
+    }
+    __syncthreads();
+    if (active && i < n && (FWD ? m > (hb >> 1) : m < (hb >> 1))) {
+      double tv[kH];
+#pragma unroll
+      for (int u = 0; u < kH; ++u) {
+        const int t = FWD ? t0 + u : t0 + kH - 1 - u;
+        tv[u] = t < n ? (TR ? T[t * ld + i] : T[i * ld + t]) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kH; ++u) {
+        const int t = FWD ? t0 + u : t0 + kH - 1 - u;
+        if (t < n) x = fma(-tv[u], xs[kH * (q & 1) + (t & (kH - 1))], x);
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kSmallSolveThreads)
+getrs_small_kernel(int n, int nrhs, int per, const double* __restrict__ lu, int64_t stride_a,
                    const int32_t* __restrict__ piv, int64_t stride_piv, double* __restrict__ b,
                    int64_t stride_b, int trans) {
   extern __shared__ double smem_x[];
   const int ld = n | 1;
+  const int nblk = (n + 31) >> 5;
   double* T = smem_x;                                   // n × ld
   double* rinv = T + (int64_t)n * ld;                   // 1 / u_tt
-  int* perm = reinterpret_cast<int*>(rinv + n);         // x_perm[i] = b[perm[i]]
+  double* xs = rinv + n;                                // finished unknowns, by right-hand side
+  int* perm = reinterpret_cast<int*>(xs + per * 2 * kSmallHalf);  // x_perm[i] = b[perm[i]]
+  int* sp = perm + n;                                   // the interchanges
   const int sys = blockIdx.x;
   const double* A = lu + (int64_t)sys * stride_a;
   const int32_t* P = piv + (int64_t)sys * stride_piv;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  for (int e = tid; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e - i * n;
-    T[i * ld + j] = A[e];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < n; i += blockDim.x) sp[i] = P[i];
+  constexpr int kLoads = 8;
+  for (int e0 = tid; e0 < n * n; e0 += kLoads * blockDim.x) {
+    double v[kLoads];
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int e = e0 + u * (int)blockDim.x;
+      v[u] = e < n * n ? A[e] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int e = e0 + u * (int)blockDim.x;
+      if (e < n * n) T[(e / n) * ld + e % n] = v[u];
+    }
   }
-  if (tid == 0) {
-    // compose the interchanges: forward order for P b, and its inverse is
-    // applied by scattering through the same index for Pᵀ y
-    for (int i = 0; i < n; ++i) perm[i] = i;
+  __syncthreads();
+  for (int i = tid; i < n; i += blockDim.x) {
+    int pos = i;                       // where element i is after the swaps
+#pragma unroll 8
     for (int k = 0; k < n; ++k) {
-      const int p = P[k];
-      if (p != k) { const int t = perm[k]; perm[k] = perm[p]; perm[p] = t; }
+      const int p = sp[k];
+      pos = pos == k ? p : (pos == p ? k : pos);
     }
+    perm[pos] = i;
+    rinv[i] = 1.0 / T[i * ld + i];
   }
   __syncthreads();
-  for (int i = tid; i < n; i += blockDim.x) rinv[i] = 1.0 / T[i * ld + i];
-  __syncthreads();
-  for (int rr = warp; rr < nrhs; rr += nw) {
-    double* g = b + (int64_t)sys * stride_b + (int64_t)rr * n;
-    double x[kSmallRegs];
+  const int rg = warp / nblk, m = warp - rg * nblk, i = 32 * m + lane;
+  const double ri = i < n ? rinv[i] : 0.0;
+  for (int r0 = 0; r0 < nrhs; r0 += per) {
+    const bool active = rg < per && r0 + rg < nrhs;
+    double* g = b + (int64_t)sys * stride_b + (int64_t)(r0 + rg) * n;
+    double* mine = xs + (active ? rg : 0) * 2 * kSmallHalf;
+    double x = 0.0;
+    if (active && i < n) x = g[trans ? i : perm[i]];
+    // every element is read before the first is written
+    __syncthreads();
     if (!trans) {
-#pragma unroll
-      for (int m = 0; m < kSmallRegs; ++m) {
-        const int i = 32 * m + lane;
-        x[m] = (i < n) ? g[perm[i]] : 0.0;
-      }
-      // L y = P b (unit lower): column t of L is read down the rows
-#pragma unroll
-      for (int tb = 0; tb < kSmallRegs; ++tb) {
-        if (32 * tb >= n) break;
-        for (int tt = 0; tt < 32; ++tt) {
-          const int t = 32 * tb + tt;
-          if (t >= n) break;
-          const double xt = __shfl_sync(0xffffffffu, x[tb], tt);
-#pragma unroll
-          for (int m = tb; m < kSmallRegs; ++m) {
-            const int i = 32 * m + lane;
-            if (i > t && i < n) x[m] = fma(-T[i * ld + t], xt, x[m]);
-          }
-        }
-      }
-      // U x = y
-#pragma unroll
-      for (int tb = kSmallRegs - 1; tb >= 0; --tb) {
-        if (32 * tb >= n) continue;
-        for (int tt = 31; tt >= 0; --tt) {
-          const int t = 32 * tb + tt;
-          if (t >= n) continue;
-          if (lane == tt) x[tb] *= rinv[t];
-          const double xt = __shfl_sync(0xffffffffu, x[tb], tt);
-#pragma unroll
-          for (int m = 0; m <= tb; ++m) {
-            const int i = 32 * m + lane;
-            if (i < t) x[m] = fma(-T[i * ld + t], xt, x[m]);
-          }
-        }
-      }
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < kSmallRegs; ++m) {
-        const int i = 32 * m + lane;
-        if (i < n) g[i] = x[m];
-      }
+      small_sweep<true, true, false>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // L y = P b
+      small_sweep<false, false, false>(n, ld, T, ri, mine, nblk, m, lane, active, x); // U x = y
     } else {
-#pragma unroll
-      for (int m = 0; m < kSmallRegs; ++m) {
-        const int i = 32 * m + lane;
-        x[m] = (i < n) ? g[i] : 0.0;
-      }
-      // Uᵀ z = b: column t of Uᵀ is row t of U
-#pragma unroll
-      for (int tb = 0; tb < kSmallRegs; ++tb) {
-        if (32 * tb >= n) break;
-        for (int tt = 0; tt < 32; ++tt) {
-          const int t = 32 * tb + tt;
-          if (t >= n) break;
-          if (lane == tt) x[tb] *= rinv[t];
-          const double xt = __shfl_sync(0xffffffffu, x[tb], tt);
-#pragma unroll
-          for (int m = tb; m < kSmallRegs; ++m) {
-            const int i = 32 * m + lane;
-            if (i > t && i < n) x[m] = fma(-T[t * ld + i], xt, x[m]);
-          }
-        }
-      }
-      // Lᵀ w = z (unit upper)
-#pragma unroll
-      for (int tb = kSmallRegs - 1; tb >= 0; --tb) {
-        if (32 * tb >= n) continue;
-        for (int tt = 31; tt >= 0; --tt) {
-          const int t = 32 * tb + tt;
-          if (t >= n) continue;
-          const double xt = __shfl_sync(0xffffffffu, x[tb], tt);
-#pragma unroll
-          for (int m = 0; m <= tb; ++m) {
-            const int i = 32 * m + lane;
-            if (i < t) x[m] = fma(-T[t * ld + i], xt, x[m]);
-          }
-        }
-      }
-      // x = Pᵀ w: x[perm[i]] = w[i]
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < kSmallRegs; ++m) {
-        const int i = 32 * m + lane;
-        if (i < n) g[perm[i]] = x[m];
-      }
+      small_sweep<true, false, true>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // Uᵀ z = b
+      small_sweep<false, true, true>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // Lᵀ w = z
     }
+    if (active && i < n) g[trans ? perm[i] : i] = x;    // x = Pᵀ w: x[perm[i]] = w[i]
   }
 }
 
@@ -1137,11 +1201,18 @@ extern "C" int lxgb_getrf_batched_f64(int64_t batch, int32_t n, double* a, int64
   }
   if (n <= kSmallMax) {
     const size_t smem = (size_t)n * (n | 1) * sizeof(double);
-    LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(getrf_small_kernel), (int)smem),
+    // More warps where the update is the longer part: us per matrix with 256 and
+    // 512 threads 14.6 and 16.6 at n = 16, 47 and 47 at 48, 191 and 176 at 100, 317
+    // and 289 at 128; 512 matrices of order 64 156 and 187.
+    const int threads = n <= 64 ? kSmallThreads : kSmallMaxThreads;
+    // registers for the rows of a column per lane of warp 0
+    auto fn = n <= 64 ? getrf_small_kernel<2>
+                      : (n <= 128 ? getrf_small_kernel<4> : getrf_small_kernel<kSmallBlocks>);
+    LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(fn), (int)smem),
                   "getrf: set smem");
     for (int64_t off = 0; off < batch; off += 65535LL * 1024) {
       const int64_t cnt = (batch - off < 65535LL * 1024) ? batch - off : 65535LL * 1024;
-      getrf_small_kernel<<<(unsigned)cnt, kSmallThreads, smem, st>>>(
+      fn<<<(unsigned)cnt, threads, smem, st>>>(
           n, a + off * stride_a, stride_a, piv + off * stride_piv, stride_piv, info + off);
     }
     return check_launch("getrf small");
@@ -1164,12 +1235,16 @@ extern "C" int lxgb_getrs_batched_f64(int64_t batch, int32_t n, int32_t nrhs, co
                "getrs: stride too small");
   LXGB_REQUIRE(batch * (int64_t)nrhs < (1LL << 31), "getrs: too many vectors in one call");
   if (n <= kSmallMax && batch < (1LL << 31)) {
+    const int per = nrhs < kSmallRhs ? nrhs : kSmallRhs;
     const size_t smem = (size_t)n * (n | 1) * sizeof(double) + (size_t)n * sizeof(double) +
-                        (size_t)n * sizeof(int32_t);
+                        (size_t)per * 2 * kSmallHalf * sizeof(double) +
+                        (size_t)n * 2 * sizeof(int32_t);
+    const int warps = (n + 31) / 32 * per;
+    const int threads = 32 * (warps < 8 ? 8 : warps);
     LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(getrs_small_kernel), (int)smem),
                   "getrs small: set smem");
-    getrs_small_kernel<<<(unsigned)batch, kSolveThreads, smem, as_stream(stream)>>>(
-        n, nrhs, lu, stride_a, piv, stride_piv, b, stride_b, trans);
+    getrs_small_kernel<<<(unsigned)batch, threads, smem, as_stream(stream)>>>(
+        n, nrhs, per, lu, stride_a, piv, stride_piv, b, stride_b, trans);
     return check_launch("getrs small");
   }
   cudaStream_t st = as_stream(stream);
