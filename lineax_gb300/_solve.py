@@ -177,6 +177,8 @@ def _any_nonfinite(tree) -> bool:
     flags = [_blas.any_nonfinite(x) for x in leaves if x.numel() > 0]
     if not flags:
         return False
+    if len(flags) == 1:
+        return flags[0].item() != 0
     return bool(torch.cat(flags).any().item())
 
 
