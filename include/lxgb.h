@@ -548,7 +548,7 @@ int lxgb_getrf_f32_tc(int32_t n, const double* a64, float* lu, int32_t* piv,
  * its upper triangle as lineax's cho_factor(lower=False) reads it; n % 4 == 0,
  * n < 32768) for mixed-precision refinement: l (n×n FP32, 16-byte aligned)
  * receives L in its lower triangle (the upper triangle is scratch).  64-column
- * panels: the diagonal block factored by one CTA, the panel below it by FP32
+ * panels: the diagonal block and the panel below it in one launch, by FP32
  * substitution (one row per thread), the trailing update on the tiles of the
  * lower triangle as a tcgen05 GEMM with 3xTF32 products.  *info = 0, or the 1-based index of the first pivot that is not
  * positive in FP32 (the factor is then unusable); *err is set if a tensor-core
@@ -661,7 +661,8 @@ int lxgb_geqrf_f32_tc(int64_t m, int64_t n, const double* a, float* h, float* ta
 /* lxgb_geqrf_f32_tc that also forms Q explicitly: the reflectors are applied
  * to the m×m identity in the same tensor-core trailing updates, leaving q
  * (m×m FP32 row-major, 16-byte aligned) = Q with A = Q [R; 0].  `work`:
- * lxgb_geqrf_f32_tc_q_workspace_size(m, n) bytes.  With the triangular
+ * lxgb_geqrf_f32_tc_q_workspace_size(m, n) bytes.  Faster with q = h + n*m (q
+ * right after h), which shares h's updates.  With the triangular
  * inverse of R (lxgb_lu32_inverse on R with identity pivots) it gives the
  * square-system preconditioner M = R^{-1} Qᵀ of lxgb_qr32_apply: the
  * low-precision QR factor of a mixed-precision square solve (lineax's QR

@@ -3,9 +3,8 @@
 // the ragged kernel's order limit):
 //
 //   lxgb_potrf_f32_tc  — A = L Lᵀ in FP32, right-looking by 64-column panels:
-//     the 64×64 diagonal block factored by one CTA in shared memory, the
-//     panel below it L21 = A21 L_jj⁻ᵀ by FP32 substitution on the CUDA cores
-//     (one row per thread), and the trailing update A22 -= L21 L21ᵀ
+//     the 64×64 diagonal block and the panel below it L21 = A21 L_jj⁻ᵀ in one
+//     launch (FP32 on the CUDA cores), and the trailing update A22 -= L21 L21ᵀ
 //     (lower-triangle tiles only) as a tcgen05 GEMM with 3xTF32 products
 //     (FP32-level accuracy).  A is read from its upper triangle, as
 //     lineax's Cholesky reads it (cho_factor(lower=False),
@@ -41,99 +40,183 @@ __global__ void c32_lower_from_upper_kernel(int64_t n, const double* __restrict_
   }
 }
 
-// Factor the nb×nb diagonal block at (j0, j0) of l (lower triangle) in
-// shared memory with 256 threads: per column one thread takes the square
-// root, the rows below divide by it, and the rank-1 update of the trailing
-// lower triangle is spread over all threads element by element.  The first
-// pivot that is not positive is recorded in *info (1-based, global index) and
-// replaced by 1 so that the launch finishes.
-constexpr int kC32DiagThreads = 256;
+// One block column: the 64×64 diagonal block at (j0, j0) of l (nb×nb at the
+// end) factored, and the rows below it L21 = A21 L_jj⁻ᵀ, 128 per CTA, one per
+// thread.  Every CTA factors the block for itself (its own copy; CTA 0 stores it
+// in diag, from where c32_store_diag_kernel takes it at the end — a CTA that
+// starts late still reads the block unfactored).
+//  * Factor: row tid & 63 in the registers of two threads, which hold the even
+//    and the odd columns.  Columns in registers are kept shifted, element 0 being
+//    the next column of its parity, so one loop body serves all 64: the owners
+//    publish the raw column, each takes the root, the owners divide, and all
+//    apply the rank-1 update.  A pivot that is not positive counts as 1; the
+//    first is recorded in *info (1-based, global).
+//  * Rows: 16 columns at a time in registers, as one body for the product with a
+//    16×16 block and one for the triangle.  L21 goes back into l and, split into
+//    TF32-exact hi and lo parts, into ph / pl (row stride 64).
+// Bound by the two chains of 64 steps (a root, a division and two barriers; a
+// division).  Measured per block column: @C@
+constexpr int kC32Threads = 128;
+constexpr int kC32T = 16;
+constexpr int kC32TLd = kC32NB + 4;
+constexpr int kC32XLd = kC32NB + 1;
+constexpr int kC32Smem = (kC32NB * kC32TLd + kC32Threads * kC32XLd) * (int)sizeof(float);
 
-__global__ void __launch_bounds__(kC32DiagThreads)
-c32_diag_kernel(int64_t n, int64_t j0, int nb, float* __restrict__ l, int32_t* __restrict__ info) {
-  __shared__ float T[kC32NB][kC32NB + 1];
-  __shared__ int s_bad;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < kC32NB * kC32NB; e += kC32DiagThreads) {
-    const int i = e / kC32NB, c = e % kC32NB;
-    T[i][c] = (i < nb && c <= i) ? l[(j0 + i) * n + j0 + c] : 0.0f;
+__global__ void __launch_bounds__(kC32Threads)
+c32_row_kernel(int64_t n, int64_t j0, int nb, int m2, float* __restrict__ l,
+               float* __restrict__ diag, float* __restrict__ ph, float* __restrict__ pl,
+               int32_t* __restrict__ info) {
+  extern __shared__ __align__(16) float c32_smem[];
+  float (*Tt)[kC32TLd] = reinterpret_cast<float (*)[kC32TLd]>(c32_smem);  // Tt[k][i] = L[i][k]
+  float (*X)[kC32XLd] = reinterpret_cast<float (*)[kC32XLd]>(c32_smem + kC32NB * kC32TLd);
+  // the raw and the scaled column, alternating with the column's parity; the
+  // scaled one by parity of the row, from the current pair of columns on
+  __shared__ __align__(16) float raw[2][kC32NB], col[2][2][kC32NB / 2];
+  constexpr int kLoads = 32;
+  const int tid = threadIdx.x, i = tid & (kC32NB - 1), h = tid >> 6;
+  const int64_t rbase = (int64_t)blockIdx.x * kC32Threads;  // first row below the block
+  {
+    float v[kLoads];
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int e = tid + u * kC32Threads, r = e / kC32NB, c = e % kC32NB;
+      v[u] = (r < nb && c <= r) ? l[(j0 + r) * n + j0 + c] : (r == c ? 1.0f : 0.0f);
+    }
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int e = tid + u * kC32Threads;
+      X[e / kC32NB][e % kC32NB] = v[u];
+    }
   }
-  if (tid == 0) s_bad = 0;
   __syncthreads();
-  for (int k = 0; k < nb; ++k) {
-    if (tid == 0) {
-      float d = T[k][k];
+  float r[kC32NB / 2];
+#pragma unroll
+  for (int j = 0; j < kC32NB / 2; ++j) r[j] = X[i][2 * j + h];
+  // the rows below, on their way while the block is factored
+  float a[kLoads];
+#pragma unroll
+  for (int u = 0; u < kLoads; ++u) {
+    const int e = tid + u * kC32Threads, rr = e / kC32NB, c = e % kC32NB;
+    a[u] = (rbase + rr < m2) ? l[(j0 + kC32NB + rbase + rr) * n + j0 + c] : 0.0f;
+  }
+  int bad = 0;
+#pragma unroll 1
+  for (int kk = 0; kk < kC32NB / 2; ++kk) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int k = 2 * kk + q;
+      if (h == q) raw[q][i] = r[0];
+      __syncthreads();
+      float d = raw[q][k];
       if (!(d > 0.0f)) {
-        if (s_bad == 0) s_bad = k + 1;
+        if (bad == 0) bad = k + 1;
         d = 1.0f;
       }
-      T[k][k] = sqrtf(d);
+      const float s = sqrtf(d);
+      if (h == q && i >= k) {
+        const float v = (i == k) ? s : r[0] / s;
+        Tt[k][i] = v;
+        col[q][i & 1][(i >> 1) - kk] = v;
+      }
+      __syncthreads();
+      const float li = (i > k) ? col[q][i & 1][(i >> 1) - kk] : 0.0f;
+      const float4* cq = reinterpret_cast<const float4*>(col[q][h]);
+#pragma unroll
+      for (int j4 = 0; j4 < kC32NB / 8; ++j4) {
+        const float4 t = cq[j4];
+        const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const int j = 4 * j4 + w;
+          // columns 2 (kk + j) + h > k; rows above the diagonal hold nothing
+          if (q == 0) {
+            if (j > 0 || h == 1) r[j] = (i > k) ? fmaf(-li, tv[w], r[j]) : 0.0f;
+          } else if (j > 0) {
+            r[j - 1] = (i > k) ? fmaf(-li, tv[w], r[j]) : 0.0f;
+          }
+        }
+      }
     }
-    __syncthreads();
-    const float s = T[k][k];
-    for (int i = k + 1 + tid; i < nb; i += kC32DiagThreads) T[i][k] = T[i][k] / s;
-    __syncthreads();
-    const int w = nb - k - 1;
-    for (int e = tid; e < w * w; e += kC32DiagThreads) {
-      const int i = k + 1 + e / w, c = k + 1 + e % w;
-      if (c <= i) T[i][c] = fmaf(-T[i][k], T[c][k], T[i][c]);
+  }
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    float* dst = diag + j0 * kC32NB;
+    for (int e = tid; e < kC32NB * kC32NB; e += kC32Threads) {
+      const int rr = e / kC32NB, c = e % kC32NB;
+      if (rr < nb && c <= rr) dst[e] = Tt[c][rr];
     }
-    __syncthreads();
+    if (tid == 0 && bad) atomicCAS(reinterpret_cast<int*>(info), 0, (int)(j0 + bad));
   }
-  for (int e = tid; e < nb * nb; e += kC32DiagThreads) {
-    const int i = e / nb, c = e % nb;
-    if (c <= i) l[(j0 + i) * n + j0 + c] = T[i][c];
+  if (m2 <= 0) return;
+  // (the block's copy in X was read before the first barrier of the factor)
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    if (g == 1) {
+#pragma unroll
+      for (int u = 0; u < kLoads; ++u) {
+        const int e = tid + (u + kLoads) * kC32Threads, rr = e / kC32NB, c = e % kC32NB;
+        a[u] = (rbase + rr < m2) ? l[(j0 + kC32NB + rbase + rr) * n + j0 + c] : 0.0f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+      const int e = tid + (u + g * kLoads) * kC32Threads;
+      X[e / kC32NB][e % kC32NB] = a[u];
+    }
   }
-  if (tid == 0 && s_bad) atomicCAS(reinterpret_cast<int*>(info), 0, (int)(j0 + s_bad));
+  __syncthreads();
+#pragma unroll 1
+  for (int bi = 0; bi < kC32NB / kC32T; ++bi) {
+    const int i0 = bi * kC32T;
+    float x[kC32T];
+#pragma unroll
+    for (int c = 0; c < kC32T; ++c) x[c] = X[tid][i0 + c];
+#pragma unroll 1
+    for (int k0 = 0; k0 < i0; k0 += kC32T) {
+#pragma unroll
+      for (int k = 0; k < kC32T; ++k) {
+        const float xk = X[tid][k0 + k];
+#pragma unroll
+        for (int c4 = 0; c4 < kC32T / 4; ++c4) {
+          const float4 t = *reinterpret_cast<const float4*>(&Tt[k0 + k][i0 + 4 * c4]);
+          x[4 * c4 + 0] = fmaf(-xk, t.x, x[4 * c4 + 0]);
+          x[4 * c4 + 1] = fmaf(-xk, t.y, x[4 * c4 + 1]);
+          x[4 * c4 + 2] = fmaf(-xk, t.z, x[4 * c4 + 2]);
+          x[4 * c4 + 3] = fmaf(-xk, t.w, x[4 * c4 + 3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kC32T; ++k) {
+      x[k] = x[k] / Tt[i0 + k][i0 + k];
+#pragma unroll
+      for (int c = k + 1; c < kC32T; ++c) x[c] = fmaf(-x[k], Tt[i0 + k][i0 + c], x[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < kC32T; ++c) X[tid][i0 + c] = x[c];
+  }
+  __syncthreads();
+#pragma unroll 16
+  for (int u = 0; u < 2 * kLoads; ++u) {
+    const int e = tid + u * kC32Threads, rr = e / kC32NB, c = e % kC32NB;
+    const int64_t pr = rbase + rr;
+    if (pr < m2) {
+      const float x = X[rr][c];
+      const float hi = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
+      l[(j0 + kC32NB + pr) * n + j0 + c] = x;
+      ph[pr * kC32NB + c] = hi;
+      pl[pr * kC32NB + c] = x - hi;
+    }
+  }
 }
 
-// The panel below the diagonal block: L21 = A21 L_jj⁻ᵀ by forward
-// substitution on the CUDA cores (FP32), one row per thread with the row in
-// registers, 96 rows per CTA staged through shared memory for coalesced
-// loads and stores; L21 goes back into l and, split into TF32-exact hi and lo
-// parts, into ph / pl (row stride 64) for the trailing update.
-constexpr int kC32Rows = 96;
-
-__global__ void __launch_bounds__(kC32Rows)
-c32_panel_kernel(int64_t n, int64_t j0, int m2, float* __restrict__ l, float* __restrict__ ph,
-                 float* __restrict__ pl) {
-  __shared__ float L[kC32NB][kC32NB];            // read as broadcasts: no padding
-  __shared__ float X[kC32Rows][kC32NB + 1];       // row per thread: padded
-  const int t = threadIdx.x;
-  const int64_t rbase = (int64_t)blockIdx.x * kC32Rows;      // first panel row of this CTA
-  for (int e = t; e < kC32NB * kC32NB; e += kC32Rows) {
-    const int r = e / kC32NB, c = e % kC32NB;
-    L[r][c] = (c <= r) ? l[(j0 + r) * n + j0 + c] : 0.0f;
-  }
-  for (int e = t; e < kC32Rows * kC32NB; e += kC32Rows) {
-    const int r = e / kC32NB, c = e % kC32NB;
-    const int64_t pr = rbase + r;
-    X[r][c] = (pr < m2) ? l[(j0 + kC32NB + pr) * n + j0 + c] : 0.0f;
-  }
-  __syncthreads();
-  float a[kC32NB];
-#pragma unroll
-  for (int c = 0; c < kC32NB; ++c) a[c] = X[t][c];
-#pragma unroll
-  for (int k = 0; k < kC32NB; ++k) {
-    const float x = a[k] / L[k][k];
-    a[k] = x;
-#pragma unroll
-    for (int j = k + 1; j < kC32NB; ++j) a[j] = fmaf(-x, L[j][k], a[j]);
-  }
-#pragma unroll
-  for (int c = 0; c < kC32NB; ++c) X[t][c] = a[c];
-  __syncthreads();
-  for (int e = t; e < kC32Rows * kC32NB; e += kC32Rows) {
-    const int r = e / kC32NB, c = e % kC32NB;
-    const int64_t pr = rbase + r;
-    if (pr < m2) {
-      const float x = X[r][c];
-      const float h = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-      l[(j0 + kC32NB + pr) * n + j0 + c] = x;
-      ph[pr * kC32NB + c] = h;
-      pl[pr * kC32NB + c] = x - h;
-    }
+// The factored diagonal blocks (64×64 each, lower triangles) into l.
+__global__ void c32_store_diag_kernel(int64_t n, const float* __restrict__ diag,
+                                      float* __restrict__ l) {
+  const int64_t j0 = (int64_t)blockIdx.x * kC32NB;
+  for (int e = threadIdx.x; e < kC32NB * kC32NB; e += blockDim.x) {
+    const int64_t r = e / kC32NB, c = e % kC32NB;
+    if (c <= r && j0 + r < n) l[(j0 + r) * n + j0 + c] = diag[j0 * kC32NB + e];
   }
 }
 
@@ -195,7 +278,9 @@ using namespace lxgb;
 
 extern "C" int64_t lxgb_potrf_f32_tc_workspace_size(int64_t n) {
   const int64_t panel = (n > 0 ? n : 1) * kC32NB * 4;
-  return 256 + 2 * ((panel + 255) / 256 * 256);
+  // two panels and the factored diagonal blocks
+  const int64_t diag = (panel / 4 + kC32NB * kC32NB) * 4;
+  return 256 + 2 * ((panel + 255) / 256 * 256) + (diag + 255) / 256 * 256;
 }
 
 extern "C" int lxgb_potrf_f32_tc(int64_t n, const double* a, float* l, int32_t* info,
@@ -218,19 +303,23 @@ extern "C" int lxgb_potrf_f32_tc(int64_t n, const double* a, float* l, int32_t* 
   char* wb = reinterpret_cast<char*>(work) + 256;
   float* ph = reinterpret_cast<float*>(wb);
   float* pl = reinterpret_cast<float*>(wb + panel);
+  float* diag = reinterpret_cast<float*>(wb + 2 * panel);
+  LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(c32_row_kernel), kC32Smem),
+                "potrf_f32_tc: set smem");
   for (int64_t j0 = 0; j0 < n; j0 += kC32NB) {
     const int nb = (int)(n - j0 < kC32NB ? n - j0 : kC32NB);
-    c32_diag_kernel<<<1, kC32DiagThreads, 0, st>>>(n, j0, nb, l, info);
-    const int m2 = (int)(n - j0 - nb);
-    if (m2 <= 0) break;          // only the last block is narrower than 64
-    c32_panel_kernel<<<(unsigned)((m2 + kC32Rows - 1) / kC32Rows), kC32Rows, 0, st>>>(
-        n, j0, m2, l, ph, pl);
+    const int m2 = (int)(n - j0 - nb);   // only the last block is narrower than 64
+    const int ctas = m2 > 0 ? (m2 + kC32Threads - 1) / kC32Threads : 1;
+    c32_row_kernel<<<(unsigned)ctas, kC32Threads, kC32Smem, st>>>(n, j0, nb, m2, l, diag, ph, pl,
+                                                                  info);
+    if (m2 <= 0) break;
     // A22 -= L21 L21ᵀ (3xTF32) on the tiles holding A22's lower triangle
     const int64_t r0 = j0 + kC32NB;
     const int rc = gemm_tf32_nt_split_lower(m2, kC32NB, ph, pl, kC32NB, l + r0 * n + r0, n,
                                             -1.0f, 1.0f, err, st);
     if (rc) return rc;
   }
+  c32_store_diag_kernel<<<(unsigned)((n + kC32NB - 1) / kC32NB), 256, 0, st>>>(n, diag, l);
   return check_launch("potrf_f32_tc");
 }
 

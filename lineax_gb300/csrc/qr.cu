@@ -1302,7 +1302,9 @@ namespace lxgb {
 // FP32 Householder QR with tcgen05 TF32 trailing updates.  With q != nullptr
 // the reflectors are also applied to the columns of the m×m identity held as
 // the rows of q (the same two GEMMs per panel, on m rows instead of the
-// trailing n2), so q ends as Q in row-major order (row j = Qᵀ e_j).
+// trailing n2), so q ends as Q in row-major order (row j = Qᵀ e_j).  A q that
+// follows h in memory (q = h + n m) shares the products of h's trailing rows:
+// half as many launches, and all but 64 rows beside the next panel.
 static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, float* tau,
                                float* t, float* q, int32_t* err, void* work, int64_t work_bytes,
                                const char* who, cudaStream_t st) {
@@ -1315,7 +1317,8 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
   LXGB_REQUIRE((((uintptr_t)h) & 15) == 0 && (((uintptr_t)work) & 255) == 0,
                "geqrf_f32_tc: h must be 16-byte and work 256-byte aligned");
   LXGB_REQUIRE(q == nullptr || (((uintptr_t)q) & 15) == 0, "geqrf_f32_tc: q must be 16-byte aligned");
-  const int64_t rows_w = q ? m : n;  // rows a trailing update may cover
+  const bool joint = q != nullptr && q == h + n * m;
+  const int64_t rows_w = q ? m + n : n;  // rows a trailing update may cover
   if (work_bytes < lxgb_geqrf_f32_tc_workspace_size(m, rows_w)) {
     set_last_error("%s: workspace too small", who);
     return LXGB_WORKSPACE_TOO_SMALL;
@@ -1357,7 +1360,9 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
     qr32_wt_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(rows, nb, used, wpart, Tp, w2);
     return update(c, 0, now, j0, nb, false);
   };
-  const bool ahead = q == nullptr;  // (w2 is one workspace: with q it is taken at once)
+  // (w2 is one workspace: with a separate q it is taken at once)
+  const bool ahead = q == nullptr || joint;
+  const int tail = joint ? (int)m : 0;   // rows after h's
   for (int j0 = 0; j0 < nn; j0 += kQrNB) {
     const int nb = min(kQrNB, nn - j0);
     float* Tp = t + (int64_t)(j0 / kQrNB) * kQrNB * kQrNB;
@@ -1372,15 +1377,16 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
       qr32_make_v_kernel<<<(unsigned)((tot + 255) / 256 < 4096 ? (tot + 255) / 256 : 4096), 256,
                            0, st>>>(m, j0, nb, h, vrows, vcols);
     }
-    // the rows of h after this panel take the panel before beside it (16384 x
-    // 2048: 64 updates of 40 us and 64 panels of 86, least squares 13.4 -> 11.5 ms)
+    // the rows after this panel take the panel before beside it (16384 x 2048: 64
+    // updates of 40 us and 64 panels of 86, least squares 13.4 -> 11.5 ms)
     int rc = 0;
-    if (ahead && j0 > 0 && n2 > 0)
-      rc = update(h + (int64_t)(j0 + nb) * m, kQrNB, n2, j0 - kQrNB, kQrNB, true);
-    // trailing rows of h: with `ahead` the next panel's now, the others beside it
-    if (!rc && n2 > 0)
-      rc = apply(h + (int64_t)(j0 + nb) * m, n2, ahead ? min(kQrNB, n2) : n2, j0, nb, Tp);
-    if (!rc && q) rc = apply(q, (int)m, (int)m, j0, nb, Tp);
+    float* rest = h + (int64_t)(j0 + nb) * m;
+    if (ahead && j0 > 0 && n2 + tail > 0)
+      rc = update(rest, nb, n2 + tail, j0 - kQrNB, kQrNB, true);
+    // trailing rows: with `ahead` the next panel's now, the others beside it
+    if (!rc && n2 + tail > 0)
+      rc = apply(rest, n2 + tail, ahead && n2 > 0 ? min(kQrNB, n2) : n2 + tail, j0, nb, Tp);
+    if (!rc && q && !joint) rc = apply(q, (int)m, (int)m, j0, nb, Tp);
     if (rc) return rc;
   }
   return check_launch(who);
@@ -1396,8 +1402,7 @@ extern "C" int lxgb_geqrf_f32_tc(int64_t m, int64_t n, const double* a, float* h
 }
 
 extern "C" int64_t lxgb_geqrf_f32_tc_q_workspace_size(int64_t m, int64_t n) {
-  (void)n;
-  return lxgb_geqrf_f32_tc_workspace_size(m, m);
+  return lxgb_geqrf_f32_tc_workspace_size(m, m + n);
 }
 
 extern "C" int lxgb_geqrf_f32_tc_q(int64_t m, int64_t n, const double* a, float* h, float* tau,

@@ -698,10 +698,10 @@ def qr_square_tf32(a: torch.Tensor, err: torch.Tensor | None = None) -> SquareQR
         raise ValueError("qr_square_tf32 needs a square matrix with n a multiple of 4")
     dev = a64.device
     lib = _ffi.load()
-    h = torch.empty((n, n), dtype=torch.float32, device=dev)
+    # q right after h: their updates share the products
+    h, q = torch.empty((2, n, n), dtype=torch.float32, device=dev)
     tau = torch.empty(n, dtype=torch.float32, device=dev)
     t = torch.empty(max(1, int(lib.lxgb_geqrf_t_elems(n))), dtype=torch.float32, device=dev)
-    q = torch.empty((n, n), dtype=torch.float32, device=dev)
     err, check = _pipeline_err(err, dev)
     wbytes = int(lib.lxgb_geqrf_f32_tc_q_workspace_size(n, n))
     work = torch.empty(wbytes // 8 + 1, dtype=torch.float64, device=dev)
