@@ -55,7 +55,8 @@ __global__ void c32_lower_from_upper_kernel(int64_t n, const double* __restrict_
 //    16×16 block and one for the triangle.  L21 goes back into l and, split into
 //    TF32-exact hi and lo parts, into ph / pl (row stride 64).
 // Bound by the two chains of 64 steps (a root, a division and two barriers; a
-// division).  Measured per block column: @C@
+// division).  Measured per block column at n = 2048, with the update: 44 us (102
+// with the block in one CTA and the panel in a launch of its own).
 constexpr int kC32Threads = 128;
 constexpr int kC32T = 16;
 constexpr int kC32TLd = kC32NB + 4;

@@ -120,10 +120,11 @@ syrk_f64_kernel(int trans, int64_t n, int64_t k, const double* __restrict__ a, i
 // scale row k of the CTA's columns and update their rows; the owners of rows
 // k + 1 and k + 2 pass on through shared memory what the next step reads.
 // (Warp 4 shares warp 0's sub-partition and stays out of its way.)  What
-// bounds it is warp 0's chain (square root, division, scaling, FMA: 1600
-// cycles a row).  Measured, n = 1531: 27 to 31 us a block row of 32; a block
+// bounds it is warp 0's chain (reciprocal square root, scaling, a barrier, FMA).
+// Measured, n = 1531: 24 to 30 us a block row of 32 (27 to 31 with a square root
+// and a division in the chain); a block
 // row of 64 as a diagonal kernel (138 us) and a column-per-thread substitution
-// (149 us) before.  The whole factorisation 8.4 to 2.3 ms.
+// (149 us) before.  The whole factorisation 8.4 to 2.2 ms.
 // The operations on each element, and their order, are cta_potrf_upper's:
 // row k scaled by 1 / sqrt(a_kk), then one FMA per later row, k ascending.
 constexpr int kPoOwners = 6;
@@ -171,8 +172,8 @@ potrf_row_kernel(int64_t n, double* __restrict__ a, int64_t lda, int64_t j0, int
     if (warp == 0) {
       const double akk = __shfl_sync(0xffffffffu, v, k);
       if (!(akk > 0.0) && bad == 0) bad = k + 1;
-      const double d = sqrt(akk);
-      const double r = 1.0 / d;
+      double d, r;
+      potrf_pivot(akk, d, r);
       u = (lane > k) ? v * r : (lane == k ? d : 0.0);
       U[k][lane] = u;
       if (lane == 0) s_r[par] = r;
