@@ -77,22 +77,6 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// Arg-max of |value| with the lowest index winning ties: the combination rule
-// of LAPACK idamax, which scans upward and only moves on a strictly larger
-// magnitude.  Each lane first scans its own rows in increasing order with the
-// same strict rule, so the warp result equals a sequential scan.
-__device__ __forceinline__ void warp_argmax_first(double& v, int& idx) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double ov = __shfl_xor_sync(0xffffffffu, v, o);
-    int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (ov > v || (ov == v && oi < idx)) {
-      v = ov;
-      idx = oi;
-    }
-  }
-}
-
 // Pivot-search key of x: |x| as its IEEE bit pattern, which orders like the
 // value for every non-NaN x; NaN maps to -1 and never wins (as "|x| > v" never
 // holds for NaN).  64-bit integer compares run on the integer pipe, not on
@@ -102,7 +86,10 @@ __device__ __forceinline__ long long pivot_key(double x) {
   return b > 0x7FF0000000000000LL ? -1LL : b;
 }
 
-// warp_argmax_first over pivot keys.
+// Arg-max of pivot keys with the lowest index winning ties: the combination rule
+// of LAPACK idamax, which scans upward and only moves on a strictly larger
+// magnitude.  Each lane first scans its own rows in increasing order with the
+// same strict rule, so the warp result equals a sequential scan.
 __device__ __forceinline__ void warp_argmax_first_key(long long& v, int& idx) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {

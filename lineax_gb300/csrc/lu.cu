@@ -21,10 +21,6 @@
 #include <float.h>
 #include <limits.h>
 
-#include <map>
-#include <mutex>
-#include <utility>
-
 #include "common.cuh"
 #include "trisolve.cuh"
 
@@ -645,48 +641,12 @@ panel_getf2_cluster_kernel(int n, int j0, int nb, int rows_per_cta, double* __re
   cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// Whether a cluster of c CTAs of this kernel can be co-scheduled on the
-// current device (asked once per device and size).
-template <int TPR>
-static bool panel_clu_fits(int c) {
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, bool> known;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
-  std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_pair(dev, c);
-  auto it = known.find(key);
-  if (it != known.end()) return it->second;
-  bool ok = cudaFuncSetAttribute(panel_getf2_cluster_kernel<TPR>,
-                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            ensure_dynamic_smem(reinterpret_cast<const void*>(panel_getf2_cluster_kernel<TPR>),
-                                kPcluReserve) == cudaSuccess;
-  if (ok) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)c);
-    cfg.blockDim = dim3(kPcluThreads);
-    cfg.dynamicSmemBytes = kPcluReserve;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)c;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    ok = cudaOccupancyMaxActiveClusters(&nclusters, panel_getf2_cluster_kernel<TPR>, &cfg) ==
-             cudaSuccess &&
-         nclusters >= 1;
-  }
-  if (!ok) cudaGetLastError();
-  known[key] = ok;
-  return ok;
-}
-
 template <int TPR>
 static int launch_panel_clu(int c, int R, int n, int j0, int nb, double* a, int32_t* piv,
                             int32_t* info, cudaStream_t st) {
-  if (!panel_clu_fits<TPR>(c)) return -1;
+  if (!cluster_fits(reinterpret_cast<const void*>(panel_getf2_cluster_kernel<TPR>), c, kPcluThreads,
+                    kPcluReserve))
+    return -1;
   const int threads = (R * TPR + 31) / 32 * 32 + 32;
   const cudaError_t e =
       launch_pdl(panel_getf2_cluster_kernel<TPR>, dim3((unsigned)c), dim3((unsigned)threads),

@@ -870,52 +870,6 @@ int gemm_bf16_nt(int M, int N, int K, const void* A, int64_t lda, const void* B,
   return check_launch("gemm_bf16");
 }
 
-// dst (rows × cols, row stride ldd) = src rounded to BF16 (nearest even).
-__global__ void bf16_convert_kernel(int64_t rows, int64_t cols, const float* __restrict__ src,
-                                    int64_t lds, __nv_bfloat16* __restrict__ dst, int64_t ldd) {
-  const int64_t total = rows * cols;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = e / cols, c = e % cols;
-    dst[r * ldd + c] = __float2bfloat16_rn(src[r * lds + c]);
-  }
-}
-
-int bf16_convert(int64_t rows, int64_t cols, const float* src, int64_t lds, void* dst, int64_t ldd,
-                 cudaStream_t st) {
-  const int64_t total = rows * cols;
-  if (total <= 0) return LXGB_SUCCESSFUL;
-  const int64_t blocks = (total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096;
-  bf16_convert_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, cols, src, lds,
-                                                        reinterpret_cast<__nv_bfloat16*>(dst), ldd);
-  return check_launch("bf16_convert");
-}
-
-// hi = x with the low 13 mantissa bits cleared (TF32-exact), lo = x - hi
-// (exact in FP32): the operand split of 3xTF32.
-__global__ void tf32_split_kernel(int64_t rows, int64_t cols, const float* __restrict__ src,
-                                  int64_t lds, float* __restrict__ hi, float* __restrict__ lo,
-                                  int64_t ldd) {
-  const int64_t total = rows * cols;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = e / cols, c = e % cols;
-    const float x = src[r * lds + c];
-    const float h = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-    hi[r * ldd + c] = h;
-    lo[r * ldd + c] = x - h;
-  }
-}
-
-int tf32_split(int64_t rows, int64_t cols, const float* src, int64_t lds, float* hi, float* lo,
-               int64_t ldd, cudaStream_t st) {
-  const int64_t total = rows * cols;
-  if (total <= 0) return LXGB_SUCCESSFUL;
-  const int64_t blocks = (total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096;
-  tf32_split_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, cols, src, lds, hi, lo, ldd);
-  return check_launch("tf32_split");
-}
-
 }  // namespace lxgb
 
 using namespace lxgb;

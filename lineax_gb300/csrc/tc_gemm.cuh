@@ -36,10 +36,4 @@ int gemm_tf32_nt_splitk(int M, int N, int K, const float* A, int64_t lda, const 
 int gemm_bf16_nt(int M, int N, int K, const void* A, int64_t lda, const void* B, int64_t ldb,
                  float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
                  bool beside = false);
-// dst = src rounded to BF16 (rows × cols; row strides in elements).
-int bf16_convert(int64_t rows, int64_t cols, const float* src, int64_t lds, void* dst, int64_t ldd,
-                 cudaStream_t st);
-// hi/lo split of a rows×cols block (row stride lds) into hi, lo (row stride ldd).
-int tf32_split(int64_t rows, int64_t cols, const float* src, int64_t lds, float* hi, float* lo,
-               int64_t ldd, cudaStream_t st);
 }
