@@ -756,9 +756,8 @@ __device__ __noinline__ void mx_solve_t(const float* U, int ld, int n, int nc, f
 }
 
 // --- residual: D = fl32(B - A X) with X = hi + lo (float2), FP64-accurate, no FP64 ops
-// A is split bitwise into hi+lo, hi*xh products made exact by an FMA
-// (TwoProd) and summed with TwoSum; ah*xl + al*xh, the product errors and the
-// summation errors go to a second FP32 accumulator.  b - Ax is formed in the
+// A is split bitwise into hi+lo, hi*xh products summed with their exact errors
+// (df_mac); those errors and ah*xl + al*xh go to a second FP32 accumulator.  b - Ax is formed in the
 // same double-float arithmetic from the split of b.  Lane c of each warp
 // finishes vector c.  Per-warp maxima of |r| and the row sums of |A| (for
 // ||A||_inf) land in sm.red / sm.red2.  Vectors nc..NC-1 are padding: b = 0
@@ -821,12 +820,7 @@ __device__ __noinline__ void mx_residual_t(const double* __restrict__ A, int n, 
             for (int k = 0; k < 2; ++k) {
               const int c = 2 * h + k;
               const float2 xv = XV[c * n + j];
-              const float xh = xv.x, xl = xv.y;
-              const float p = ah[u] * xh;
-              const float pe = fmaf(ah[u], xh, -p);
-              float err;
-              two_sum(S[c], p, err);
-              C[c] += fmaf(ah[u], xl, fmaf(al[u], xh, pe + err));
+              df_mac<true>(S[c], C[c], ah[u], al[u], xv.x, xv.y);
             }
           }
         }

@@ -91,4 +91,19 @@ __device__ __forceinline__ void fast_two_sum(float& s, float t, float& err) {
   s = r;
 }
 
+// (s, sl) += (a + al)(x + xl): the sum with the rounded product, the error of
+// both (exact), the two mixed products and their sum in sl.  Ten operations; with
+// the product, its error and a two-sum of six each formed for itself twelve.
+template <bool LO>
+__device__ __forceinline__ void df_mac(float& s, float& sl, float a, float al, float x, float xl) {
+  const float r = __fadd_rn(s, __fmul_rn(a, x));  // not to be contracted to an FMA
+  const float z = r - s;
+  const float t = r - z;
+  float e = (s - t) + fmaf(a, x, -z);
+  e = fmaf(a, xl, e);
+  if (LO) e = fmaf(al, x, e);
+  s = r;
+  sl += e;
+}
+
 }  // namespace lxgb

@@ -445,18 +445,6 @@ constexpr int kDfK = 64;        // columns per stage
 constexpr int kDfLd = kDfK + 4; // padded row: 16-byte aligned, conflict-free over 8 rows
 constexpr int kDfThreads = 256;
 
-template <bool LO>
-__device__ __forceinline__ void df_mac(float& s, float& sl, float a, float al, float x, float xl) {
-  const float r = __fadd_rn(s, __fmul_rn(a, x));  // not to be contracted to an FMA
-  const float z = r - s;
-  const float t = r - z;
-  float e = (s - t) + fmaf(a, x, -z);
-  e = fmaf(a, xl, e);
-  if (LO) e = fmaf(al, x, e);
-  s = r;
-  sl += e;
-}
-
 // `bytes` of the 4 VEC bytes at src (the rest zero) into shared memory.
 template <int VEC>
 __device__ __forceinline__ void df_copy(float* dst, const float* src, int bytes) {
