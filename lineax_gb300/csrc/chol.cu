@@ -772,40 +772,48 @@ __device__ __noinline__ void mx_residual_t(const double* __restrict__ A, int n, 
   const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
   float rmax = 0.0f;                   // lane 4c: max |r| of vector c
   float rowmax = 0.0f;
-  // The warp walks (row, 256-column chunk) pairs; the loads of the next pair
-  // (and b of the next row) are issued before the current chunk is used, so
-  // the DRAM latency of A overlaps the arithmetic.
-  const int nch = (n + 255) >> 8;
+  // The warp takes two rows at a time, so that a value of x read from shared
+  // memory serves both, and walks (rows, 128-column chunk) pairs; the loads of
+  // the next pair (and b of the next rows) are issued before the current chunk
+  // is used, so the DRAM latency of A overlaps the arithmetic.
+  const int nch = (n + 127) >> 7;
   auto load_chunk = [&](int r, int ch, uint2 (&v)[8]) {
-    const uint2* rowp = reinterpret_cast<const uint2*>(A + (int64_t)r * n);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int j = (ch << 8) + lane + 32 * u;
-      v[u] = (r < n && j < n) ? rowp[j] : make_uint2(0u, 0u);
+    for (int q = 0; q < 2; ++q) {
+      const uint2* rowp = reinterpret_cast<const uint2*>(A + (int64_t)(r + q * nw) * n);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = (ch << 7) + lane + 32 * u;
+        v[4 * q + u] = (r + q * nw < n && j < n) ? rowp[j] : make_uint2(0u, 0u);
+      }
     }
   };
+  auto load_b = [&](int r) { return (r < n && cl < nc) ? B[(int64_t)cl * n + r] : 0.0; };
   uint2 av[8];
   load_chunk(warp, 0, av);
-  double bnext = (warp < n && cl < nc) ? B[(int64_t)cl * n + warp] : 0.0;
-  for (int i = warp; i < n; i += nw) {
-    float S[NC], C[NC];
+  double bnext[2] = {load_b(warp), load_b(warp + nw)};
+  for (int i = warp; i < n; i += 2 * nw) {
+    float S[2][NC], C[2][NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) { S[c] = 0.0f; C[c] = 0.0f; }
-    float rs = 0.0f;
-    const double bval = bnext;
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) { S[q][c] = 0.0f; C[q][c] = 0.0f; }
+    float rs[2] = {0.0f, 0.0f};
+    double bval[2] = {bnext[0], bnext[1]};
     for (int ch = 0; ch < nch; ++ch) {
-      const int j0 = ch << 8;
+      const int j0 = ch << 7;
       uint2 an[8];
       if (ch + 1 < nch) {
         load_chunk(i, ch + 1, an);
       } else {
-        load_chunk(i + nw, 0, an);
-        bnext = (i + nw < n && cl < nc) ? B[(int64_t)cl * n + i + nw] : 0.0;
+        load_chunk(i + 2 * nw, 0, an);
+        bnext[0] = load_b(i + 2 * nw);
+        bnext[1] = load_b(i + 3 * nw);
       }
       float ah[8], al[8];
       splitw<8>(av, ah, al);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) rs += fabsf(ah[u]);   // ah = 0 past the row's end
+      for (int u = 0; u < 8; ++u) rs[u >> 2] += fabsf(ah[u]);   // ah = 0 past the row's end
       // vectors in pairs, a pair only when it holds a live one (the rest
       // are padding); per vector the terms go in j order.  x is read as one
       // 8-byte (hi, lo) pair per element.
@@ -813,14 +821,15 @@ __device__ __noinline__ void mx_residual_t(const double* __restrict__ A, int n, 
       for (int h = 0; h < 4; ++h) {
         if (h > 0 && 2 * h >= nc) break;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < 4; ++u) {
           const int j = j0 + lane + 32 * u;
           if (j < n) {
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
               const int c = 2 * h + k;
               const float2 xv = XV[c * n + j];
-              df_mac<true>(S[c], C[c], ah[u], al[u], xv.x, xv.y);
+              df_mac<true>(S[0][c], C[0][c], ah[u], al[u], xv.x, xv.y);
+              df_mac<true>(S[1][c], C[1][c], ah[4 + u], al[4 + u], xv.x, xv.y);
             }
           }
         }
@@ -832,57 +841,66 @@ __device__ __noinline__ void mx_residual_t(const double* __restrict__ A, int n, 
     // (xor 16: 4 of 8, xor 8: 2, xor 4: 1), then two plain steps; lane L ends
     // with the row's sum for vector L >> 2.  Nine double-float additions per
     // lane instead of forty.
-    float S4[4], C4[4];
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+      float S4[4], C4[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float ss = __shfl_xor_sync(0xffffffffu, b4 ? S[k] : S[4 + k], 16);
-      const float cs = __shfl_xor_sync(0xffffffffu, b4 ? C[k] : C[4 + k], 16);
-      S4[k] = b4 ? S[4 + k] : S[k];
-      C4[k] = b4 ? C[4 + k] : C[k];
-      float err;
-      two_sum(S4[k], ss, err);
-      C4[k] += cs + err;
-    }
-    float S2[2], C2[2];
+      for (int k = 0; k < 4; ++k) {
+        const float ss = __shfl_xor_sync(0xffffffffu, b4 ? S[0][k] : S[0][4 + k], 16);
+        const float cs = __shfl_xor_sync(0xffffffffu, b4 ? C[0][k] : C[0][4 + k], 16);
+        S4[k] = b4 ? S[0][4 + k] : S[0][k];
+        C4[k] = b4 ? C[0][4 + k] : C[0][k];
+        float err;
+        two_sum(S4[k], ss, err);
+        C4[k] += cs + err;
+      }
+      float S2[2], C2[2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float ss = __shfl_xor_sync(0xffffffffu, b3 ? S4[k] : S4[2 + k], 8);
-      const float cs = __shfl_xor_sync(0xffffffffu, b3 ? C4[k] : C4[2 + k], 8);
-      S2[k] = b3 ? S4[2 + k] : S4[k];
-      C2[k] = b3 ? C4[2 + k] : C4[k];
-      float err;
-      two_sum(S2[k], ss, err);
-      C2[k] += cs + err;
-    }
-    float S1, C1;
-    {
-      const float ss = __shfl_xor_sync(0xffffffffu, b2 ? S2[0] : S2[1], 4);
-      const float cs = __shfl_xor_sync(0xffffffffu, b2 ? C2[0] : C2[1], 4);
-      S1 = b2 ? S2[1] : S2[0];
-      C1 = b2 ? C2[1] : C2[0];
-      float err;
-      two_sum(S1, ss, err);
-      C1 += cs + err;
-    }
+      for (int k = 0; k < 2; ++k) {
+        const float ss = __shfl_xor_sync(0xffffffffu, b3 ? S4[k] : S4[2 + k], 8);
+        const float cs = __shfl_xor_sync(0xffffffffu, b3 ? C4[k] : C4[2 + k], 8);
+        S2[k] = b3 ? S4[2 + k] : S4[k];
+        C2[k] = b3 ? C4[2 + k] : C4[k];
+        float err;
+        two_sum(S2[k], ss, err);
+        C2[k] += cs + err;
+      }
+      float S1, C1;
+      {
+        const float ss = __shfl_xor_sync(0xffffffffu, b2 ? S2[0] : S2[1], 4);
+        const float cs = __shfl_xor_sync(0xffffffffu, b2 ? C2[0] : C2[1], 4);
+        S1 = b2 ? S2[1] : S2[0];
+        C1 = b2 ? C2[1] : C2[0];
+        float err;
+        two_sum(S1, ss, err);
+        C1 += cs + err;
+      }
 #pragma unroll
-    for (int o = 2; o > 0; o >>= 1) {
-      const float ss = __shfl_xor_sync(0xffffffffu, S1, o);
-      const float cs = __shfl_xor_sync(0xffffffffu, C1, o);
-      float err;
-      two_sum(S1, ss, err);
-      C1 += cs + err;
-    }
+      for (int o = 2; o > 0; o >>= 1) {
+        const float ss = __shfl_xor_sync(0xffffffffu, S1, o);
+        const float cs = __shfl_xor_sync(0xffffffffu, C1, o);
+        float err;
+        two_sum(S1, ss, err);
+        C1 += cs + err;
+      }
+      float ra = rs[0];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
-    rowmax = fmaxf(rowmax, rs);
-    if ((lane & 3) == 0) {
-      float bh, bl;
-      split_f64(bval, bh, bl);
-      float rh = bh, re;
-      two_sum(rh, -S1, re);
-      const float r = rh + ((bl - C1) + re);
-      D[i * kMxKc + cl] = r;
-      rmax = fmaxf(rmax, fabsf(r));
+      for (int o = 16; o > 0; o >>= 1) ra += __shfl_xor_sync(0xffffffffu, ra, o);
+      rowmax = fmaxf(rowmax, ra);
+      if ((lane & 3) == 0 && i + q * nw < n) {
+        float bh, bl;
+        split_f64(bval[0], bh, bl);
+        float rh = bh, re;
+        two_sum(rh, -S1, re);
+        const float r = rh + ((bl - C1) + re);
+        D[(i + q * nw) * kMxKc + cl] = r;
+        rmax = fmaxf(rmax, fabsf(r));
+      }
+      // the second row in the first one's place
+#pragma unroll
+      for (int c = 0; c < NC; ++c) { S[0][c] = S[1][c]; C[0][c] = C[1][c]; }
+      rs[0] = rs[1];
+      bval[0] = bval[1];
     }
   }
   if ((lane & 3) == 0) sm.red[warp][cl] = rmax;
