@@ -721,11 +721,14 @@ __device__ __noinline__ void mx_solve_t(const float* U, int ld, int n, int nc, f
 #pragma unroll
       for (int t = 0; t < 32; ++t) col[t] = (t < lane && lane < rn) ? U[(r0 + t) * ld + r0 + lane] : 0.0f;
       const float rdl = (lane < rn) ? rd[r0 + lane] : 0.0f;
-      float v = (lane < rn) ? D[(r0 + lane) * kMxKc + c] : 0.0f;
+      // rows scaled by 1 / diagonal first: a step is then a shuffle and an FMA
+      float v = (lane < rn) ? D[(r0 + lane) * kMxKc + c] * rdl : 0.0f;
+#pragma unroll
+      for (int t = 0; t < 32; ++t) col[t] *= rdl;
 #pragma unroll
       for (int t = 0; t < 32; ++t) {  // lanes >= rn carry zeros, so all 32 steps run
-        const float yt = __shfl_sync(0xffffffffu, v * rdl, t);
-        v = (lane == t) ? yt : ((lane > t) ? fmaf(-col[t], yt, v) : v);
+        const float yt = __shfl_sync(0xffffffffu, v, t);
+        if (lane > t) v = fmaf(-col[t], yt, v);
       }
       if (lane < rn) D[(r0 + lane) * kMxKc + c] = v;
     }
@@ -741,11 +744,13 @@ __device__ __noinline__ void mx_solve_t(const float* U, int ld, int n, int nc, f
 #pragma unroll
       for (int t = 0; t < 32; ++t) row[t] = (t > lane && t < rn) ? U[(r0 + lane) * ld + r0 + t] : 0.0f;
       const float rdl = (lane < rn) ? rd[r0 + lane] : 0.0f;
-      float v = (lane < rn) ? D[(r0 + lane) * kMxKc + c] : 0.0f;
+      float v = (lane < rn) ? D[(r0 + lane) * kMxKc + c] * rdl : 0.0f;
+#pragma unroll
+      for (int t = 0; t < 32; ++t) row[t] *= rdl;
 #pragma unroll
       for (int tt = 31; tt >= 0; --tt) {
-        const float xt = __shfl_sync(0xffffffffu, v * rdl, tt);
-        v = (lane == tt) ? xt : ((lane < tt) ? fmaf(-row[tt], xt, v) : v);
+        const float xt = __shfl_sync(0xffffffffu, v, tt);
+        if (lane < tt) v = fmaf(-row[tt], xt, v);
       }
       if (lane < rn) D[(r0 + lane) * kMxKc + c] = v;
     }
