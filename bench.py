@@ -871,7 +871,7 @@ def run_cg_poisson(args):
             # (12); the FP64 replacement every 16 iterations: fold x += x_lo (24)
             # and r = b - A x (20), 44 / 16 = 2.75
             ("mixed", lambda m: _krylov.cg_poisson_mixed(op, b, rtol=rtol, atol=atol,
-                                                         max_steps=m), 8 + 24 + 12 + 2.75)):
+                                                         max_steps=m), 12 + 20 + 3)):
         fn(args.warmup)
         torch.cuda.synchronize()
         e0.record()
