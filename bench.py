@@ -866,10 +866,10 @@ def run_cg_poisson(args):
     for name, fn, bpp in (
             ("fp64", lambda m: _krylov.cg_block(op, b, rtol=rtol, atol=atol, max_steps=m),
              16 + 48 + 24 + 2.4),
-            # FP32 vectors: stencil reads p, writes Ap (8); update reads p, Ap,
-            # x_lo, r and writes x_lo, r (24); direction reads r, p, writes p
-            # (12); the FP64 replacement every 16 iterations: fold x += x_lo (24)
-            # and r = b - A x (20), 44 / 16 = 2.75
+            # FP32 vectors: the residual pass reads p, r and writes r (12); the step
+            # reads r, p, x_lo and writes p, x_lo (20); the FP64 replacement every
+            # 16 iterations: fold x += x_lo (24), r = b - A x (20) and <p, Ap> of
+            # the kept p (4), 48 / 16 = 3
             ("mixed", lambda m: _krylov.cg_poisson_mixed(op, b, rtol=rtol, atol=atol,
                                                          max_steps=m), 12 + 20 + 3)):
         fn(args.warmup)
