@@ -210,7 +210,7 @@ __global__ void c32_alpha_kernel(int k, C32State s, int P) {
 // except one row at each end.  Measured at 2048 x 2048, 64 right-hand sides (12
 // bytes per point, 450 us at HBM's rate): one partial per CTA, three rows read
 // from L2 for one updated, 759 us; G = 32 643; with the next points prefetched
-// into L2 540.
+// into L2 540; G = 16 523.
 constexpr int kC32ResThreads = 512;
 
 template <int G>
@@ -581,11 +581,16 @@ extern "C" int lxgb_cg32_iterate(int32_t k, int64_t nx, int64_t ny, int32_t iter
   const dim3 gv((unsigned)Pv, (unsigned)k), g1((unsigned)k), bt(kC32Threads), bw(32);
   const bool vec = ny % 4 == 0 && (((uintptr_t)p | (uintptr_t)ap | (uintptr_t)xlo | (uintptr_t)r) & 15) == 0;
   float *cur = p, *nxt = ap;
-  // partials per CTA of the residual pass: as many as leave two CTAs per SM
-  int g = 32;
-  if ((int64_t)k * ((Pv + g - 1) / g) < 2 * sm_count()) g = 8;
-  if ((int64_t)k * ((Pv + g - 1) / g) < 2 * sm_count()) g = 2;
-  auto resid = g == 32 ? c32_residual_kernel<32> : (g == 8 ? c32_residual_kernel<8> : c32_residual_kernel<2>);
+  // Partials per CTA of the residual pass: sixteen where two CTAs per SM remain,
+  // four where one does.  ms for 32 steps with 16, 4 and 2: 2048 x 2048, one
+  // right-hand side 1.91, 1.58 and 1.67, four 4.59, 4.67 and 4.78; 701 x 1333, 64
+  // 16.3, 16.7 and 17.2; 256 x 256, one 1.03, 0.73 and 0.68 (32: 2.63, 5.05, 16.7
+  // and 1.49).
+  int g = 16;
+  if ((int64_t)k * ((Pv + g - 1) / g) < 2 * sm_count()) g = 4;
+  if ((int64_t)k * ((Pv + g - 1) / g) < sm_count()) g = 2;
+  auto resid = g == 16 ? c32_residual_kernel<16>
+                       : (g == 4 ? c32_residual_kernel<4> : c32_residual_kernel<2>);
   const dim3 gr((unsigned)((Pv + g - 1) / g), (unsigned)k), br(kC32ResThreads);
   cudaError_t e = launch_pdl(vec ? c32_step_kernel<false, 4> : c32_step_kernel<false, 1>, gs, bt, 0,
                              st, 1, nx, ny, s, r, cur, nxt, xlo);
