@@ -20,9 +20,14 @@
 // n = 128 and 767, and a diagonal and an update launch per block 549 and 1104
 // at n = 1000 and 2003.  getrs at n = 2003: 511 us against 2500 to 6200 (the
 // more interchanges, the longer: one thread ran them in order).
+// Few vectors of up to 2048 unknowns: trisolve_cluster_kernel below.
+#include <cooperative_groups.h>
+
 #include "trisolve.cuh"
 
 namespace lxgb {
+
+namespace cg = cooperative_groups;
 
 constexpr int kTsThreads = 256;
 
@@ -173,11 +178,176 @@ trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t s
   }
 }
 
+// The whole solve in one launch for n up to 64 kTcMaxBlocks: a cluster of C CTAs
+// per vector, CTA r holding the blocks r, r + C, ... of x in shared memory.  Step
+// b + 1: its owner subtracts x_b from its block, solves it and writes x_{b+1} into
+// every CTA's shared memory; then, and in the other CTAs meanwhile, x_b is
+// subtracted from the later blocks.  Matrix entries of the chain are loaded before
+// the wait for x_b.  A CTA arrives at the cluster barrier of step b + 1 before its
+// own later blocks' updates, so it may lag behind the chain by a step or two (four
+// buffers of x; program order keeps a buffer's last read before the arrival that
+// lets it be overwritten).  The operations on every element, and their order, are
+// trisolve_step_kernel's.
+// Measured (one vector, us): n = 401 55, 1000 120, 1531 177, 2003 235, against 64,
+// 132, 206 and 267 with a launch per block, whose hand-over it saves; the chain of
+// a block (two substitutions, the update, the push and the barrier) remains.
+constexpr int kTcMaxBlocks = 32;
+constexpr int kTcMax = 16;
+
+__global__ void __launch_bounds__(kTsThreads, 1)
+trisolve_cluster_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t stride_t,
+                        int fwd, int trans, int unit, double* __restrict__ x, int64_t stride_x) {
+  __shared__ double xs[kTcMaxBlocks / kTcMax][kTsNB];  // this CTA's blocks, in turn
+  __shared__ double xb[4][kTsNB];              // solved blocks, written by their owners
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nblk = (n + kTsNB - 1) / kTsNB;
+  const TsView T{t + (int64_t)blockIdx.z * stride_t, ldt, n, fwd != 0, trans != 0};
+  double* xv = x + (int64_t)blockIdx.z * stride_x + (int64_t)blockIdx.y * n;
+  const int wi = tid >> 2, wq = tid & 3;           // row, part: columns 4 pp + wq
+  double cu[16], d[32], dd = 1.0, rinv = 1.0, cs[4];
+  bool scaled = true;
+  auto load_update = [&](int w, int b) {
+#pragma unroll
+    for (int pp = 0; pp < 16; ++pp)
+      cu[pp] = (w * kTsNB + wi < n) ? T.op(w * kTsNB + wi, b * kTsNB + 4 * pp + wq) : 0.0;
+  };
+  auto update = [&](double* xw, const double* xp) {
+    double acc[2] = {0.0, 0.0};
+#pragma unroll
+    for (int pp = 0; pp < 16; ++pp) acc[pp & 1] = fma(cu[pp], xp[4 * pp + wq], acc[pp & 1]);
+    double s = acc[0] + acc[1];
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (wq == 0) xw[wi] -= s;
+  };
+  auto load_diag = [&](int b) {
+    const int u0 = b * kTsNB;
+    scaled = true;
+    dd = rinv = 1.0;
+    if (warp < 2) {
+      const int ul = u0 + 32 * warp + lane;
+      bool ok = true;
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        const int uk = u0 + 32 * warp + k;
+        d[k] = (ul < n && k < lane) ? T.op(ul, uk) : 0.0;
+      }
+      if (!unit && ul < n) dd = T.op(ul, ul);
+      if (!unit) {
+#pragma unroll
+        for (int k = 0; k < 32; ++k) ok = ok && ts_moderate(d[k], true);
+        ok = ok && ts_moderate(dd, false);
+        scaled = __all_sync(0xffffffffu, ok);
+        if (scaled) {
+          rinv = 1.0 / dd;
+#pragma unroll
+          for (int k = 0; k < 32; ++k) d[k] *= __shfl_sync(0xffffffffu, rinv, k);
+        }
+      }
+    }
+#pragma unroll
+    for (int pp = 0; pp < 4; ++pp) {
+      const int ur = u0 + 32 + (tid >> 3);
+      cs[pp] = (ur < n) ? T.op(ur, u0 + 8 * pp + (tid & 7)) : 0.0;
+    }
+  };
+  // block b solved in place in xc, out to memory and to every CTA's buffer
+  auto solve = [&](double* xc, int b) {
+    const int u0 = b * kTsNB;
+    if (warp == 0) xc[lane] = ts_solve32(xc[lane], d, dd, rinv, scaled);
+    __syncthreads();
+    double s = 0.0;
+#pragma unroll
+    for (int pp = 0; pp < 4; ++pp) s = fma(cs[pp], xc[8 * pp + (tid & 7)], s);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    if ((tid & 7) == 0) xc[32 + (tid >> 3)] -= s;
+    __syncthreads();
+    if (warp == 1) xc[32 + lane] = ts_solve32(xc[32 + lane], d, dd, rinv, scaled);
+    __syncthreads();
+    const double v = xc[tid & (kTsNB - 1)];
+#pragma unroll
+    for (int q = 0; q < kTcMax / 4; ++q) {
+      const int dst = 4 * q + (tid >> 6);
+      if (dst < C) *cluster.map_shared_rank(&xb[b & 3][tid & (kTsNB - 1)], dst) = v;
+    }
+    if (tid < kTsNB && u0 + tid < n) xv[T.row(u0 + tid)] = v;
+  };
+  for (int e = tid; rank + (e / kTsNB) * C < nblk; e += kTsThreads) {
+    const int u = (rank + (e / kTsNB) * C) * kTsNB + e % kTsNB;
+    xs[e / kTsNB][e % kTsNB] = (u < n) ? xv[T.row(u)] : 0.0;
+  }
+  cluster.sync();                                  // all run before any remote store
+  if (rank == 0) {
+    load_diag(0);
+    solve(xs[0], 0);
+  }
+  cluster.barrier_arrive();
+  for (int b = 0; b + 1 < nblk; ++b) {
+    const bool next = rank == (b + 1) % C;
+    if (next) {
+      load_diag(b + 1);
+      load_update(b + 1, b);
+    }
+    cluster.barrier_wait();                        // x_b is here
+    const double* xp = xb[b & 3];
+    if (next) {
+      double* xc = xs[(b + 1) / C];
+      update(xc, xp);
+      __syncthreads();
+      solve(xc, b + 1);
+    }
+    cluster.barrier_arrive();
+    // this CTA's blocks after b + 1
+    for (int w = rank + ((b + 2 - rank + C - 1) / C) * C; w < nblk; w += C) {
+      load_update(w, b);
+      update(xs[w / C], xp);
+    }
+  }
+  cluster.barrier_wait();  // no CTA leaves while another may still write its shared memory
+}
+
+// CTAs per vector of the one-launch solve, 0 where a launch per block is taken:
+// n above its blocks (two per CTA: more of them would hold up the chain) or one
+// block, more vectors than clusters fit on the SMs at once, or no cluster to be
+// had.  us at n = 1000 here and with a launch per block: 4 vectors 120 and 132, 8
+// vectors 231 and 138 (the clusters run one after the other).
+static int ts_cluster_size(int64_t vectors, int n) {
+  const int nblk = (n + kTsNB - 1) / kTsNB;
+  if (nblk < 2 || nblk > kTcMaxBlocks) return 0;
+  const int c = nblk < kTcMax ? nblk : kTcMax;
+  int room = kTcMax;                 // SMs of one processing cluster that it takes
+  while (room / 2 >= c) room /= 2;
+  if (vectors * room > 4 * kTcMax) return 0;
+  return cluster_fits(reinterpret_cast<const void*>(trisolve_cluster_kernel), c, kTsThreads, 0) ? c : 0;
+}
+
 int trisolve_blocked(int64_t batch, int n, int nrhs, const double* t, int64_t ldt,
                      int64_t stride_t, int lower, int trans, int unit, double* x,
                      int64_t stride_x, cudaStream_t st) {
   const int fwd = (lower != 0) != (trans != 0);
   const int nblk = (n + kTsNB - 1) / kTsNB;
+  const int c = ts_cluster_size(batch * nrhs, n);
+  if (c > 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)c, (unsigned)nrhs, (unsigned)batch);
+    cfg.blockDim = dim3(kTsThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LXGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, trisolve_cluster_kernel, n, t, ldt, stride_t, fwd, trans,
+                                     unit, x, stride_x),
+                  "trisolve: launch");
+    return check_launch("trisolve");
+  }
   for (int b = 0; b < nblk; ++b) {
     const int after = n - (b + 1) * kTsNB;         // rows after this block
     const unsigned gx = 1u + (unsigned)((b > 0 && after > 0) ? (after + kTsNB - 1) / kTsNB : 0);
