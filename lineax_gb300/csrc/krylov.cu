@@ -763,7 +763,8 @@ __global__ void gm_snapshot_kernel(int k, GmWork w, int cur, int* on) {
 // linear_solve(..., QR()) of gmres.py:301-303).  H is upper Hessenberg (row kk of
 // coeff ends at kk + 1), so each reflection has two rows; a lane takes every 32nd
 // column.  A chain of R reflections and R back-substitution steps bounds it:
-// 44 us for R = 20 (116 with full columns and one thread's sums).
+// 34 us for R = 20 (44 with hypot and two divisions, 116 with full columns and one
+// thread's sums).
 __global__ void __launch_bounds__(32)
 gm_lstsq_kernel(int k, GmWork w, int cur) {
   extern __shared__ double smem_h[];  // (R+1)×(R+1) matrix, then rhs
@@ -782,8 +783,20 @@ gm_lstsq_kernel(int k, GmWork w, int cur) {
     const double alpha = H(j, j), below = H(j + 1, j);
     double tau = 0.0, v = below, beta = alpha;
     if (below != 0.0) {  // (NaN included)
-      beta = -copysign(hypot(alpha, below), alpha);
-      tau = (beta - alpha) / beta;
+      const double sq = fma(alpha, alpha, below * below);
+      const unsigned ex = (unsigned)__double2hiint(sq) >> 20;
+      if (ex - 123u < 1800u) {         // 2^-900 <= sq < 2^900
+        // ||(alpha, below)|| by a Newton step on sq / sqrt(sq): a reciprocal root
+        // and a division in the chain instead of hypot and two divisions
+        const double y = rsqrt(sq);
+        double nrm = sq * y;
+        nrm = fma(0.5 * y, fma(-nrm, nrm, sq), nrm);
+        beta = -copysign(nrm, alpha);
+        tau = fma(fabs(alpha), y, 1.0);
+      } else {
+        beta = -copysign(hypot(alpha, below), alpha);
+        tau = (beta - alpha) / beta;
+      }
       v = below / (alpha - beta);
     }
     for (int q = j + 1 + lane; q <= R; q += 32) {  // q = R: the right-hand side
