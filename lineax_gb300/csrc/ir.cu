@@ -175,6 +175,7 @@ block_row_kernel(BlockRowArgs g) {
   const int tid = threadIdx.x;
   const int n = g.n, j0 = g.j0, nb = g.nb;
   pdl_wait();
+  pdl_trigger();  // a product that needs nothing of this row may start beside it
   if ((int)blockIdx.x >= g.strips) {               // the other operand
     if (PREC != 0) {
       const int r0 = ((int)blockIdx.x - g.strips) * kInvNB;
@@ -843,7 +844,8 @@ static int64_t vec_bytes(int n, int nrhs) {
 using namespace lxgb;
 
 extern "C" int64_t lxgb_lu32_inverse_workspace_size(int32_t n, int32_t precision) {
-  return 256 + (precision == 1 ? 5 : 1) * blk_bytes(n);
+  // the update's operands, one set for each of the two inverses
+  return 256 + 2 * (precision == 1 ? 5 : 1) * blk_bytes(n);
 }
 
 extern "C" int lxgb_lu32_inverse(int32_t n, const float* lu, const int32_t* piv, float* linv,
@@ -871,14 +873,17 @@ extern "C" int lxgb_lu32_inverse(int32_t n, const float* lu, const int32_t* piv,
   if (linv) set_identity_f32_kernel<<<idg, 256, 0, st>>>(n, linv);
   if (uinv) set_identity_f32_kernel<<<idg, 256, 0, st>>>(n, uinv);
   const int64_t blk = blk_bytes(n);
-  char* wb = reinterpret_cast<char*>(work) + 256;
-  float* xt = reinterpret_cast<float*>(wb);
-  float* ah = reinterpret_cast<float*>(wb + blk);
-  float* al = reinterpret_cast<float*>(wb + 2 * blk);
-  float* bh = reinterpret_cast<float*>(wb + 3 * blk);
-  float* bl = reinterpret_cast<float*>(wb + 4 * blk);
   const bool split = precision == 1;
-  auto block = [&](float* w, int j0, int nb, int c_begin, int c_end, const float* a_src, int na) {
+  // operands of an inverse's update: a hi, lo; X^T hi (or FP32), lo
+  struct Operands { float *ah, *al, *b, *bl; };
+  auto operands = [&](int set) {
+    char* p = reinterpret_cast<char*>(work) + 256 + (int64_t)set * (split ? 5 : 1) * blk;
+    auto at = [&](int i) { return reinterpret_cast<float*>(p + i * blk); };
+    return split ? Operands{at(1), at(2), at(3), at(4)} : Operands{nullptr, nullptr, at(0), nullptr};
+  };
+  const Operands ol = operands(0), ou = operands(1);
+  auto block = [&](const Operands& o, float* w, int j0, int nb, int c_begin, int c_end,
+                   const float* a_src, int na) {
     BlockRowArgs g = {};
     g.n = n;
     g.j0 = j0;
@@ -887,39 +892,52 @@ extern "C" int lxgb_lu32_inverse(int32_t n, const float* lu, const int32_t* piv,
     g.w = w;
     g.c_begin = c_begin;
     g.c_end = c_end;
-    g.b0 = split ? bh : xt;
-    g.b1 = bl;
+    g.b0 = o.b;
+    g.b1 = o.bl;
     g.a_src = a_src;
     g.na = na;
-    g.a0 = ah;
-    g.a1 = al;
+    g.a0 = o.ah;
+    g.a1 = o.al;
     return g;
   };
-  auto update = [&](int rows, int cols, int nb, const float* a_src, float* c) {
+  auto update = [&](const Operands& o, int rows, int cols, int nb, const float* a_src, float* c,
+                    int beside) {
+    if (rows <= 0) return (int)LXGB_SUCCESSFUL;
     if (split)
-      return gemm_tf32_nt_split(rows, cols, nb, ah, al, kInvNB, bh, bl, kInvNB, c, n, -1.0f, 1.0f,
-                                err, st);
-    return gemm_tf32_nt(rows, cols, nb, a_src, n, xt, kInvNB, c, n, -1.0f, 1.0f, err, st);
+      return gemm_tf32_nt_split(rows, cols, nb, o.ah, o.al, kInvNB, o.b, o.bl, kInvNB, c, n, -1.0f,
+                                1.0f, err, st, beside);
+    return gemm_tf32_nt(rows, cols, nb, a_src, n, o.b, kInvNB, c, n, -1.0f, 1.0f, err, st, beside);
   };
-  // L^{-1}: top to bottom.  Row block j of W = L^{-1} has nonzeros in
-  // columns < j0 + nb only.  (Skipped when linv is NULL: the square QR needs
-  // only R^{-1}.)
-  for (int j0 = 0; linv && j0 < n; j0 += kInvNB) {
-    const int nb = min(kInvNB, n - j0);
-    const int ncols = j0 + nb, m2 = n - ncols;
-    const float* a21 = lu + (int64_t)ncols * n + j0;
-    int rc = launch_block_row<1>(precision, block(linv, j0, nb, 0, ncols, a21, m2), st);
-    if (!rc && m2 > 0) rc = update(m2, ncols, nb, a21, linv + (int64_t)ncols * n);
-    if (rc) return rc;
-  }
-  // U^{-1}: bottom to top.  Row block j of W = U^{-1} has nonzeros in
-  // columns >= j0 only.  (Skipped when uinv is NULL: a Cholesky factor forms
-  // it from L^{-1} with lxgb_chol32_uinv.)
-  for (int j0 = ((n - 1) / kInvNB) * kInvNB; uinv && j0 >= 0; j0 -= kInvNB) {
-    const int nb = min(kInvNB, n - j0);
-    const float* a01 = lu + j0;  // rows [0, j0), columns [j0, j0 + nb)
-    int rc = launch_block_row<2>(precision, block(uinv, j0, nb, j0, n, a01, j0), st);
-    if (!rc && j0 > 0) rc = update(j0, n - j0, nb, a01, uinv + j0);
+  // L^{-1} top to bottom: row block j of W = L^{-1} has nonzeros in columns
+  // < j0 + nb only.  U^{-1} bottom to top: row block j has nonzeros in columns
+  // >= j0 only.  Either may be NULL: the square QR needs only R^{-1}, and a
+  // Cholesky factor forms U^{-1} from L^{-1} with lxgb_chol32_uinv.  Both together
+  // go step by step, the update of one beside the other's block row: 0.88 ms at n =
+  // 2048, 2.43 at 4096, 9.2 at 8192, against 1.40, 3.27 and 10.5 one after the other.
+  const int steps = (n + kInvNB - 1) / kInvNB;
+  auto update_l = [&](int s, int beside) {
+    const int j0 = s * kInvNB, nb = min(kInvNB, n - j0), ncols = j0 + nb;
+    return update(ol, n - ncols, ncols, nb, lu + (int64_t)ncols * n + j0,
+                  linv + (int64_t)ncols * n, beside);
+  };
+  auto update_u = [&](int s, int beside) {
+    const int j0 = (steps - 1 - s) * kInvNB, nb = min(kInvNB, n - j0);
+    return update(ou, j0, n - j0, nb, lu + j0, uinv + j0, beside);
+  };
+  for (int s = 0; s < steps; ++s) {
+    int rc = LXGB_SUCCESSFUL;
+    if (linv) {
+      const int j0 = s * kInvNB, nb = min(kInvNB, n - j0), ncols = j0 + nb;
+      rc = launch_block_row<1>(precision, block(ol, linv, j0, nb, 0, ncols,
+                                                lu + (int64_t)ncols * n + j0, n - ncols), st);
+      if (!rc && uinv && s > 0) rc = update_u(s - 1, kBesideRow);
+      if (!rc && !uinv) rc = update_l(s, 0);
+    }
+    if (!rc && uinv) {
+      const int j0 = (steps - 1 - s) * kInvNB, nb = min(kInvNB, n - j0);
+      rc = launch_block_row<2>(precision, block(ou, uinv, j0, nb, j0, n, lu + j0, j0), st);
+      if (!rc) rc = linv ? update_l(s, kBesideRow) : update_u(s, 0);
+    }
     if (rc) return rc;
   }
   return check_launch("lu32_inverse");

@@ -574,7 +574,7 @@ extern "C" int lxgb_getrf_f32_tc(int32_t n, const double* a64, float* lu, int32_
   float* bh = reinterpret_cast<float*>(wb + 3 * blk);
   float* bl = reinterpret_cast<float*>(wb + 4 * blk);
   // A22 -= L21 U12 on columns [c0, c0 + cols) of the matrix, after step j0
-  auto update = [&](int j0, int c0, int cols, bool beside) -> int {
+  auto update = [&](int j0, int c0, int cols, int beside) -> int {
     const int r0 = j0 + kLu32NB, rows = n - r0;
     float* c = lu + (int64_t)r0 * n + c0;
     const int64_t at = (int64_t)(c0 - r0) * kLu32NB;  // in the operand from U12
@@ -597,13 +597,13 @@ extern "C" int lxgb_getrf_f32_tc(int32_t n, const double* a64, float* lu, int32_
     // leaves 136 SMs idle and is the longer of the two from n = 8192 down: 14.4
     // ms for the factor at n = 8192, 6.4 at 4096, 2.99 at 2048, against 18.9,
     // 7.0 and 3.09 with panel and update one after the other.
-    if (j0 > 0 && j0 + nb < n) rc = update(j0 - kLu32NB, j0 + nb, n - j0 - nb, true);
+    if (j0 > 0 && j0 + nb < n) rc = update(j0 - kLu32NB, j0 + nb, n - j0 - nb, kBesidePanel);
     // interchanges, U12 in place and the operands of the update
     if (!rc)
       rc = lu32_block_row(precision, n, j0, nb, lu, piv, ah, al, precision == 0 ? bt : bh, bl, st);
     // the next panel's columns
     const int n2 = n - j0 - nb;
-    if (!rc && n2 > 0) rc = update(j0, j0 + nb, min(kLu32NB, n2), false);
+    if (!rc && n2 > 0) rc = update(j0, j0 + nb, min(kLu32NB, n2), 0);
     if (rc) return rc;
   }
   return check_launch("getrf_f32_tc");

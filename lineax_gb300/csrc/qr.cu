@@ -1342,7 +1342,7 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
   float* w2 = reinterpret_cast<float*>(wb + 3 * vb + wpb);
   const int nn = (int)n;
   // C -= W' V on `rows` rows from c, W' from w2's row w0 on
-  auto update = [&](float* c, int w0, int rows, int j0, int nb, bool beside) -> int {
+  auto update = [&](float* c, int w0, int rows, int j0, int nb, int beside) -> int {
     return gemm_tf32_nt(rows, (int)(m - j0), nb, w2 + (int64_t)w0 * kQrNB, kQrNB,
                         vcols2[(j0 / kQrNB) & 1] + (int64_t)j0 * kQrNB, kQrNB, c + j0, m, -1.0f,
                         1.0f, err, st, beside);
@@ -1358,7 +1358,7 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
                                   (int)chunk, used, err, st);
     if (rc0) return rc0;
     qr32_wt_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(rows, nb, used, wpart, Tp, w2);
-    return update(c, 0, now, j0, nb, false);
+    return update(c, 0, now, j0, nb, 0);
   };
   // (w2 is one workspace: with a separate q it is taken at once)
   const bool ahead = q == nullptr || joint;
@@ -1382,7 +1382,7 @@ static int geqrf_f32_tc_driver(int64_t m, int64_t n, const double* a, float* h, 
     int rc = 0;
     float* rest = h + (int64_t)(j0 + nb) * m;
     if (ahead && j0 > 0 && n2 + tail > 0)
-      rc = update(rest, nb, n2 + tail, j0 - kQrNB, kQrNB, true);
+      rc = update(rest, nb, n2 + tail, j0 - kQrNB, kQrNB, kBesidePanel);
     // trailing rows: with `ahead` the next panel's now, the others beside it
     if (!rc && n2 + tail > 0)
       rc = apply(rest, n2 + tail, ahead && n2 > 0 ? min(kQrNB, n2) : n2 + tail, j0, nb, Tp);

@@ -651,8 +651,8 @@ __global__ void scale_c_kernel(int M, int N, float* C, int64_t ldc, float beta) 
 // can be addressed by a tensor map; 0: one CTA per 128×128 tile.
 static int g_gemm_persistent = 1;
 
-// SMs left to the panel kernel by a product launched beside it: the largest
-// cluster a panel takes.
+// SMs left to a panel by a product launched beside it: the largest cluster that a
+// panel takes.
 constexpr int kBesideSms = 16;
 
 // Persistent launch; returns -1 when C cannot be addressed by a tensor map
@@ -661,7 +661,7 @@ template <int MODE, class Cfg>
 static int gemm_persistent_cfg(int M, int N, int K, const void* A, const void* Al, int64_t lda,
                                const void* B, const void* Bl, int64_t ldb, float* C, int64_t ldc,
                                float alpha, float beta, int* err, cudaStream_t st,
-                               int lower = 0, bool beside = false) {
+                               int lower = 0, int beside = 0) {
   constexpr bool BF = MODE == 2;
   if (!g_gemm_persistent) return -1;
   if ((((uintptr_t)C) & 15) != 0 || (ldc % 4) != 0) return -1;
@@ -683,7 +683,7 @@ static int gemm_persistent_cfg(int M, int N, int K, const void* A, const void* A
     if (rc) return rc;
   }
   const int64_t tiles = (int64_t)((M + kTcM - 1) / kTcM) * ((N + Cfg::BN - 1) / Cfg::BN);
-  const int ctas = sm_count() - (beside ? kBesideSms : 0);
+  const int ctas = sm_count() - (beside == kBesidePanel ? kBesideSms : 0);
   const int grid = (int)(tiles < ctas ? tiles : ctas);
   auto kern = gemm_nt_persistent_kernel<MODE, Cfg>;
   LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg::SMEM),
@@ -704,7 +704,7 @@ template <int MODE>
 static int gemm_persistent(int M, int N, int K, const void* A, const void* Al, int64_t lda,
                            const void* B, const void* Bl, int64_t ldb, float* C, int64_t ldc,
                            float alpha, float beta, int* err, cudaStream_t st,
-                           bool beside = false) {
+                           int beside = 0) {
   const int kstage = MODE == 2 ? 2 * kTcK : kTcK;
   const bool short_k = beta != 0.0f && K <= 2 * kstage;
   if constexpr (MODE == 0) {
@@ -727,7 +727,7 @@ static int gemm_persistent(int M, int N, int K, const void* A, const void* Al, i
 
 int gemm_tf32_nt_split(int M, int N, int K, const float* A, const float* Al, int64_t lda,
                        const float* B, const float* Bl, int64_t ldb, float* C, int64_t ldc,
-                       float alpha, float beta, int* err, cudaStream_t st, bool beside) {
+                       float alpha, float beta, int* err, cudaStream_t st, int beside) {
   if (M <= 0 || N <= 0) return LXGB_SUCCESSFUL;
   if (K == 0) {  // C = beta * C
     const int64_t total = (int64_t)M * N;
@@ -805,7 +805,7 @@ int gemm_tf32_nt_split_lower(int M, int K, const float* A, const float* Al, int6
 
 int gemm_tf32_nt(int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb,
                  float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
-                 bool beside) {
+                 int beside) {
   return gemm_tf32_nt_split(M, N, K, A, nullptr, lda, B, nullptr, ldb, C, ldc, alpha, beta, err,
                             st, beside);
 }
@@ -838,7 +838,7 @@ int gemm_tf32_nt_splitk(int M, int N, int K, const float* A, int64_t lda, const 
 // strides multiples of 8 elements, 16-byte aligned), FP32 C.
 int gemm_bf16_nt(int M, int N, int K, const void* A, int64_t lda, const void* B, int64_t ldb,
                  float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
-                 bool beside) {
+                 int beside) {
   if (M <= 0 || N <= 0) return LXGB_SUCCESSFUL;
   if (K == 0) {
     const int64_t total = (int64_t)M * N;

@@ -5,17 +5,19 @@
 #include "common.cuh"
 
 namespace lxgb {
-// beside: the kernel before it on the stream is a panel that lets its successor
-// start at once and touches nothing of this product; the product then runs on
-// the SMs the panel leaves and ends no earlier than the panel.  (Without the
-// persistent kernel it runs after the panel.)
+// beside: the kernel before it on the stream lets its successor start at once and
+// touches nothing of this product, which then runs beside it and ends no earlier:
+// kBesidePanel on the SMs that a panel's cluster leaves, kBesideRow on all (a block
+// row, whose CTAs are short and leave one by one).  Without the persistent kernel
+// the product runs after the other.
+constexpr int kBesidePanel = 1, kBesideRow = 2;
 int gemm_tf32_nt(int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb,
                  float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
-                 bool beside = false);
+                 int beside = 0);
 // 3xTF32 when Al and Bl (the lo parts) are given, plain TF32 otherwise.
 int gemm_tf32_nt_split(int M, int N, int K, const float* A, const float* Al, int64_t lda,
                        const float* B, const float* Bl, int64_t ldb, float* C, int64_t ldc,
-                       float alpha, float beta, int* err, cudaStream_t st, bool beside = false);
+                       float alpha, float beta, int* err, cudaStream_t st, int beside = 0);
 // C = alpha A Aᵀ + beta C on the tiles holding C's lower triangle (M×M),
 // 3xTF32 when Al is given; the full product when tiles cannot be skipped.
 int gemm_tf32_nt_split_lower(int M, int K, const float* A, const float* Al, int64_t lda, float* C,
@@ -35,5 +37,5 @@ int gemm_tf32_nt_splitk(int M, int N, int K, const float* A, int64_t lda, const 
 // BF16 operands (kind::f16, FP32 accumulation); A and B hold __nv_bfloat16.
 int gemm_bf16_nt(int M, int N, int K, const void* A, int64_t lda, const void* B, int64_t ldb,
                  float* C, int64_t ldc, float alpha, float beta, int* err, cudaStream_t st,
-                 bool beside = false);
+                 int beside = 0);
 }
