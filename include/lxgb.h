@@ -108,11 +108,10 @@ int lxgb_potrf_ragged_f64(int64_t batch, int32_t max_n, const int32_t* n,
                           void* stream);
 
 /* Upper Cholesky A = Uᵀ U of one n×n SPD matrix (row stride lda), in place,
- * on many CTAs: 64-row block rows, the diagonal block by one CTA, the block
- * row by column-parallel substitution, the trailing matrix by
- * lxgb_syrk_f64's update.  Every element receives the same FMA chain as in
- * lxgb_potrf_ragged_f64, so the two return the same bits; the strictly lower
- * triangle is zeroed.  *info (device) = 0, or k+1 for the first pivot that is
+ * on many CTAs by 32-row block rows.  Every element receives the same FMA
+ * chain as in lxgb_potrf_ragged_f64, so the two return the same bits; the
+ * strictly lower triangle is scratch and is zeroed in the end.  *info (device)
+ * = 0, or k+1 for the first pivot that is
  * not positive (the factor is then unspecified).  Replaces
  * jax.scipy.linalg.cho_factor(lower=False) at lineax/_solver/cholesky.py:60
  * for one large matrix. */

@@ -127,6 +127,12 @@ syrk_f64_kernel(int trans, int64_t n, int64_t k, const double* __restrict__ a, i
 // (149 us) before.  The whole factorisation 8.4 to 2.2 ms.
 // The operations on each element, and their order, are cta_potrf_upper's:
 // row k scaled by 1 / sqrt(a_kk), then one FMA per later row, k ascending.
+// Except for the last block, the factored block does not go back to its place: a CTA
+// that starts late (more of them than SMs, or SMs taken by other streams) still
+// reads the block unfactored.  CTA 0 keeps it below the diagonal, which no kernel
+// of the sweep reads: off-diagonal entries transposed into the block's own lower
+// triangle, its diagonal in the 32 entries of the row below the block;
+// potrf_finish_kernel moves both.
 constexpr int kPoOwners = 6;
 constexpr int kPoRows = (kPoNB + kPoOwners - 1) / kPoOwners;
 
@@ -210,9 +216,17 @@ potrf_row_kernel(int64_t n, double* __restrict__ a, int64_t lda, int64_t j0, int
   }
   if (blockIdx.x == 0) {
     __syncthreads();
-    for (int t = tid; t < nb * nb; t += 256) {
-      const int i = t / nb, j = t % nb;
-      if (j >= i) a[(j0 + i) * lda + j0 + j] = U[i][j];
+    if (j0 + nb == n) {                                // no CTA beside this one
+      for (int t = tid; t < nb * nb; t += 256) {
+        const int i = t / nb, j = t % nb;
+        if (j >= i) a[(j0 + i) * lda + j0 + j] = U[i][j];
+      }
+    } else {                                           // (nb is kPoNB)
+      for (int t = tid; t < kPoNB * kPoNB; t += 256) {
+        const int i = t % kPoNB, j = t / kPoNB;
+        if (j > i) a[(j0 + j) * lda + j0 + i] = U[i][j];
+      }
+      if (tid < kPoNB) a[(j0 + kPoNB) * lda + j0 + tid] = U[tid][tid];
     }
     if (tid == 0 && bad != 0 && info[0] == 0) info[0] = (int32_t)(j0 + bad);
   }
@@ -313,9 +327,35 @@ potrf_trailing_kernel(int64_t n, double* a, int64_t lda, int64_t j0, int nb, int
   pdl_wait();
 }
 
-__global__ void zero_lower_kernel(int64_t n, double* __restrict__ a, int64_t lda) {
-  for (int64_t i = blockIdx.x; i < n; i += gridDim.x)
-    for (int64_t j = threadIdx.x; j < i; j += blockDim.x) a[i * lda + j] = 0.0;
+// The block columns of the finished factor: the diagonal block that
+// potrf_row_kernel left below the diagonal into its place (but for the last block,
+// which is there), and zeros below the diagonal.  CTA (b, y): block b, rows
+// [kPoFinish y, kPoFinish (y + 1)) below it; y = 0 also the block.
+constexpr int kPoFinish = 256;
+
+__global__ void __launch_bounds__(256)
+potrf_finish_kernel(int64_t n, double* __restrict__ a, int64_t lda) {
+  __shared__ double U[kPoNB][kPoNB + 1];
+  const int64_t j0 = (int64_t)blockIdx.x * kPoNB;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t s = j0 + kPoNB;                        // first row below the block
+  if (blockIdx.y == 0) {
+    const bool moved = s < n;
+    if (moved) {
+      for (int i = warp; i < kPoNB; i += 8)
+        U[i][lane] = (lane < i) ? a[(j0 + i) * lda + j0 + lane]
+                                : (lane == i ? a[s * lda + j0 + lane] : 0.0);
+      __syncthreads();
+    }
+    for (int i = warp; i < kPoNB && j0 + i < n; i += 8) {
+      double* row = a + (j0 + i) * lda + j0;
+      if (lane < i) row[lane] = 0.0;
+      else if (moved) row[lane] = U[lane][i];
+    }
+    __syncthreads();                                   // the row below was read above
+  }
+  const int64_t lo = s + (int64_t)blockIdx.y * kPoFinish;
+  for (int64_t i = lo + warp; i < n && i < lo + kPoFinish; i += 8) a[i * lda + j0 + lane] = 0.0;
 }
 
 __global__ void set_info_kernel(int32_t* info) { info[0] = 0; }
@@ -379,7 +419,9 @@ extern "C" int lxgb_potrf_f64(int64_t n, double* a, int64_t lda, int32_t* info, 
                                0, st, 1, n, a, lda, j0, nb),
                     "potrf: next row update launch");
   }
-  const int64_t g = (n < 4096) ? n : 4096;
-  zero_lower_kernel<<<(unsigned)g, 256, 0, st>>>(n, a, lda);
+  const int64_t blocks = (n + kPoNB - 1) / kPoNB;
+  const int64_t below = n > kPoNB ? (n - kPoNB + kPoFinish - 1) / kPoFinish : 1;
+  LXGB_REQUIRE(below <= 65535, "potrf: n too large");
+  potrf_finish_kernel<<<dim3((unsigned)blocks, (unsigned)below), 256, 0, st>>>(n, a, lda);
   return check_launch("potrf_f64");
 }

@@ -187,3 +187,48 @@ def test_potrf_block_edges(dev, n):
     _ffi.call("lxgb_potrf_ragged_f64", 1, n, _ffi.ptr(meta), _ffi.ptr(off), _ffi.ptr(u_one),
               _ffi.ptr(info), _ffi.stream_handle(dev))
     assert torch.equal(u, u_one)
+
+
+@pytest.mark.parametrize("n", [9760, 9761, 10240, 16384])
+def test_potrf_more_block_row_ctas_than_sms(dev, n):
+    """Block rows whose CTAs (64 columns each, one per SM) run in more than one
+    wave: a CTA of the second wave starts when the first ones have finished.
+    Every entry of UᵀU is a sum of at most n products and U comes from n updates
+    and a scaling, so |A - UᵀU|_ij <= 2 (n + 4) u (|U|ᵀ|U|)_ij, and by Cauchy-Schwarz
+    (|U|ᵀ|U|)_ij <= sqrt(a_ii a_jj) (1 + (n + 4) u)."""
+    gen = torch.Generator(device=dev).manual_seed(n)
+    a = torch.rand(n, n, dtype=torch.float64, device=dev, generator=gen)
+    a += a.T.clone()
+    a.diagonal().add_(2.0 * n)
+    diag = a.diagonal().clone()
+    rows = torch.unique(torch.cat([torch.arange(0, n, 97), torch.arange(40),
+                                   torch.arange(n - 70, n)])).to(dev)
+    rows_a = a[rows].clone()
+    u = _dense.cho_factor(a)
+    del a
+    got = torch.zeros_like(rows_a)
+    for k in range(0, n, 2048):                  # rows of UᵀU
+        got += u[k:k + 2048, rows].T @ u[k:k + 2048]
+    eps = 2.0 ** -53
+    bound = 2 * (n + 4) * eps * torch.sqrt(diag[rows, None] * diag[None, :]) * 1.01
+    assert bool(((got - rows_a).abs() <= bound).all())
+    assert int(torch.count_nonzero(u[-1, :-1])) == 0 and int(torch.count_nonzero(u[:, 0])) == 1
+
+
+@pytest.mark.parametrize("n", [700, 1531])
+def test_potrf_same_bits_beside_another_stream(dev, n):
+    """The factor while another stream's products hold the SMs, so that CTAs of a
+    block row start at different times: the bits of the factor made alone."""
+    rng = np.random.default_rng(n)
+    a = t(spd(rng, n), dev)
+    alone = _dense.cho_factor(a)
+    w = torch.randn(6144, 6144, dtype=torch.bfloat16, device=dev)
+    other = torch.cuda.Stream(dev)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(other):
+            for _ in range(8):
+                w @ w
+        u = _dense.cho_factor(a)
+        assert torch.equal(u, alone)
+    torch.cuda.synchronize()
