@@ -553,7 +553,8 @@ gm_step_cluster_kernel(int n, GmWork w, int cur, int kk, double* __restrict__ wv
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool live = gm_live(w, c, cur) && !w.fl[c * 8 + 2];
   if (rank == 0 && tid == 0) on[c] = live;
-  if (!live) return;  // uniform over the cluster: the flags change after its first barrier
+  if (!live) return;  // uniform over the cluster: the flags change at its end
+  cluster.barrier_arrive();  // waited for before the first remote store: every CTA runs by then
   const int per = (n + C - 1) / C, i0 = rank * per, m = max(0, min(per, n - i0));
   double* V = w.V + (int64_t)c * (R + 1) * n + i0;
   double* wc = wv + (int64_t)c * n + i0;
@@ -576,6 +577,7 @@ gm_step_cluster_kernel(int n, GmWork w, int cur, int kk, double* __restrict__ wv
     if (lane == 0) loc[j] = t;
   }
   __syncthreads();
+  cluster.barrier_wait();
   for (int e = tid; e < C * (kk + 2); e += kGmClusterThreads) {
     const int dst = e / (kk + 2), j = e - dst * (kk + 2);
     *cluster.map_shared_rank(&sp[rank][j], dst) = loc[j];

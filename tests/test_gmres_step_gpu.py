@@ -51,3 +51,40 @@ def test_arnoldi_step_against_gram_schmidt(dev, n, k, restart):
             scale = np.linalg.norm(w[c]) / np.linalg.norm(u)
             assert np.max(np.abs(got[c] - ref)) <= 4 * (j + 2) * n * 2.0 ** -53 * scale
         vs.append(got)
+
+
+@pytest.mark.parametrize("n,k", [(130, 3), (300, 40), (5000, 9)])
+def test_arnoldi_step_same_bits_beside_another_stream(dev, n, k):
+    """The first step of a cycle (little work before the CTAs of a cluster exchange
+    their sums) while another stream's products hold the SMs: the bits of the step
+    made alone."""
+    lib = _ffi.load()
+    restart = 4
+    nb = int(lib.lxgb_gmres_workspace_size(k, n, restart))
+    buf = torch.zeros(nb // 8 + 64, dtype=torch.float64, device=dev)
+    work = buf[(-buf.data_ptr() % 256) // 8:]
+    st = torch.cuda.current_stream().cuda_stream
+    rng = np.random.default_rng(n)
+    r = torch.tensor(rng.standard_normal((k, n)), device=dev)
+    w = torch.tensor(rng.standard_normal((k, n)), device=dev)
+    on = torch.empty(k, dtype=torch.int32, device=dev)
+    off = int(lib.lxgb_gmres_basis_offset(k, n, restart, 1)) // 8
+
+    def step():
+        _ffi.call("lxgb_gmres_init", k, n, restart, _ffi.ptr(work), nb, st)
+        _ffi.call("lxgb_gmres_cycle_begin", k, n, restart, 0, _ffi.ptr(r), _ffi.ptr(work), nb, st)
+        _ffi.call("lxgb_gmres_arnoldi", k, n, restart, 0, 0, _ffi.ptr(w.clone()), _ffi.ptr(on),
+                  _ffi.ptr(work), nb, st)
+        v = torch.as_strided(work, (k, n), ((restart + 1) * n, 1), work.storage_offset() + off)
+        return v.clone()
+
+    alone = step()
+    g = torch.randn(6144, 6144, dtype=torch.bfloat16, device=dev)
+    other = torch.cuda.Stream(dev)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(other):
+            for _ in range(4):
+                g @ g
+        assert torch.equal(step(), alone)
+    torch.cuda.synchronize()
