@@ -57,18 +57,19 @@ __device__ __forceinline__ bool ts_moderate(double x, bool zero_ok) {
 // so a step is v_l -= d[t] v_t on unscaled v and x_l = v_l / op(l, l) at the
 // end: a shuffle and an FMA per step.  Otherwise (entries whose scaling could
 // overflow or underflow, zeros and non-finite values on the diagonal) every
-// unknown is divided in turn.
+// unknown is divided in turn.  Lanes already solved take no part in a step, so a
+// non-finite unknown leaves them alone.
 __device__ __forceinline__ double ts_solve32(double v, const double (&d)[32], double dd,
                                              double rinv, bool scaled) {
+  const int lane = threadIdx.x & 31;
   if (scaled) {
 #pragma unroll
     for (int t = 0; t < 31; ++t) {
       const double vt = __shfl_sync(0xffffffffu, v, t);
-      v = fma(-d[t], vt, v);  // d[t] = 0 for t >= lane
+      if (lane > t) v = fma(-d[t], vt, v);
     }
     return v * rinv;
   }
-  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int t = 0; t < 32; ++t) {
     double xt = (lane == t) ? v / dd : 0.0;

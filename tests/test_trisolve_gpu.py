@@ -76,3 +76,30 @@ def test_getrs_interchanges(dev, n, kind):
             ref[..., [i, piv[i]]] = ref[..., [piv[i], i]]
         got = _dense.lu_solve_batched(lu, pv, _t(b, dev), trans=trans).cpu().numpy()
         np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("lower,trans", [(True, False), (False, False), (True, True),
+                                         (False, True)])
+@pytest.mark.parametrize("unit", [False, True])
+@pytest.mark.parametrize("n", [40, 65, 300, 2100])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_trsm_non_finite_right_hand_side(dev, n, lower, trans, unit, bad):
+    """A non-finite b_k with finite, well-scaled entries: the unknowns solved before
+    it have the bits of the finite solve, x_k is b_k (a positive diagonal keeps its
+    sign), those after it are not finite.  One vector, and as many as take the other
+    path."""
+    rng = np.random.default_rng(n)
+    m = _t(rng.uniform(0.5, 1.0, (n, n)) / n, dev)
+    m.diagonal().add_(1.0)
+    b = rng.standard_normal(n)
+    order = np.arange(n) if lower != trans else np.arange(n)[::-1]
+    for k in (0, 7, n // 2, n - 1):
+        b2 = b.copy()
+        b2[order[k]] = bad
+        for nv in (1, 40):
+            args = dict(lower=lower, trans=trans, unit=unit)
+            good = _dense.trsv(m, _t(np.tile(b, (nv, 1)), dev), **args).cpu().numpy()
+            x = _dense.trsv(m, _t(np.tile(b2, (nv, 1)), dev), **args).cpu().numpy()
+            np.testing.assert_array_equal(x[:, order[:k]], good[:, order[:k]])
+            np.testing.assert_array_equal(x[:, order[k]], np.full(nv, bad))
+            assert not np.isfinite(x[:, order[k + 1:]]).any()
