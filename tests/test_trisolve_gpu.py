@@ -103,3 +103,22 @@ def test_trsm_non_finite_right_hand_side(dev, n, lower, trans, unit, bad):
             np.testing.assert_array_equal(x[:, order[:k]], good[:, order[:k]])
             np.testing.assert_array_equal(x[:, order[k]], np.full(nv, bad))
             assert not np.isfinite(x[:, order[k + 1:]]).any()
+
+
+@pytest.mark.parametrize("n", [1, 40, 65, 300, 2100])
+@pytest.mark.parametrize("lower", [True, False])
+def test_trsm_diagonal_matrix_is_correctly_rounded(dev, n, lower):
+    """With a diagonal T each unknown is one quotient, rounded once: the bits of
+    b / t, for three vectors and for as many as take the other path."""
+    rng = np.random.default_rng(n)
+    d = rng.uniform(1.0, 100.0, n).round(1)
+    b = rng.standard_normal((40, n))
+    b[0] = d                                     # x = 1
+    b[1] = np.resize([0.0, -0.0, 5e-324, -1e-310, 1e300, -1.7e308, 3e-200, 7e180], n)
+    b[2] = -0.0
+    for nv in (3, 40):
+        x = _dense.trsv(_t(np.diag(d), dev), _t(b[:nv], dev), lower=lower, trans=False,
+                        unit=False).cpu().numpy()
+        np.testing.assert_array_equal(x, b[:nv] / d)
+        # (the zeros of T turn the sign of a zero after the first unknown)
+        assert np.signbit(x[2, 0 if lower else n - 1])
