@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "df.cuh"
+#include "swaps.cuh"
 #include "tc_gemm.cuh"
 
 namespace lxgb {
@@ -31,77 +32,23 @@ constexpr int kGvRhs = 16;     // right-hand sides per CTA of the products
 constexpr int kPermMaxN = 25600;
 constexpr int kPermRows = 25;  // rows per thread of the 1024 at kPermMaxN
 
-// (P b)_i = b[perm[i]]: the getrf row interchanges composed into one gather.
-// Output i is final after interchange i, so its source is found by walking
-// back through the earlier interchanges with the same partner (as the FP64
-// solve's getrs_perm_kernel does on values): a linked list per partner, a few
-// links per row, instead of one thread running n dependent exchanges (327 us
-// at n = 8192).
-__global__ void perm_from_swaps_kernel(int n, const int32_t* __restrict__ piv,
-                                       int32_t* __restrict__ perm) {
+// (P b)_i = b[perm[i]]: the getrf row interchanges composed into one gather
+// (swaps.cuh).  The third array of the walk lives in the output until every row's source
+// is known.  One thread running the n dependent exchanges took 327 us at n = 8192.
+__global__ void __launch_bounds__(1024)
+perm_from_swaps_kernel(int n, const int32_t* __restrict__ piv, int32_t* perm) {
   extern __shared__ int32_t sp[];
-  int32_t* head = sp;            // last-inserted interchange with partner q
-  int32_t* next = sp + n;        // its list
-  int32_t* last = perm;          // the latest interchange with partner k (all < k); see below
-  int odd = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) head[i] = -1;
-  __syncthreads();
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const int q = piv[j];
-    if (q < j || q >= n) odd = 1;
-    else if (q != j) next[j] = atomicExch(&head[q], j);
-  }
-  if (__syncthreads_or(odd)) {
-    // not a pivot sequence of getrf: in order, one thread
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sp[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < n; ++k) {
-        const int p = piv[k];
-        if (p != k && p >= 0 && p < n) {
-          const int t = sp[k];
-          sp[k] = sp[p];
-          sp[p] = t;
-        }
-      }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = sp[i];
-    return;
-  }
-  // `last` needs a third array: it lives in the output until every row has been
-  // walked (kPermRows rows per thread), then the sources replace it
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    int m = -1;
-    for (int j = head[k]; j >= 0; j = next[j]) m = max(m, j);
-    last[k] = m;
-  }
-  __syncthreads();
+  const SwapMode mode = swap_build(n, piv, sp, sp + n, perm, false);
   int src[kPermRows];
 #pragma unroll
   for (int u = 0; u < kPermRows; ++u) {
-    const int i = threadIdx.x + u * blockDim.x;
-    src[u] = 0;
-    if (i < n) {
-      const int q = piv[i];
-      int at = q, from = -1;
-      if (q == i) {
-        from = last[i];
-      } else {
-        for (int j = head[q]; j >= 0; j = next[j])
-          if (j < i) from = max(from, j);
-      }
-      while (from >= 0) {
-        at = from;
-        from = last[at];
-      }
-      src[u] = at;
-    }
+    const int i = threadIdx.x + u * (int)blockDim.x;
+    src[u] = i < n ? swap_source(mode, i, piv, sp, sp + n, perm) : 0;
   }
   __syncthreads();
 #pragma unroll
   for (int u = 0; u < kPermRows; ++u) {
-    const int i = threadIdx.x + u * blockDim.x;
+    const int i = threadIdx.x + u * (int)blockDim.x;
     if (i < n) perm[i] = src[u];
   }
 }

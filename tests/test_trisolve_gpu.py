@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from lineax_gb300 import _dense
+from lineax_gb300 import _dense, _ffi
 
 pytestmark = pytest.mark.gpu
 U = 2.0 ** -53
@@ -122,3 +122,78 @@ def test_trsm_diagonal_matrix_is_correctly_rounded(dev, n, lower):
         np.testing.assert_array_equal(x, b[:nv] / d)
         # (the zeros of T turn the sign of a zero after the first unknown)
         assert np.signbit(x[2, 0 if lower else n - 1])
+
+
+def _partners(kind, n, rng):
+    k = np.arange(n)
+    return {"random": k + (rng.random(n) * (n - k)).astype(int), "shift": np.minimum(k + 1, n - 1),
+            "last": np.full(n, n - 1), "halves": np.where(k < n // 2, n // 2 + k % 3, n - 1 - k % 2),
+            "any": rng.integers(0, n, n), "none": k}[kind].astype(np.int32)
+
+
+def _interchanged(b, piv, trans):
+    ref = b.copy()
+    for i in (range(len(piv)) if not trans else range(len(piv) - 1, -1, -1)):
+        if piv[i] != i:
+            ref[..., [i, piv[i]]] = ref[..., [piv[i], i]]
+    return ref
+
+
+@pytest.mark.parametrize("n", [1001, 11000])
+@pytest.mark.parametrize("kind", ["random", "shift", "last", "halves", "any"])
+def test_getrs_interchanges_long_lists_and_large_orders(dev, n, kind):
+    """The interchanges at the ends of the ranges of the one-gather path, with lists of
+    one partner longer than a row walks (they are then ordered by one warp) and with
+    chains of n links: exact, through identity factors."""
+    rng = np.random.default_rng(n)
+    piv = np.maximum(_partners(kind, n, rng), np.arange(n) if kind != "any" else 0).astype(np.int32)
+    b = rng.standard_normal((2, n))
+    lu = torch.eye(n, dtype=torch.float64, device=dev)
+    for trans in (0, 1):
+        got = _dense.lu_solve_batched(lu[None], torch.tensor(piv[None], device=dev), _t(b[None], dev),
+                                      trans=trans).cpu().numpy()[0]
+        np.testing.assert_array_equal(got, _interchanged(b, piv, trans))
+
+
+@pytest.mark.parametrize("n", [64, 1028, 8192, 20000])
+@pytest.mark.parametrize("kind", ["random", "shift", "last", "halves", "any"])
+def test_lu32_interchanges_as_one_gather(dev, n, kind):
+    """The gather that lxgb_lu32_inverse returns, for the same sequences."""
+    rng = np.random.default_rng(n)
+    piv = np.maximum(_partners(kind, n, rng), np.arange(n) if kind != "any" else 0).astype(np.int32)
+    lib = _ffi.load()
+    lu, linv = (torch.eye(n, dtype=torch.float32, device=dev) for _ in range(2))
+    perm = torch.empty(n, dtype=torch.int32, device=dev)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    nb = int(lib.lxgb_lu32_inverse_workspace_size(n, 0))
+    work = torch.empty(nb // 8 + 1, dtype=torch.float64, device=dev)
+    pv = torch.tensor(piv, device=dev)
+    _ffi.call("lxgb_lu32_inverse", n, _ffi.ptr(lu), _ffi.ptr(pv), _ffi.ptr(linv), None,
+              _ffi.ptr(perm), 0, _ffi.ptr(err), _ffi.ptr(work), nb,
+              torch.cuda.current_stream().cuda_stream)
+    np.testing.assert_array_equal(perm.cpu().numpy(), _interchanged(np.arange(n), piv, 0))
+
+
+def test_getrs_interchanges_time_does_not_grow_with_the_list(dev):
+    """All rows with one partner, and a cyclic shift: the solve takes no longer than
+    without interchanges by more than a quarter (walking every list from every row it
+    took 1.3 times as long and more; a row walks at most 64 links)."""
+    n = 11000
+    lu = torch.eye(n, dtype=torch.float64, device=dev)
+    b = torch.ones(1, 1, n, dtype=torch.float64, device=dev)
+
+    def ms(kind):
+        piv = torch.tensor(_partners(kind, n, np.random.default_rng(0))[None], device=dev)
+        best = np.inf
+        for _ in range(6):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            _dense.lu_solve_batched(lu[None], piv, b, trans=0)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    none = ms("none")
+    for kind in ("last", "shift", "random"):
+        assert ms(kind) <= 1.25 * none
