@@ -902,25 +902,35 @@ int getrf_blocked(int n, double* a, int32_t* piv, int32_t* info, cudaStream_t st
 // vector, then two multi-CTA triangular solves (trisolve.cu).
 // ---------------------------------------------------------------------------
 constexpr int kPermThreads = 1024;
-constexpr int kPermMaxN = 11000;   // 20 bytes of shared memory per row
+constexpr int kPermRows = 19;                      // values per thread, in registers
+constexpr int kPermFew = 4;                        // and up to 4096 rows
+constexpr int kPermMaxN = 19200;                   // 12 bytes of shared memory per row
+static_assert(kPermMaxN <= kPermRows * kPermThreads, "a register per value");
 
-// x = P x (or Pᵀ x), one CTA per vector.
+// x = P x (or Pᵀ x), one CTA per vector: every value is read before the first is written.
+template <int ROWS>
 __global__ void __launch_bounds__(kPermThreads)
 getrs_perm_kernel(int n, const int32_t* __restrict__ piv, int64_t stride_piv,
                   double* __restrict__ b, int64_t stride_b, int trans) {
-  extern __shared__ double smem_x[];
-  double* x = smem_x;
-  int* head = reinterpret_cast<int*>(x + n);
-  int *next = head + n, *root = next + n;
+  extern __shared__ int smem_swaps[];
+  int *head = smem_swaps, *next = head + n, *root = next + n;
   const int32_t* p = piv + (int64_t)blockIdx.y * stride_piv;
   double* g = b + (int64_t)blockIdx.y * stride_b + (int64_t)blockIdx.x * n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = g[i];
   const SwapMode mode = swap_build(n, p, head, next, root, trans != 0);
   const bool scatter = trans && mode != kSwapInOrder;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int src = swap_source(mode, i, p, head, next, root);
-    if (scatter) g[src] = x[i];
-    else g[i] = x[src];
+  double v[ROWS];
+#pragma unroll
+  for (int u = 0; u < ROWS; ++u) {
+    const int i = threadIdx.x + u * (int)blockDim.x;
+    if (u * (int)blockDim.x >= n) break;           // uniform
+    v[u] = i < n ? g[scatter ? i : swap_source(mode, i, p, head, next, root)] : 0.0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < ROWS; ++u) {
+    const int i = threadIdx.x + u * (int)blockDim.x;
+    if (u * (int)blockDim.x >= n) break;
+    if (i < n) g[scatter ? swap_source(mode, i, p, head, next, root) : i] = v[u];
   }
 }
 
@@ -943,11 +953,12 @@ static int getrs_perm(int64_t batch, int n, int nrhs, const int32_t* piv, int64_
     getrs_swap_kernel<<<grid, 1, 0, st>>>(n, piv, stride_piv, b, stride_b, trans);
     return check_launch("getrs swap");
   }
-  const size_t smem = (size_t)n * (sizeof(double) + 3 * sizeof(int));
-  LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(getrs_perm_kernel), (int)smem),
+  const size_t smem = (size_t)n * 3 * sizeof(int);
+  auto fn = n <= kPermFew * kPermThreads ? getrs_perm_kernel<kPermFew> : getrs_perm_kernel<kPermRows>;
+  LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(fn), (int)smem),
                 "getrs: set smem");
   const int threads = n < kPermThreads ? (n + 31) / 32 * 32 : kPermThreads;
-  getrs_perm_kernel<<<grid, threads, smem, st>>>(n, piv, stride_piv, b, stride_b, trans);
+  fn<<<grid, threads, smem, st>>>(n, piv, stride_piv, b, stride_b, trans);
   return check_launch("getrs perm");
 }
 
