@@ -584,14 +584,16 @@ def qr_factor_tf32(a: torch.Tensor) -> QR32:
     return QR32(h, tau, t, rt, inv)
 
 
-def _upper_inverse(r_sq: torch.Tensor, err: torch.Tensor | None = None):
+def _upper_inverse(r_sq: torch.Tensor, err: torch.Tensor | None = None,
+                   out: torch.Tensor | None = None):
     """(R^{-1}, identity perm) for R in the upper triangle of a square FP32
     array (its lower triangle holds Householder vectors and is not read):
-    lxgb_lu32_inverse with linv NULL, 3xTF32 off-diagonal updates."""
+    lxgb_lu32_inverse with linv NULL, 3xTF32 off-diagonal updates.  R^{-1} goes
+    to `out` when given."""
     n = r_sq.shape[0]
     dev = r_sq.device
     piv = torch.arange(n, dtype=torch.int32, device=dev)
-    uinv = torch.empty((n, n), dtype=torch.float32, device=dev)
+    uinv = torch.empty((n, n), dtype=torch.float32, device=dev) if out is None else out
     perm = torch.empty(n, dtype=torch.int32, device=dev)
     err, check = _pipeline_err(err, dev)
     wbytes = int(_ffi.load().lxgb_lu32_inverse_workspace_size(n, 1))
@@ -698,7 +700,8 @@ def qr_square_tf32(a: torch.Tensor, err: torch.Tensor | None = None) -> SquareQR
         raise ValueError("qr_square_tf32 needs a square matrix with n a multiple of 4")
     dev = a64.device
     lib = _ffi.load()
-    # q right after h: their updates share the products
+    # q right after h: their updates share the products.  One allocation for both,
+    # which then holds the results: Qᵀ where h was, R^{-1} where q was.
     h, q = torch.empty((2, n, n), dtype=torch.float32, device=dev)
     tau = torch.empty(n, dtype=torch.float32, device=dev)
     t = torch.empty(max(1, int(lib.lxgb_geqrf_t_elems(n))), dtype=torch.float32, device=dev)
@@ -712,9 +715,9 @@ def qr_square_tf32(a: torch.Tensor, err: torch.Tensor | None = None) -> SquareQR
         raise RuntimeError("tensor-core pipeline timed out during the QR update")
     del work, t, tau
     r_sq = h.t().contiguous()  # R on and above the diagonal
-    del h
-    uinv, _ = _upper_inverse(r_sq, None if check else err)
-    return SquareQR32(q.t().contiguous(), uinv)
+    qt = h.copy_(q.t())
+    rinv, _ = _upper_inverse(r_sq, None if check else err, out=q)
+    return SquareQR32(qt, rinv)
 
 
 class QRPreconditioner(_BlockOperator):

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from lineax_gb300 import _ffi
+from lineax_gb300 import _ffi, mixed
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +44,26 @@ def test_qr32_q_joint_and_separate(dev, n):
     assert torch.all(err <= tol * torch.linalg.norm(a, dim=0))
     eye = torch.eye(n, dtype=torch.float64, device=dev)
     assert torch.all(torch.linalg.norm(qd.t() @ qd - eye, dim=0) <= 2 * tol)
+
+
+def test_qr_square_memory(dev):
+    """The square QR's peak beside A: h and q, then R as rows beside them and the
+    inversion's workspace (three matrices, not four); what stays is Qᵀ and R^{-1}."""
+    n = 2048
+    a = torch.tensor(np.random.default_rng(n).standard_normal((n, n)), device=dev)
+    lib = _ffi.load()
+    work = max(int(lib.lxgb_lu32_inverse_workspace_size(n, 1)),
+               int(lib.lxgb_geqrf_f32_tc_q_workspace_size(n, n)))
+    mixed.qr_square_tf32(a)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    before = torch.cuda.memory_allocated(dev)
+    torch.cuda.reset_peak_memory_stats(dev)
+    qr = mixed.qr_square_tf32(a)
+    small = 64 * n + 4 * 32 * n + (1 << 16)      # tau, T blocks, interchanges, rounding up
+    assert torch.cuda.max_memory_allocated(dev) - before <= 12 * n * n + work + small
+    assert torch.cuda.memory_allocated(dev) - before <= 8 * n * n + small
+    x = torch.linalg.solve(a, torch.ones(n, dtype=torch.float64, device=dev))
+    got = qr.rinv.double() @ (qr.qt.double() @ torch.ones(n, dtype=torch.float64, device=dev))
+    # (TF32 products: a preconditioner's accuracy)
+    assert torch.linalg.norm(got - x) <= 0.1 * torch.linalg.norm(x)
