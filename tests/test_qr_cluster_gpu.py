@@ -51,3 +51,26 @@ def test_qr_zero_columns_and_extreme_scales(dev):
     r = torch.triu(h[:, :40].T)
     err = (qta[:, :40].T - r).abs().amax(0)
     assert bool((err <= 20 * 40 * U * a.norm(dim=0)).all())
+
+
+@pytest.mark.parametrize("m,n", [(300, 40), (3001, 33)])
+@pytest.mark.parametrize("scale", [1e-150, 1e-130, 1e-100, 1e100, 1e150])
+def test_qr_columns_outside_the_reciprocal_root_range(dev, m, n, scale):
+    """Squared norms below and above the exponents for which a reflector is formed from
+    a reciprocal root (2^-823 and 2^877, a leading entry above 2^477): the error bound
+    of test_q_transposed_a_is_r, for those columns and their neighbours.  (300 squares of
+    1e-150 are normal numbers and of 1e150 finite.)"""
+    rng = np.random.default_rng(m)
+    a = rng.standard_normal((m, n))
+    a[:, 3:6] *= scale
+    a[:, n // 2:] *= scale
+    a = torch.tensor(a, device=dev)
+    h, tau, t = _dense.geqrf(a)
+    qta = _dense.ormqr(h, tau, t, a.T.contiguous(), trans=True)
+    want = torch.zeros(n, m, dtype=torch.float64, device=dev)
+    want[:, :n] = torch.triu(h[:, :n].T).T
+    err = ((qta - want) / scale).norm(dim=1) * scale if scale < 1 else (qta - want).norm(dim=1)
+    assert bool((err <= 20 * n * U * a.norm(dim=0)).all())
+    v = torch.tril(h.T, -1)
+    v[torch.arange(n), torch.arange(n)] = 1.0
+    assert bool(((tau * (v * v).sum(0) - 2).abs() <= 100 * U).all())
