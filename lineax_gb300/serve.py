@@ -144,7 +144,9 @@ def footprint(route: str, n: int, nrhs: int) -> int:
         return resident_bytes(route, n) + vec
     if route == "qr_mixed":
         return resident_bytes(route, n) + 20 * n4 * n4 + vec  # h, q, R, inversion work
-    return resident_bytes(route, n) + 5 * 4 * 64 * n4 + vec
+    # the inversion's workspace (lxgb_lu32_inverse_workspace_size: ten blocks of 64
+    # columns), then the refinement's vectors: x, b, residuals, a basis of nine
+    return resident_bytes(route, n) + 10 * 4 * 64 * n4 + 4096 + 3 * vec
 
 
 def resident_bytes(route: str, n: int) -> int:

@@ -162,3 +162,39 @@ def test_resident_of_a_timed_out_factor_is_dropped():
     assert srv.sched.lookup(7) is None and srv.sched.resident_total == 0
     srv.sched.forget(7)                                            # absent: no effect
     assert srv.sched.resident_total == 0
+
+
+@pytest.mark.parametrize("n", [512, 1030, 4096, 20000])
+def test_footprint_holds_the_inversion_workspace(lib_built, n):
+    """What the mixed routes are charged beside the resident operator covers the
+    library's workspaces for the factor and its inverses."""
+    from lineax_gb300 import _ffi
+
+    lib, n4 = _ffi.load(), (n + 3) // 4 * 4
+    need = max(int(lib.lxgb_lu32_inverse_workspace_size(n4, 1)),
+               int(lib.lxgb_getrf_f32_tc_workspace_size(n4, 1)),
+               int(lib.lxgb_potrf_f32_tc_workspace_size(n4)))
+    for route in ("lu_mixed", "chol_mixed"):
+        assert serve.footprint(route, n, 1) - serve.resident_bytes(route, n) >= need
+    need = 4 * n4 * n4 + max(int(lib.lxgb_lu32_inverse_workspace_size(n4, 1)),
+                             int(lib.lxgb_geqrf_f32_tc_q_workspace_size(n4, n4)))
+    assert serve.footprint("qr_mixed", n, 1) - serve.resident_bytes("qr_mixed", n) >= need
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["lu", "cholesky", "qr"])
+@pytest.mark.parametrize("n,k", [(1030, 1), (1030, 16), (2050, 16)])
+def test_footprint_covers_the_peak_of_a_mixed_request(dev, kind, n, k):
+    a = torch.randn(n, n, dtype=torch.float64, generator=torch.Generator().manual_seed(n))
+    a = a @ a.T / n + torch.eye(n) if kind == "cholesky" else a / n ** 0.5 + torch.eye(n)
+    b = torch.ones(k, n, dtype=torch.float64)
+    for _ in range(2):                           # the second without first-use allocations
+        srv = serve.SolveServer(device=dev, streams=1)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        before = torch.cuda.memory_allocated(dev)
+        torch.cuda.reset_peak_memory_stats(dev)
+        srv.run([serve.Request(0, kind, b, 0, a, 0.0)], realtime=False)
+        peak = torch.cuda.max_memory_allocated(dev) - before
+        del srv
+    assert peak <= serve.footprint(serve.route_of(kind, n, "mixed"), n, k)
