@@ -20,7 +20,8 @@
 // n = 128 and 767, and a diagonal and an update launch per block 549 and 1104
 // at n = 1000 and 2003.  getrs at n = 2003: 511 us against 2500 to 6200 (the
 // more interchanges, the longer: one thread ran them in order).
-// Few vectors of up to 2048 unknowns: trisolve_cluster_kernel below.
+// Few vectors of up to 2048 unknowns: trisolve_cluster_kernel below; many of up to
+// 4096: trisolve_many_kernel.
 #include <cooperative_groups.h>
 
 #include "trisolve.cuh"
@@ -73,25 +74,49 @@ __device__ __forceinline__ double ts_quotient(double v, double dd, double rinv) 
 // Otherwise (entries whose scaling could overflow or underflow, zeros and non-finite
 // values on the diagonal) every unknown is divided in turn.  Lanes already solved take
 // no part in a step, so a non-finite unknown leaves them alone.
-__device__ __forceinline__ double ts_solve32(double v, const double (&d)[32], double dd,
-                                             double rinv, bool unit, bool scaled) {
+// V vectors side by side; d in registers or, D[t][l], in shared memory; m: the block's
+// unknowns, uniform (32 where d holds zeros past them).
+__device__ __forceinline__ double ts_coef(const double (&d)[32], int t, int) { return d[t]; }
+__device__ __forceinline__ double ts_coef(const double (&d)[32][33], int t, int lane) {
+  return d[t][lane];
+}
+
+template <int V, typename Coef>
+__device__ __forceinline__ void ts_solve32(double (&v)[V], const Coef& d, int m, double dd,
+                                           double rinv, bool unit, bool scaled) {
   const int lane = threadIdx.x & 31;
   if (scaled) {
 #pragma unroll
     for (int t = 0; t < 31; ++t) {
-      const double vt = __shfl_sync(0xffffffffu, v, t);
-      if (lane > t) v = fma(-d[t], vt, v);
+      if (t + 1 >= m) break;
+      double vt[V];
+#pragma unroll
+      for (int q = 0; q < V; ++q) vt[q] = __shfl_sync(0xffffffffu, v[q], t);
+#pragma unroll
+      for (int q = 0; q < V; ++q)
+        if (lane > t) v[q] = fma(-ts_coef(d, t, lane), vt[q], v[q]);
     }
-    return unit ? v : ts_quotient(v, dd, rinv);
+#pragma unroll
+    for (int q = 0; q < V; ++q)
+      if (!unit) v[q] = ts_quotient(v[q], dd, rinv);
+    return;
   }
 #pragma unroll
-  for (int t = 0; t < 32; ++t) {
-    double xt = (lane == t) ? v / dd : 0.0;
-    xt = __shfl_sync(0xffffffffu, xt, t);
-    if (lane == t) v = xt;
-    if (lane > t) v = fma(-d[t], xt, v);
-  }
-  return v;
+  for (int t = 0; t < 32; ++t)
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      double xt = (lane == t) ? v[q] / dd : 0.0;
+      xt = __shfl_sync(0xffffffffu, xt, t);
+      if (lane == t) v[q] = xt;
+      if (lane > t) v[q] = fma(-ts_coef(d, t, lane), xt, v[q]);
+    }
+}
+
+__device__ __forceinline__ double ts_solve32(double v, const double (&d)[32], double dd,
+                                             double rinv, bool unit, bool scaled) {
+  double w[1] = {v};
+  ts_solve32(w, d, 32, dd, rinv, unit, scaled);
+  return w[0];
 }
 
 __global__ void __launch_bounds__(kTsThreads)
@@ -191,6 +216,157 @@ trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t s
     const double v = ts_solve32(xc[32 + lane], d, dd, rinv, unit, scaled);
     if (u0 + 32 + lane < n) xv[T.row(u0 + 32 + lane)] = v;
   }
+}
+
+// Many vectors: a CTA solves V of them from the first block to the last, in shared
+// memory.  The four CTAs of an SM are at different places of their chains, so the
+// substitutions of one hide behind the updates of others, and there is no launch
+// between blocks.  Bound by the FP64 pipe.  A row of an update belongs to four lanes,
+// with a transpose (rows along the lanes) to one thread, which saves the shuffles'
+// additions.  The operations on every element, and their order, are
+// trisolve_step_kernel's.
+// Measured, n = 1000 with a transpose, us here (V = 1) and with a launch per block: 300
+// vectors 524 and 766, 500 766 and 1155, 1000 1312 and 2102; without one 589 and 765,
+// 872 and 1155, 1475 and 2104.  2000 vectors with V = 2: 2446 (V = 1: 2527).
+constexpr int kTmCtas = 4;
+
+template <int V>
+__global__ void __launch_bounds__(kTsThreads, kTmCtas)
+trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt, int64_t stride_t,
+                     int fwd, int trans, int unit, double* __restrict__ x, int64_t stride_x) {
+  extern __shared__ double ts_x[];                 // V vectors in solve order, zeros past n
+  __shared__ double D[2][32][33];                  // the diagonal block's halves, by column
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nblk = (n + kTsNB - 1) / kTsNB, np = nblk * kTsNB;
+  const TsView T{t + (int64_t)blockIdx.y * stride_t, ldt, n, fwd != 0, trans != 0};
+  double* xv = x + (int64_t)blockIdx.y * stride_x + (int64_t)blockIdx.x * V * n;
+  const int nv = min(V, nrhs - (int)blockIdx.x * V);
+  const int wi = tid >> 2, wq = tid & 3;           // row, part: columns 4 pp + wq
+#pragma unroll
+  for (int q = 0; q < V; ++q)
+    for (int u = tid; u < np; u += kTsThreads)
+      ts_x[q * np + u] = (q < nv && u < n) ? xv[(int64_t)q * n + T.row(u)] : 0.0;
+  for (int b = 0; b < nblk; ++b) {
+    const int u0 = b * kTsNB;
+    double dd = 1.0, rinv = 1.0, cs[4];
+    bool scaled = true;
+    if (warp < 2) {
+      const int ul = u0 + 32 * warp + lane, m = min(32, n - u0 - 32 * warp);
+      bool ok = true;
+#pragma unroll 8
+      for (int k = 0; k < m; ++k) {
+        const double v = (ul < n && k < lane) ? T.op(ul, u0 + 32 * warp + k) : 0.0;
+        D[warp][k][lane] = v;
+        ok = ok && ts_moderate(v, true);
+      }
+      if (!unit) {
+        if (ul < n) dd = T.op(ul, ul);
+        scaled = __all_sync(0xffffffffu, ok && ts_moderate(dd, false));
+        if (scaled) {
+          rinv = 1.0 / dd;
+#pragma unroll 8
+          for (int k = 0; k < m; ++k) D[warp][k][lane] *= __shfl_sync(0xffffffffu, rinv, k);
+        }
+      }
+    }
+#pragma unroll
+    for (int pp = 0; pp < 4; ++pp) {
+      const int ur = u0 + 32 + (tid >> 3);
+      cs[pp] = (ur < n) ? T.op(ur, u0 + 8 * pp + (tid & 7)) : 0.0;
+    }
+    double* xc = ts_x + u0;
+    auto solve = [&](int half) {
+      double v[V];
+#pragma unroll
+      for (int q = 0; q < V; ++q) v[q] = xc[q * np + 32 * half + lane];
+      ts_solve32(v, D[half], min(32, n - u0 - 32 * half), dd, rinv, unit, scaled);
+#pragma unroll
+      for (int q = 0; q < V; ++q) xc[q * np + 32 * half + lane] = v[q];
+    };
+    __syncthreads();
+    if (warp == 0) solve(0);
+    __syncthreads();
+    if (u0 + 32 < n) {                             // uniform
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        double s = 0.0;
+#pragma unroll
+        for (int pp = 0; pp < 4; ++pp) s = fma(cs[pp], xc[q * np + 8 * pp + (tid & 7)], s);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        if ((tid & 7) == 0) xc[q * np + 32 + (tid >> 3)] -= s;
+      }
+      __syncthreads();
+      if (warp == 1) solve(1);
+      __syncthreads();
+    }
+    if (trans) {
+      for (int u = u0 + kTsNB + tid; u < n; u += kTsThreads) {
+        double acc[V][4][2];
+#pragma unroll
+        for (int q = 0; q < V; ++q)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) acc[q][r][0] = acc[q][r][1] = 0.0;
+#pragma unroll 1
+        for (int c = 0; c < kTsNB; c += 16) {
+          double cu[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) cu[e] = T.op(u, u0 + c + e);
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+              double& a = acc[q][e & 3][(e >> 2) & 1];
+              a = fma(cu[e], xc[q * np + c + e], a);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < V; ++q)
+          ts_x[q * np + u] -= ((acc[q][0][0] + acc[q][0][1]) + (acc[q][1][0] + acc[q][1][1])) +
+                              ((acc[q][2][0] + acc[q][2][1]) + (acc[q][3][0] + acc[q][3][1]));
+      }
+      continue;
+    }
+    for (int w = b + 1; w < nblk; ++w) {
+      double cu[16];
+#pragma unroll
+      for (int pp = 0; pp < 16; ++pp)
+        cu[pp] = (w * kTsNB + wi < n) ? T.op(w * kTsNB + wi, u0 + 4 * pp + wq) : 0.0;
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        double acc[2] = {0.0, 0.0};
+#pragma unroll
+        for (int pp = 0; pp < 16; ++pp)
+          acc[pp & 1] = fma(cu[pp], xc[q * np + 4 * pp + wq], acc[pp & 1]);
+        double s = acc[0] + acc[1];
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if (wq == 0) ts_x[q * np + w * kTsNB + wi] -= s;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < V; ++q)
+    for (int u = tid; u < n; u += kTsThreads)
+      if (q < nv) xv[(int64_t)q * n + T.row(u)] = ts_x[q * np + u];
+}
+
+// Vectors per CTA of the many-vector solve, 0 where a launch per block is taken: fewer
+// vectors than one and a half per SM (n = 1000, 150 vectors: 399 to 452 us against 480;
+// n = 4000 4285 to 4718 against 4390), or a matrix whose triangle the L2 cache may not
+// hold, since every CTA reads all of it.
+// Two per CTA above eight per SM, and where one each is more than the SMs take at once
+// but two each are not, for small n, whose second round is the longer part (us with one
+// and two, 1000 vectors: n = 200 177 and 142, 700 774 and 721, 1000 1312 and 1442; 700
+// vectors: n = 1000 1280 and 1060, 2000 3360 and 3870).
+constexpr int kTmMaxN = 4096;
+
+static int ts_many(int64_t vectors, int n) {
+  if (n > kTmMaxN || 2 * vectors < 3 * sm_count()) return 0;
+  const int64_t per_sm = (vectors + sm_count() - 1) / sm_count();
+  return per_sm > 8 || (per_sm > kTmCtas && n <= (per_sm <= 6 ? 1024 : 768)) ? 2 : 1;
 }
 
 // The whole solve in one launch for n up to 64 kTcMaxBlocks: a cluster of C CTAs
@@ -361,6 +537,15 @@ int trisolve_blocked(int64_t batch, int n, int nrhs, const double* t, int64_t ld
     LXGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, trisolve_cluster_kernel, n, t, ldt, stride_t, fwd, trans,
                                      unit, x, stride_x),
                   "trisolve: launch");
+    return check_launch("trisolve");
+  }
+  if (const int v = ts_many(batch * nrhs, n)) {
+    auto fn = v == 2 ? trisolve_many_kernel<2> : trisolve_many_kernel<1>;
+    const size_t smem = (size_t)v * nblk * kTsNB * sizeof(double);
+    LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(fn), (int)smem),
+                  "trisolve: set smem");
+    fn<<<dim3((unsigned)((nrhs + v - 1) / v), (unsigned)batch), kTsThreads, smem, st>>>(
+        n, nrhs, t, ldt, stride_t, fwd, trans, unit, x, stride_x);
     return check_launch("trisolve");
   }
   for (int b = 0; b < nblk; ++b) {

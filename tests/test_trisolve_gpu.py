@@ -202,3 +202,36 @@ def test_getrs_interchanges_time_of_large_orders(dev):
     """Orders above 11000 take the same path: per unknown no more than a quarter above
     n = 11000 (one thread exchanging in memory took 1.5 ms of a solve of 3)."""
     assert _solve_ms(dev, 13000, "random") <= 1.25 * 13000 / 11000 * _solve_ms(dev, 11000, "random")
+
+
+@pytest.mark.parametrize("lower,trans,unit", [(a, b, c) for a in (True, False)
+                                              for b in (True, False) for c in (True, False)])
+@pytest.mark.parametrize("n", [1, 32, 33, 64, 65, 96, 97, 129, 1000, 4096, 4097])
+def test_trsm_many_vectors_same_bits_as_some(dev, n, lower, trans, unit):
+    """The vectors that one launch takes together (from one and a half per SM on, and two
+    per CTA above four or eight) against the same vectors 40 at a time."""
+    g = torch.Generator(device=dev).manual_seed(n)
+    t = torch.randn(n, n, dtype=torch.float64, device=dev, generator=g) / n
+    t.diagonal().add_(1.0)
+    if n == 129:
+        t[70, 70] = 2.0 ** -600                  # one block is divided in turn
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    ks = (3 * sms // 2, 3 * sms // 2 + 1, 4 * sms + 3, 8 * sms + 1) if n < 4000 else (3 * sms // 2,)
+    b = torch.randn(max(ks), n, dtype=torch.float64, device=dev, generator=g)
+    args = dict(lower=lower, trans=trans, unit=unit)
+    some = torch.cat([_dense.trsv(t, b[i:i + 40], **args) for i in range(0, max(ks), 40)])
+    for k in ks:
+        assert torch.equal(_dense.trsv(t, b[:k], **args), some[:k])
+
+
+def test_getrs_many_vectors_of_several_systems(dev):
+    n, bt, k = 180, 5, 61                        # 305 vectors in all, an odd count per system
+    g = torch.Generator(device=dev).manual_seed(1)
+    a = torch.randn(bt, n, n, dtype=torch.float64, device=dev, generator=g)
+    b = torch.randn(bt, k, n, dtype=torch.float64, device=dev, generator=g)
+    lu, piv, _ = _dense.lu_factor_batched(a)
+    for trans in (0, 1):
+        x = _dense.lu_solve_batched(lu, piv, b, trans)
+        for s in range(bt):
+            assert torch.equal(x[s], _dense.lu_solve_batched(lu[s:s + 1], piv[s:s + 1], b[s:s + 1],
+                                                             trans)[0])
