@@ -30,6 +30,7 @@ namespace lxgb {
 constexpr int kSmallMax = 168;   // 168*169*8 B = 227 KB of shared memory
 constexpr int kSmallThreads = 256;
 constexpr int kSmallMaxThreads = 512;
+constexpr size_t kSmSharedBytes = 228 * 1024;   // of an SM, with 1 KB and the static part per CTA
 constexpr int kSmallBlocks = (kSmallMax + 31) / 32;
 constexpr int kNB = 32;          // panel width of the blocked path
 constexpr int kPanelThreads = 1024;
@@ -1130,8 +1131,16 @@ extern "C" int lxgb_getrf_batched_f64(int64_t batch, int32_t n, double* a, int64
     const size_t smem = (size_t)n * (n | 1) * sizeof(double);
     // More warps where the update is the longer part: us per matrix with 256 and
     // 512 threads 14.6 and 16.6 at n = 16, 47 and 47 at 48, 191 and 176 at 100, 317
-    // and 289 at 128; 512 matrices of order 64 156 and 187.
-    const int threads = n <= 64 ? kSmallThreads : kSmallMaxThreads;
+    // and 289 at 128; 512 matrices of order 64 156 and 187.  Fewer where the shared
+    // memory of an SM holds several matrices and there is more than one for each SM: a
+    // CTA of 512 threads takes more than half of an SM's registers.  us for 4096 matrices with
+    // 128, 256 and 512 threads: n = 65 1067, 1209 and 2278, 80 1850, 1856 and 3071, 96
+    // 3124, 2812 and 4240, 119 7206, 5391 and 6746; for 304: n = 65 141, 124 and 185.
+    const bool several = batch > sm_count() && 2 * (smem + 2048) <= kSmSharedBytes;
+    const int threads = n <= 64 ? kSmallThreads
+                                : (!several ? kSmallMaxThreads
+                                            : (n <= 80 && batch > 2 * sm_count() ? kSmallThreads / 2
+                                                                                 : kSmallThreads));
     // registers for the rows of a column per lane of warp 0
     auto fn = n <= 64 ? getrf_small_kernel<2>
                       : (n <= 128 ? getrf_small_kernel<4> : getrf_small_kernel<kSmallBlocks>);

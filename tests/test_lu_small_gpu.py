@@ -82,3 +82,37 @@ def test_lu_small_tiny_pivots_divide(dev, n):
     assert int(info) == 0 and list(piv.cpu().numpy()) == list(range(n))
     ref = np.tril(a * s, -1) / s
     assert np.array_equal(np.tril(lu.cpu().numpy(), -1), ref)
+
+
+@pytest.mark.parametrize("n", [64, 65, 80, 81, 96, 119, 120, 168])
+def test_lu_small_large_batches_same_bits(dev, n):
+    """More matrices than SMs, and than two per SM: fewer threads per matrix where an SM
+    holds several, the bits of the matrix factored alone."""
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    g = torch.Generator(device=dev).manual_seed(n)
+    a = torch.randn(2 * sms + 1, n, n, dtype=torch.float64, device=dev, generator=g)
+    one = [_dense.lu_factor_batched(a[s:s + 1]) for s in range(0, 2 * sms + 1, 37)]
+    for batch in (sms + 1, 2 * sms + 1):
+        lu, piv, info = _dense.lu_factor_batched(a[:batch])
+        assert torch.all(info == 0)
+        for i, s in enumerate(range(0, batch, 37)):
+            assert torch.equal(lu[s], one[i][0][0]) and torch.equal(piv[s], one[i][1][0])
+
+
+def test_lu_small_time_of_large_batches(dev):
+    """A matrix of order 65 in a batch of 4096 takes little more than one of order 64
+    (65^3 / 64^3 = 1.05, and one more block of rows): not half as long again."""
+    def us(n):
+        g = torch.Generator(device=dev).manual_seed(n)
+        a = torch.randn(4096, n, n, dtype=torch.float64, device=dev, generator=g)
+        best = np.inf
+        for _ in range(6):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            _dense.lu_factor_batched(a)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+
+    assert us(65) <= 1.5 * us(64)
