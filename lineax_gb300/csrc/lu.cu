@@ -977,17 +977,18 @@ static int getrs_perm(int64_t batch, int n, int nrhs, const int32_t* piv, int64_
 // Measured (one right-hand side): 16.6 us at n = 48, 37 at 128, 53 at 168, against
 // 29, 72 and 98 with one warp per right-hand side.
 // ---------------------------------------------------------------------------
-constexpr int kSmallRhs = 4;           // right-hand sides at a time
+constexpr int kSmallRhs = 4;           // groups of right-hand sides at a time
 constexpr int kSmallSolveThreads = 32 * kSmallBlocks * kSmallRhs;
 constexpr int kSmallHalf = 16;
 
 // One sweep over op(T), ascending (FWD) or descending, on the x of this thread
-// (row 32 m + lane, rinv the inverse of its diagonal); op(T)[i][t] is T[t][i]
-// with TR.  xs: the unknowns of two half blocks in turn.
-template <bool FWD, bool UNIT, bool TR>
+// (row 32 m + lane of NV right-hand sides, rinv the inverse of its diagonal);
+// op(T)[i][t] is T[t][i] with TR.  xs: the unknowns of two half blocks in turn, by
+// right-hand side.
+template <bool FWD, bool UNIT, bool TR, int NV>
 __device__ __forceinline__ void small_sweep(int n, int ld, const double* T, double rinv,
                                             double* xs, int nblk, int m, int lane, bool active,
-                                            double& x) {
+                                            double (&x)[NV]) {
   constexpr int kH = kSmallHalf;
   const int i = 32 * m + lane;
   for (int q = 0; q < 2 * nblk; ++q) {
@@ -1005,12 +1006,21 @@ __device__ __forceinline__ void small_sweep(int n, int ld, const double* T, doub
       for (int u = 0; u < kH; ++u) {
         const int t = FWD ? t0 + u : t0 + kH - 1 - u;
         if (t < n) {
-          if (!UNIT && i == t) x *= rinv;
-          const double xt = __shfl_sync(0xffffffffu, x, t & 31);
-          if (i < n && (FWD ? i > t : i < t)) x = fma(-tv[u], xt, x);
+          double xt[NV];
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            if (!UNIT && i == t) x[v] *= rinv;
+            xt[v] = __shfl_sync(0xffffffffu, x[v], t & 31);
+          }
+#pragma unroll
+          for (int v = 0; v < NV; ++v)
+            if (i < n && (FWD ? i > t : i < t)) x[v] = fma(-tv[u], xt[v], x[v]);
         }
       }
-      if ((i >> 4) == hb) xs[kH * (q & 1) + (i & (kH - 1))] = x;
+      if ((i >> 4) == hb) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) xs[2 * kH * v + kH * (q & 1) + (i & (kH - 1))] = x[v];
+      }
     }
     __syncthreads();
     if (active && i < n && (FWD ? m > (hb >> 1) : m < (hb >> 1))) {
@@ -1023,12 +1033,17 @@ __device__ __forceinline__ void small_sweep(int n, int ld, const double* T, doub
 #pragma unroll
       for (int u = 0; u < kH; ++u) {
         const int t = FWD ? t0 + u : t0 + kH - 1 - u;
-        if (t < n) x = fma(-tv[u], xs[kH * (q & 1) + (t & (kH - 1))], x);
+        if (t < n) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v)
+            x[v] = fma(-tv[u], xs[2 * kH * v + kH * (q & 1) + (t & (kH - 1))], x[v]);
+        }
       }
     }
   }
 }
 
+template <int NV>
 __global__ void __launch_bounds__(kSmallSolveThreads)
 getrs_small_kernel(int n, int nrhs, int per, const double* __restrict__ lu, int64_t stride_a,
                    const int32_t* __restrict__ piv, int64_t stride_piv, double* __restrict__ b,
@@ -1039,7 +1054,7 @@ getrs_small_kernel(int n, int nrhs, int per, const double* __restrict__ lu, int6
   double* T = smem_x;                                   // n × ld
   double* rinv = T + (int64_t)n * ld;                   // 1 / u_tt
   double* xs = rinv + n;                                // finished unknowns, by right-hand side
-  int* perm = reinterpret_cast<int*>(xs + per * 2 * kSmallHalf);  // x_perm[i] = b[perm[i]]
+  int* perm = reinterpret_cast<int*>(xs + per * NV * 2 * kSmallHalf);  // x_perm[i] = b[perm[i]]
   int* sp = perm + n;                                   // the interchanges
   const int sys = blockIdx.x;
   const double* A = lu + (int64_t)sys * stride_a;
@@ -1074,22 +1089,27 @@ getrs_small_kernel(int n, int nrhs, int per, const double* __restrict__ lu, int6
   __syncthreads();
   const int rg = warp / nblk, m = warp - rg * nblk, i = 32 * m + lane;
   const double ri = i < n ? rinv[i] : 0.0;
-  for (int r0 = 0; r0 < nrhs; r0 += per) {
-    const bool active = rg < per && r0 + rg < nrhs;
-    double* g = b + (int64_t)sys * stride_b + (int64_t)(r0 + rg) * n;
-    double* mine = xs + (active ? rg : 0) * 2 * kSmallHalf;
-    double x = 0.0;
-    if (active && i < n) x = g[trans ? i : perm[i]];
+  for (int r0 = 0; r0 < nrhs; r0 += per * NV) {
+    const int first = r0 + rg * NV;                      // this warp's right-hand sides
+    const bool active = rg < per && first < nrhs;
+    double* g = b + (int64_t)sys * stride_b + (int64_t)first * n;
+    double* mine = xs + (active ? rg : 0) * NV * 2 * kSmallHalf;
+    double x[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+      x[v] = (active && i < n && first + v < nrhs) ? g[v * n + (trans ? i : perm[i])] : 0.0;
     // every element is read before the first is written
     __syncthreads();
     if (!trans) {
-      small_sweep<true, true, false>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // L y = P b
-      small_sweep<false, false, false>(n, ld, T, ri, mine, nblk, m, lane, active, x); // U x = y
+      small_sweep<true, true, false, NV>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // L y = P b
+      small_sweep<false, false, false, NV>(n, ld, T, ri, mine, nblk, m, lane, active, x); // U x = y
     } else {
-      small_sweep<true, false, true>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // Uᵀ z = b
-      small_sweep<false, true, true>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // Lᵀ w = z
+      small_sweep<true, false, true, NV>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // Uᵀ z = b
+      small_sweep<false, true, true, NV>(n, ld, T, ri, mine, nblk, m, lane, active, x);   // Lᵀ w = z
     }
-    if (active && i < n) g[trans ? perm[i] : i] = x;    // x = Pᵀ w: x[perm[i]] = w[i]
+#pragma unroll
+    for (int v = 0; v < NV; ++v)                         // x = Pᵀ w: x[perm[i]] = w[i]
+      if (active && i < n && first + v < nrhs) g[v * n + (trans ? perm[i] : i)] = x[v];
   }
 }
 
@@ -1171,15 +1191,23 @@ extern "C" int lxgb_getrs_batched_f64(int64_t batch, int32_t n, int32_t nrhs, co
                "getrs: stride too small");
   LXGB_REQUIRE(batch * (int64_t)nrhs < (1LL << 31), "getrs: too many vectors in one call");
   if (n <= kSmallMax && batch < (1LL << 31)) {
-    const int per = nrhs < kSmallRhs ? nrhs : kSmallRhs;
+    // Two right-hand sides per warp above four: their chains run side by side (us for 16
+    // with one and two: n = 128 149 and 141, 168 246 and 239).  Small orders have little
+    // to load, so threads that no right-hand side needs only cost CTAs per SM (us for
+    // 4096 systems of one, with 8, 4 and 2 warps: n = 16 57, 39 and 33, 64 161, 123 and
+    // 147, 96 267, 310 and 345).
+    const int nv = nrhs > kSmallRhs ? 2 : 1;
+    const int groups = (nrhs + nv - 1) / nv;
+    const int per = groups < kSmallRhs ? groups : kSmallRhs;
     const size_t smem = (size_t)n * (n | 1) * sizeof(double) + (size_t)n * sizeof(double) +
-                        (size_t)per * 2 * kSmallHalf * sizeof(double) +
+                        (size_t)per * nv * 2 * kSmallHalf * sizeof(double) +
                         (size_t)n * 2 * sizeof(int32_t);
-    const int warps = (n + 31) / 32 * per;
-    const int threads = 32 * (warps < 8 ? 8 : warps);
-    LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(getrs_small_kernel), (int)smem),
+    const int warps = (n + 31) / 32 * per, least = n <= 32 ? 2 : (n <= 64 ? 4 : 8);
+    const int threads = 32 * (warps < least ? least : warps);
+    auto fn = nv == 2 ? getrs_small_kernel<2> : getrs_small_kernel<1>;
+    LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(fn), (int)smem),
                   "getrs small: set smem");
-    getrs_small_kernel<<<(unsigned)batch, threads, smem, as_stream(stream)>>>(
+    fn<<<(unsigned)batch, threads, smem, as_stream(stream)>>>(
         n, nrhs, per, lu, stride_a, piv, stride_piv, b, stride_b, trans);
     return check_launch("getrs small");
   }

@@ -116,3 +116,17 @@ def test_lu_small_time_of_large_batches(dev):
         return best
 
     assert us(65) <= 1.5 * us(64)
+
+
+@pytest.mark.parametrize("n", [1, 16, 31, 32, 33, 64, 65, 128, 168])
+@pytest.mark.parametrize("nrhs", [5, 8, 9, 17])
+def test_lu_small_solve_same_bits_one_by_one(dev, n, nrhs):
+    """More than four right-hand sides go two to a warp: the bits of each alone."""
+    g = torch.Generator(device=dev).manual_seed(n)
+    a = torch.randn(2, n, n, dtype=torch.float64, device=dev, generator=g)
+    b = torch.randn(2, nrhs, n, dtype=torch.float64, device=dev, generator=g)
+    lu, piv, _ = _dense.lu_factor_batched(a)
+    for trans in (0, 1):
+        x = _dense.lu_solve_batched(lu, piv, b, trans)
+        for c in range(nrhs):
+            assert torch.equal(x[:, c], _dense.lu_solve_batched(lu, piv, b[:, c].contiguous(), trans))
