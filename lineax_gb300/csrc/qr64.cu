@@ -454,6 +454,7 @@ qr32_merge_t_kernel(int64_t mm, int nn, const double* __restrict__ h, double* __
 constexpr int kOmThreads = 256;
 constexpr int kOmSlots = 6;          // rows per lane held in registers
 constexpr int kOmMaxRows = 2048;     // rows per CTA: 9 doubles of shared memory each
+constexpr int kOmManyRows = 1024;    // of many vectors: two CTAs per SM
 
 __global__ void __launch_bounds__(kOmThreads)
 ormqr_cluster_kernel(int64_t mm, int nn, int R, const double* __restrict__ h,
@@ -696,6 +697,14 @@ int ormqr64_cluster(int64_t m, int n, const double* h, const double* t, int nrhs
                     int trans, cudaStream_t st) {
   int64_t ctas = (m + 127) / 128;
   if (ctas > kQClu) ctas = kQClu;
+  // One vector wants many CTAs.  With more of them than eight per SM what counts is the
+  // work between a panel's two cluster barriers, so the rows go to fewer CTAs, up to
+  // kOmManyRows each.  us for 500 vectors with 16, 8, 4, 2 and 1: 2000 x 2000 20250,
+  // 14937, 10958, 8835, 8524 (two launches per panel: 11965), 8192 x 64 2028, 1499, 1848
+  // (2334).
+  while (ctas > 1 && nrhs * ctas > 8LL * sm_count() &&
+         (m + ctas / 2 - 1) / (ctas / 2) <= kOmManyRows)
+    ctas /= 2;
   const int64_t R = (m + ctas - 1) / ctas;
   if (R > kOmMaxRows) return -1;
   const size_t smem = (size_t)R * (1 + kOmThreads / 32) * sizeof(double);

@@ -74,3 +74,22 @@ def test_qr_columns_outside_the_reciprocal_root_range(dev, m, n, scale):
     v = torch.tril(h.T, -1)
     v[torch.arange(n), torch.arange(n)] = 1.0
     assert bool(((tau * (v * v).sum(0) - 2).abs() <= 100 * U).all())
+
+
+@pytest.mark.parametrize("m,n", [(300, 40), (1025, 33), (2000, 100), (4100, 18), (8192, 35)])
+@pytest.mark.parametrize("k", [100, 300, 650])
+def test_q_of_many_vectors(dev, m, n, k):
+    """Many vectors at once, with fewer CTAs for each: within the bound of
+    test_q_transposed_a_is_r of the vectors taken three at a time, and back."""
+    g = torch.Generator(device=dev).manual_seed(k)
+    h, tau, t = _dense.geqrf(torch.randn(m, n, dtype=torch.float64, device=dev, generator=g))
+    c = torch.randn(k, m, dtype=torch.float64, device=dev, generator=g)
+    some = list(range(0, k, 37))
+    for trans in (True, False):
+        y = _dense.ormqr(h, tau, t, c, trans=trans)
+        for i in range(0, len(some), 3):
+            s = some[i:i + 3]
+            few = _dense.ormqr(h, tau, t, c[s].contiguous(), trans=trans)
+            assert bool(((y[s] - few).norm(dim=1) <= 40 * n * U * c[s].norm(dim=1)).all())
+        back = _dense.ormqr(h, tau, t, y, trans=not trans)
+        assert bool(((back - c).norm(dim=1) <= 40 * n * U * c.norm(dim=1)).all())
