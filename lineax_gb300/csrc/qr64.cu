@@ -225,8 +225,10 @@ qr16_panel_kernel(int64_t mm, int j0, int nb, int R, double* __restrict__ h,
         for (int c = q; c < 4; ++c) {
           if (c > q || t > tt) {
             const double w = sm.tws[par][4 * c + t];
+            // (rows up to kk are in the first slot; their v is 0, w may be infinite or NaN)
 #pragma unroll
-            for (int rr = 0; rr < RR; ++rr) r[rr][c] = fma(-w, v[rr], r[rr][c]);
+            for (int rr = 0; rr < RR; ++rr)
+              if (rr > 0 || row0 + g > kk) r[rr][c] = fma(-w, v[rr], r[rr][c]);
             if (rowk) r[0][c] -= sm.tw[par][4 * c + t];
           }
         }

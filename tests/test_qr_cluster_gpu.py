@@ -93,3 +93,17 @@ def test_q_of_many_vectors(dev, m, n, k):
             assert bool(((y[s] - few).norm(dim=1) <= 40 * n * U * c[s].norm(dim=1)).all())
         back = _dense.ormqr(h, tau, t, y, trans=not trans)
         assert bool(((back - c).norm(dim=1) <= 40 * n * U * c.norm(dim=1)).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(5, 3, 1), (40, 16, 5), (300, 16, 0), (300, 16, 15), (700, 12, 7)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_qr_non_finite_column_leaves_finished_rows_alone(dev, m, n, k, bad):
+    """Column k with a non-finite entry in the last row: the columns before it, and the
+    rows of R that the reflectors before k made, keep the bits they have without it."""
+    rng = np.random.default_rng(m + n)
+    a = torch.tensor(rng.standard_normal((m, n)), device=dev)
+    h0, tau0, _ = _dense.geqrf(a)
+    a[m - 1, k] = bad
+    h, tau, _ = _dense.geqrf(a)
+    assert torch.equal(h[:k], h0[:k]) and torch.equal(tau[:k], tau0[:k])
+    assert torch.equal(h[k + 1:, :k], h0[k + 1:, :k])
