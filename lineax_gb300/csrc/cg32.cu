@@ -86,9 +86,10 @@ static int c32_parts(int64_t nx, int64_t ny) {
 // and all pointers on 16 bytes; one float at a time otherwise), then one thread
 // per column walks the rows, so a thread's sum has the same terms in the same
 // order whatever VEC is.
-// Bound by HBM.  Measured at 2048 x 2048, 64 right-hand sides: 762 us, 7.0 TB/s
-// (the passes it replaces, a stencil with A p stored, p and half of the update:
-// 847, 584 and about 620 us).
+// Bound by HBM.  Measured at 2048 x 2048, 64 right-hand sides: 761 us, 7.0 TB/s of these
+// 20 bytes.  That is 3 % above a plain copy's rate (6.79): three bytes are read for two
+// written, and L2 may still hold a part of p and r.  (The passes it replaces, a stencil
+// with A p stored, p and half of the update: 847, 584 and about 620 us.)
 template <bool STEP, int VEC>
 __global__ void __launch_bounds__(kC32Threads)
 c32_step_kernel(int64_t nx, int64_t ny, C32State s, const float* __restrict__ r,

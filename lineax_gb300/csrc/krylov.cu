@@ -639,10 +639,10 @@ gm_step_cluster_kernel(int n, GmWork w, int cur, int kk, double* __restrict__ wv
 // added while the clusters of all right-hand sides leave an SM to every CTA.
 // Measured, us per step of a cycle of 20, here and on the general path:
 //   n      rhs  here  general      n      rhs  here  general
-//   200      1  11.9    15.1       8192     1  16.8    25.4
-//   2000     1  12.9    25.8       8192    16  34.9    35.8
-//   2000    16  20.3    29.8       8192    64  76.9    83.1
-//   2000   200  52.1    71.5       16384   16  50.4    51.1
+//   200      1  12.0    15.1       8192     1  17.0    25.4
+//   2000     1  13.3    25.8       8192    16  35.3    35.8
+//   2000    16  20.7    29.8       8192    64  77.8    83.1
+//   2000   200  52.7    71.5       16384   16  50.9    51.1
 // (both with a copy of w, 3 to 10 us, in front of each step; the general path's
 // dots one after the other in one CTA took 47.5 at 2000 and 48.3 at 8192 x 16).
 static int gm_cluster_size(int64_t n, int k) {

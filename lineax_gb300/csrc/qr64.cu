@@ -619,10 +619,13 @@ static size_t apply_smem(int R) {
 }
 
 // Rows per CTA aimed at: 64 for the next panel's strips (2 columns each; their
-// time is on the critical path, so as many CTAs as a cluster may have), 320 for
-// the others (8 columns each; whole solve of a 3001 x 401 problem with 500,
-// 376, 300, 251 and 188 rows: 2.53, 2.65, 2.55, 2.65 and 2.91 ms — clusters of
-// 16 find fewer places beside the panel's).
+// time is on the critical path, so as many CTAs as a cluster may have; 32 and 128
+// measure the same within 1 %), 320 for the others (8 columns each).  Small strips make
+// clusters of 16, which find fewer places beside the panel's; large ones hold few CTAs
+// per SM.  us for the factor with 188, 320, 500 and 700 rows: 1000 x 1000 4164, 3947,
+// 3817, 3811; 2000 x 500 2583, 2539, 2365, 2547; 3001 x 401 2568, 2398, 2266, 2485;
+// 5000 x 1000 15860, 16530, 14520, 17760; 8192 x 2000 87440, 87450, 91480, 106700.
+// 320 is never far off; 500 is better below 8192 rows.
 constexpr int kQNextRows = 64, kQWideRows = 320;
 
 int geqrf64_cluster(int64_t m, int n, double* h, double* tau, double* t, cudaStream_t st) {

@@ -5,9 +5,10 @@
 // tiles of an n×n result, one CTA per tile (256 threads, 4×4 outputs each,
 // A staged through shared memory in 16-deep slices).  Either as a Gram matrix
 // (C = S, optionally mirrored into the lower triangle: the normal equations
-// of lineax's Normal solver, lineax/_solver/normal.py:112-118) or as the
-// Cholesky trailing update C -= S, where every element continues its FMA
-// chain from its stored value in k order.
+// of lineax's Normal solver, lineax/_solver/normal.py:112-118) or as an update
+// C -= S of the upper triangle, where every element continues its FMA chain
+// from its stored value in k order (the Cholesky below has its own, 32 rows at
+// a time).
 //
 // lxgb_potrf_f64 factors one n×n SPD matrix (A = UᵀU, upper) right-looking
 // by 32-row block rows: the diagonal block and its block row in one sweep
@@ -26,7 +27,9 @@ constexpr int kPoNB = 32;       // block rows of the multi-CTA Cholesky
 // Columns per CTA of the block-row kernel: 32 G.  G = 2 above kPoWide trailing
 // columns, where the trailing update beside it wants the SMs (n = 1531: 24
 // instead of 48 of them); G = 1 below, where the block row's own time counts
-// (27 us against 31).  At n = 1531 both alone take 2.68 ms in all.
+// (24 us against 30).  us for the factor with this line, with G = 1 and with G = 2
+// throughout: n = 1000 974, 971 and 1106, 1531 1971, 2089 and 2076, 3000 9334, 9600 and
+// 9439, 8192 153200, 154900 and 153300.
 constexpr int kPoWide = 1024;
 // Unused dynamic shared memory that a block-row CTA reserves, so that no CTA
 // of the trailing update running beside it (17 KB each) shares its SM.

@@ -15,11 +15,10 @@
 // per step), the 64x64 update (2 FP64 FMA per clock and SM: 1 us) and the
 // hand-over between launches.  Four lanes share a row in the updates: 16 FMAs
 // and two shuffle additions per lane, against 2 FMAs and five additions with
-// a warp per row.  Measured (one vector, us): n = 128 26, n = 1000 128, n =
-// 2003 268; one CTA per vector with a division per unknown took 68 and 452 at
+// a warp per row.  Measured (five vectors, us): n = 128 23, n = 1000 135, n =
+// 2003 282; one CTA per vector with a division per unknown took 68 and 452 at
 // n = 128 and 767, and a diagonal and an update launch per block 549 and 1104
-// at n = 1000 and 2003.  getrs at n = 2003: 511 us against 2500 to 6200 (the
-// more interchanges, the longer: one thread ran them in order).
+// at n = 1000 and 2003.
 // Few vectors of up to 2048 unknowns: trisolve_cluster_kernel below; many of up to
 // 4096: trisolve_many_kernel.
 #include <cooperative_groups.h>
@@ -379,9 +378,10 @@ static int ts_many(int64_t vectors, int n) {
 // buffers of x; program order keeps a buffer's last read before the arrival that
 // lets it be overwritten).  The operations on every element, and their order, are
 // trisolve_step_kernel's.
-// Measured (one vector, us): n = 401 55, 1000 120, 1531 177, 2003 235, against 64,
-// 132, 206 and 267 with a launch per block, whose hand-over it saves; the chain of
-// a block (two substitutions, the update, the push and the barrier) remains.
+// Measured (one vector, us): n = 401 60, 1000 126, 1531 185, 2003 246, against 69, 135,
+// 217 and 282 with a launch per block (five or more vectors), whose hand-over it saves;
+// the chain of a block (two substitutions, the update, the push and the barrier)
+// remains.
 constexpr int kTcMaxBlocks = 32;
 constexpr int kTcMax = 16;
 
