@@ -65,16 +65,26 @@ __device__ __forceinline__ double ts_quotient(double v, double dd, double rinv) 
 
 // One warp solves a 32-unknown block: lane l holds v = b_l and d[t] = op(l, t)
 // (0 for t >= l, or past the block's end), dd = op(l, l) (1 for unit
-// diagonals and past the end).  `scaled`: d[t] was multiplied by 1/op(t, t),
-// so a step is v_l -= d[t] v_t on unscaled v: a shuffle and an FMA, and the quotients
-// x_l = v_l / op(l, l) of all lanes come at the end.  Errors against 128 bits (n = 32
-// to 300, mean over 40 systems of three kinds): those of a division per step, within
-// 3 % either way; with the bare product by the reciprocal at the end up to 10 % above.
-// Otherwise (entries whose scaling could overflow or underflow, zeros and non-finite
-// values on the diagonal) every unknown is divided in turn.  Lanes already solved take
-// no part in a step, so a non-finite unknown leaves them alone.
+// diagonals and past the end), and for moderate entries rinv = 1 / dd.
+//  * kTsScaled: d[t] was multiplied by 1/op(t, t), so a step is v_l -= d[t] v_t on
+//    unscaled v: a shuffle and an FMA, and the quotients x_l = v_l / op(l, l) of all
+//    lanes come at the end.  Forward errors against 128 bits (n = 32 to 300, mean over
+//    40 systems of three kinds): those of a division per step, within 3 % either way;
+//    with the bare product by the reciprocal at the end up to 10 % above.
+//  * kTsQuotient (one block of 64): x_t is rounded before it is used, as with a division
+//    per step.  Up to n = 16 the scaled form's backward errors are 10 to 20 %
+//    larger, from n = 33 on the same.
+//  * kTsDivide (entries whose scaling could overflow or underflow, zeros and non-finite
+//    values on the diagonal): every unknown is divided in turn.
+// Lanes already solved take no part in a step, so a non-finite unknown leaves them alone.
+enum TsForm { kTsScaled, kTsQuotient, kTsDivide };
+
+__device__ __forceinline__ TsForm ts_form(int n, bool moderate) {
+  return !moderate ? kTsDivide : (n <= kTsNB ? kTsQuotient : kTsScaled);
+}
+
 // V vectors side by side; d in registers or, D[t][l], in shared memory; m: the block's
-// unknowns, uniform (32 where d holds zeros past them).
+// unknowns, uniform.
 __device__ __forceinline__ double ts_coef(const double (&d)[32], int t, int) { return d[t]; }
 __device__ __forceinline__ double ts_coef(const double (&d)[32][33], int t, int lane) {
   return d[t][lane];
@@ -82,12 +92,13 @@ __device__ __forceinline__ double ts_coef(const double (&d)[32][33], int t, int 
 
 template <int V, typename Coef>
 __device__ __forceinline__ void ts_solve32(double (&v)[V], const Coef& d, int m, double dd,
-                                           double rinv, bool unit, bool scaled) {
+                                           double rinv, bool unit, TsForm form) {
+  constexpr bool kRegs = sizeof(Coef) == 32 * sizeof(double);  // all steps: d holds zeros
   const int lane = threadIdx.x & 31;
-  if (scaled) {
+  if (form == kTsScaled) {
 #pragma unroll
     for (int t = 0; t < 31; ++t) {
-      if (t + 1 >= m) break;
+      if (!kRegs && t + 1 >= m) break;
       double vt[V];
 #pragma unroll
       for (int q = 0; q < V; ++q) vt[q] = __shfl_sync(0xffffffffu, v[q], t);
@@ -100,21 +111,25 @@ __device__ __forceinline__ void ts_solve32(double (&v)[V], const Coef& d, int m,
       if (!unit) v[q] = ts_quotient(v[q], dd, rinv);
     return;
   }
+  const bool quick = form == kTsQuotient;
 #pragma unroll
-  for (int t = 0; t < 32; ++t)
+  for (int t = 0; t < 32; ++t) {
+    if (t >= m) break;
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      double xt = (lane == t) ? v[q] / dd : 0.0;
+      double xt = 0.0;
+      if (lane == t) xt = quick ? ts_quotient(v[q], dd, rinv) : v[q] / dd;
       xt = __shfl_sync(0xffffffffu, xt, t);
       if (lane == t) v[q] = xt;
       if (lane > t) v[q] = fma(-ts_coef(d, t, lane), xt, v[q]);
     }
+  }
 }
 
-__device__ __forceinline__ double ts_solve32(double v, const double (&d)[32], double dd,
-                                             double rinv, bool unit, bool scaled) {
+__device__ __forceinline__ double ts_solve32(double v, const double (&d)[32], int m, double dd,
+                                             double rinv, bool unit, TsForm form) {
   double w[1] = {v};
-  ts_solve32(w, d, 32, dd, rinv, unit, scaled);
+  ts_solve32(w, d, m, dd, rinv, unit, form);
   return w[0];
 }
 
@@ -142,7 +157,7 @@ trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t s
   // warp 1 the second 32's; every thread 4 entries of the block below the
   // first (row tid >> 3, columns 8 pp + (tid & 7)).
   double d[32], dd = 1.0, rinv = 1.0, cs[4];
-  bool scaled = true;
+  TsForm form = kTsScaled;
   if (chain) {
     if (warp < 2) {
       const int ul = u0 + 32 * warp + lane;
@@ -156,9 +171,9 @@ trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t s
       if (!unit) {
         if (ul < n) dd = T.op(ul, ul);
         ok = ok && ts_moderate(dd, false);
-        scaled = __all_sync(0xffffffffu, ok);
-        if (scaled) {
-          rinv = 1.0 / dd;
+        form = ts_form(n, __all_sync(0xffffffffu, ok));
+        if (form != kTsDivide) rinv = 1.0 / dd;
+        if (form == kTsScaled) {
 #pragma unroll
           for (int k = 0; k < 32; ++k) d[k] *= __shfl_sync(0xffffffffu, rinv, k);
         }
@@ -195,7 +210,7 @@ trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t s
   if (!chain) return;
   __syncthreads();
   if (warp == 0) {
-    const double v = ts_solve32(xc[lane], d, dd, rinv, unit, scaled);
+    const double v = ts_solve32(xc[lane], d, min(32, n - u0), dd, rinv, unit, form);
     xc[lane] = v;
     if (u0 + lane < n) xv[T.row(u0 + lane)] = v;
   }
@@ -212,7 +227,7 @@ trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t s
   }
   __syncthreads();
   if (warp == 1) {
-    const double v = ts_solve32(xc[32 + lane], d, dd, rinv, unit, scaled);
+    const double v = ts_solve32(xc[32 + lane], d, min(32, n - u0 - 32), dd, rinv, unit, form);
     if (u0 + 32 + lane < n) xv[T.row(u0 + 32 + lane)] = v;
   }
 }
@@ -248,7 +263,7 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
   for (int b = 0; b < nblk; ++b) {
     const int u0 = b * kTsNB;
     double dd = 1.0, rinv = 1.0, cs[4];
-    bool scaled = true;
+    TsForm form = kTsScaled;
     if (warp < 2) {
       const int ul = u0 + 32 * warp + lane, m = min(32, n - u0 - 32 * warp);
       bool ok = true;
@@ -260,9 +275,9 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
       }
       if (!unit) {
         if (ul < n) dd = T.op(ul, ul);
-        scaled = __all_sync(0xffffffffu, ok && ts_moderate(dd, false));
-        if (scaled) {
-          rinv = 1.0 / dd;
+        form = ts_form(n, __all_sync(0xffffffffu, ok && ts_moderate(dd, false)));
+        if (form != kTsDivide) rinv = 1.0 / dd;
+        if (form == kTsScaled) {
 #pragma unroll 8
           for (int k = 0; k < m; ++k) D[warp][k][lane] *= __shfl_sync(0xffffffffu, rinv, k);
         }
@@ -278,7 +293,7 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
       double v[V];
 #pragma unroll
       for (int q = 0; q < V; ++q) v[q] = xc[q * np + 32 * half + lane];
-      ts_solve32(v, D[half], min(32, n - u0 - 32 * half), dd, rinv, unit, scaled);
+      ts_solve32(v, D[half], min(32, n - u0 - 32 * half), dd, rinv, unit, form);
 #pragma unroll
       for (int q = 0; q < V; ++q) xc[q * np + 32 * half + lane] = v[q];
     };
@@ -398,7 +413,7 @@ trisolve_cluster_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_
   double* xv = x + (int64_t)blockIdx.z * stride_x + (int64_t)blockIdx.y * n;
   const int wi = tid >> 2, wq = tid & 3;           // row, part: columns 4 pp + wq
   double cu[16], d[32], dd = 1.0, rinv = 1.0, cs[4];
-  bool scaled = true;
+  TsForm form = kTsScaled;                         // (two blocks and more)
   auto load_update = [&](int w, int b) {
 #pragma unroll
     for (int pp = 0; pp < 16; ++pp)
@@ -415,7 +430,7 @@ trisolve_cluster_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_
   };
   auto load_diag = [&](int b) {
     const int u0 = b * kTsNB;
-    scaled = true;
+    form = kTsScaled;
     dd = rinv = 1.0;
     if (warp < 2) {
       const int ul = u0 + 32 * warp + lane;
@@ -430,9 +445,9 @@ trisolve_cluster_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_
 #pragma unroll
         for (int k = 0; k < 32; ++k) ok = ok && ts_moderate(d[k], true);
         ok = ok && ts_moderate(dd, false);
-        scaled = __all_sync(0xffffffffu, ok);
-        if (scaled) {
-          rinv = 1.0 / dd;
+        form = ts_form(n, __all_sync(0xffffffffu, ok));
+        if (form != kTsDivide) rinv = 1.0 / dd;
+        if (form == kTsScaled) {
 #pragma unroll
           for (int k = 0; k < 32; ++k) d[k] *= __shfl_sync(0xffffffffu, rinv, k);
         }
@@ -447,7 +462,7 @@ trisolve_cluster_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_
   // block b solved in place in xc, out to memory and to every CTA's buffer
   auto solve = [&](double* xc, int b) {
     const int u0 = b * kTsNB;
-    if (warp == 0) xc[lane] = ts_solve32(xc[lane], d, dd, rinv, unit, scaled);
+    if (warp == 0) xc[lane] = ts_solve32(xc[lane], d, 32, dd, rinv, unit, form);
     __syncthreads();
     double s = 0.0;
 #pragma unroll
@@ -457,7 +472,7 @@ trisolve_cluster_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_
     s += __shfl_xor_sync(0xffffffffu, s, 4);
     if ((tid & 7) == 0) xc[32 + (tid >> 3)] -= s;
     __syncthreads();
-    if (warp == 1) xc[32 + lane] = ts_solve32(xc[32 + lane], d, dd, rinv, unit, scaled);
+    if (warp == 1) xc[32 + lane] = ts_solve32(xc[32 + lane], d, 32, dd, rinv, unit, form);
     __syncthreads();
     const double v = xc[tid & (kTsNB - 1)];
 #pragma unroll

@@ -235,3 +235,27 @@ def test_getrs_many_vectors_of_several_systems(dev):
         for s in range(bt):
             assert torch.equal(x[s], _dense.lu_solve_batched(lu[s:s + 1], piv[s:s + 1], b[s:s + 1],
                                                              trans)[0])
+
+
+@pytest.mark.parametrize("n", [2, 3, 8, 31, 32])
+@pytest.mark.parametrize("lower", [True, False])
+def test_trsm_one_block_rounds_each_unknown(dev, n, lower):
+    """Up to 32 unknowns: substitution with each unknown rounded once before it is used,
+    x_t = v_t / t_tt and v_l = fma(-t_lt, x_t, v_l), bit for bit (the FMA in extended
+    precision: a product of two 53-bit values and one sum, rounded once)."""
+    if np.finfo(np.longdouble).nmant < 106:
+        pytest.skip("needs quadruple precision on the host for the exact FMA")
+    rng = np.random.default_rng(n)
+    m = rng.standard_normal((n, n))
+    m[np.arange(n), np.arange(n)] += np.sign(m[np.arange(n), np.arange(n)])
+    b = rng.standard_normal((40, n))
+    order = np.arange(n) if lower else np.arange(n)[::-1]
+    for nv in (1, 40):
+        x = _dense.trsv(_t(m, dev), _t(b[:nv], dev), lower=lower, trans=False, unit=False)
+        v = b[:nv].copy()
+        for i, t in enumerate(order):
+            v[:, t] = v[:, t] / m[t, t]
+            for r in order[i + 1:]:
+                v[:, r] = (v[:, r].astype(np.longdouble) -
+                           np.longdouble(m[r, t]) * v[:, t].astype(np.longdouble)).astype(np.float64)
+        np.testing.assert_array_equal(x.cpu().numpy(), v)
