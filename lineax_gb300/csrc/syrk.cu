@@ -27,9 +27,9 @@ constexpr int kPoNB = 32;       // block rows of the multi-CTA Cholesky
 // Columns per CTA of the block-row kernel: 32 G.  G = 2 above kPoWide trailing
 // columns, where the trailing update beside it wants the SMs (n = 1531: 24
 // instead of 48 of them); G = 1 below, where the block row's own time counts
-// (24 us against 30).  us for the factor with this line, with G = 1 and with G = 2
-// throughout: n = 1000 974, 971 and 1106, 1531 1971, 2089 and 2076, 3000 9334, 9600 and
-// 9439, 8192 153200, 154900 and 153300.
+// (25 us against 30).  us for the factor with this line, with G = 1 and with G = 2
+// throughout: n = 1000 1002, 997 and 1126, 1531 1999, 2120 and 2098, 3000 9367, 9663 and
+// 9455, 8192 153400, 155200 and 153500.
 constexpr int kPoWide = 1024;
 // Unused dynamic shared memory that a block-row CTA reserves, so that no CTA
 // of the trailing update running beside it (17 KB each) shares its SM.
@@ -123,11 +123,11 @@ syrk_f64_kernel(int trans, int64_t n, int64_t k, const double* __restrict__ a, i
 // scale row k of the CTA's columns and update their rows; the owners of rows
 // k + 1 and k + 2 pass on through shared memory what the next step reads.
 // (Warp 4 shares warp 0's sub-partition and stays out of its way.)  What
-// bounds it is warp 0's chain (reciprocal square root, scaling, a barrier, FMA).
-// Measured, n = 1531: 24 to 30 us a block row of 32 (27 to 31 with a square root
+// bounds it is warp 0's chain (the pivot's root and reciprocal, scaling, a barrier, FMA).
+// Measured, n = 1531: 25 to 30 us a block row of 32 (27 to 31 with a square root
 // and a division in the chain); a block
 // row of 64 as a diagonal kernel (138 us) and a column-per-thread substitution
-// (149 us) before.  The whole factorisation 8.4 to 2.2 ms.
+// (149 us) before.  The whole factorisation 8.4 to 2.0 ms.
 // The operations on each element, and their order, are cta_potrf_upper's:
 // row k scaled by 1 / sqrt(a_kk), then one FMA per later row, k ascending.
 // Except for the last block, the factored block does not go back to its place: a CTA
