@@ -41,6 +41,10 @@ struct TsView {
     const int64_t i = row(u), j = row(v);
     return trans ? t[j * ldt + i] : t[i * ldt + j];
   }
+  __device__ __forceinline__ const double* at(int u, int v) const {
+    const int64_t i = row(u), j = row(v);
+    return t + (trans ? j * ldt + i : i * ldt + j);
+  }
 };
 
 // Whether x is zero or of moderate size (2^-500 < |x| < 2^500), by its exponent.
@@ -235,24 +239,36 @@ trisolve_step_kernel(int n, const double* __restrict__ t, int64_t ldt, int64_t s
 // Many vectors: a CTA solves V of them from the first block to the last, in shared
 // memory.  The four CTAs of an SM are at different places of their chains, so the
 // substitutions of one hide behind the updates of others, and there is no launch
-// between blocks.  Bound by the FP64 pipe.  A row of an update belongs to four lanes,
-// with a transpose (rows along the lanes) to one thread, which saves the shuffles'
-// additions.  The operations on every element, and their order, are
-// trisolve_step_kernel's.
+// between blocks.  Bound by the FP64 pipe, or by the matrices where each vector has its
+// own.  The rows of an update:
+//  * kTmRows, no transpose: four lanes to a row, two shuffles;
+//  * kTmColumns, a transpose (the rows lie along the lanes) and a matrix that many
+//    vectors share, and so find in L2: a thread per row, without shuffles;
+//  * kTmSpread, a transpose and few vectors per matrix, which comes from memory: lanes
+//    along 32 rows, a part of the columns per warp and all its loads in flight, the parts
+//    summed through shared memory; and the next diagonal block's entries on their way
+//    during the updates.
+// The operations on every element, and their order, are trisolve_step_kernel's.
 // Measured, n = 1000 with a transpose, us here (V = 1) and with a launch per block: 300
 // vectors 524 and 766, 500 766 and 1155, 1000 1312 and 2102; without one 589 and 765,
-// 872 and 1155, 1475 and 2104.  2000 vectors with V = 2: 2446 (V = 1: 2527).
+// 872 and 1155, 1475 and 2104.  2000 vectors with V = 2: 2446 (V = 1: 2527).  LU solves of
+// 1300 systems of n = 300 with a transpose: one right-hand side 578 (four lanes to a row
+// 862, a launch per block 733), nine 3477 (a thread per row 4252, a launch per block 5224);
+// of one system of n = 2000 with 2000: 17314 with a thread per row, 18365 spread.
 constexpr int kTmCtas = 4;
+constexpr int kTmShared = 64;       // vectors of one matrix from which it is read from L2
+enum TmForm { kTmRows, kTmColumns, kTmSpread };
 
-template <int V>
+template <int V, TmForm FORM>
 __global__ void __launch_bounds__(kTsThreads, kTmCtas)
 trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt, int64_t stride_t,
-                     int fwd, int trans, int unit, double* __restrict__ x, int64_t stride_x) {
+                     int fwd, int unit, double* __restrict__ x, int64_t stride_x) {
   extern __shared__ double ts_x[];                 // V vectors in solve order, zeros past n
   __shared__ double D[2][32][33];                  // the diagonal block's halves, by column
+  __shared__ double P[2][FORM == kTmSpread ? V : 1][4][kTsNB];  // partial sums of two tiles
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nblk = (n + kTsNB - 1) / kTsNB, np = nblk * kTsNB;
-  const TsView T{t + (int64_t)blockIdx.y * stride_t, ldt, n, fwd != 0, trans != 0};
+  const TsView T{t + (int64_t)blockIdx.y * stride_t, ldt, n, fwd != 0, FORM != kTmRows};
   double* xv = x + (int64_t)blockIdx.y * stride_x + (int64_t)blockIdx.x * V * n;
   const int nv = min(V, nrhs - (int)blockIdx.x * V);
   const int wi = tid >> 2, wq = tid & 3;           // row, part: columns 4 pp + wq
@@ -260,6 +276,19 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
   for (int q = 0; q < V; ++q)
     for (int u = tid; u < np; u += kTsThreads)
       ts_x[q * np + u] = (q < nv && u < n) ? xv[(int64_t)q * n + T.row(u)] : 0.0;
+  // the halves of block b (warps 0 and 1) on their way to D, a lane's own entries
+  auto fetch = [&](int b) {
+    const int u1 = b * kTsNB + 32 * warp, m = min(32, n - u1);
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+      const bool in = k < lane && lane < m;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(&D[warp][k][lane]);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst),
+                   "l"(in ? T.at(u1 + lane, u1 + k) : T.t), "r"(in ? 8 : 0)
+                   : "memory");
+    }
+  };
+  if (FORM == kTmSpread && warp < 2) fetch(0);
   for (int b = 0; b < nblk; ++b) {
     const int u0 = b * kTsNB;
     double dd = 1.0, rinv = 1.0, cs[4];
@@ -267,10 +296,16 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
     if (warp < 2) {
       const int ul = u0 + 32 * warp + lane, m = min(32, n - u0 - 32 * warp);
       bool ok = true;
+      if (FORM == kTmSpread) asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll 8
       for (int k = 0; k < m; ++k) {
-        const double v = (ul < n && k < lane) ? T.op(ul, u0 + 32 * warp + k) : 0.0;
-        D[warp][k][lane] = v;
+        double v;
+        if (FORM == kTmSpread) {
+          v = D[warp][k][lane];
+        } else {
+          v = (ul < n && k < lane) ? T.op(ul, u0 + 32 * warp + k) : 0.0;
+          D[warp][k][lane] = v;
+        }
         ok = ok && ts_moderate(v, true);
       }
       if (!unit) {
@@ -315,7 +350,7 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
       if (warp == 1) solve(1);
       __syncthreads();
     }
-    if (trans) {
+    if constexpr (FORM == kTmColumns) {
       for (int u = u0 + kTsNB + tid; u < n; u += kTsThreads) {
         double acc[V][4][2];
 #pragma unroll
@@ -340,23 +375,46 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
           ts_x[q * np + u] -= ((acc[q][0][0] + acc[q][0][1]) + (acc[q][1][0] + acc[q][1][1])) +
                               ((acc[q][2][0] + acc[q][2][1]) + (acc[q][3][0] + acc[q][3][1]));
       }
-      continue;
-    }
-    for (int w = b + 1; w < nblk; ++w) {
-      double cu[16];
+    } else if constexpr (FORM == kTmSpread) {
+      if (warp < 2 && b + 1 < nblk) fetch(b + 1);
+      const int part = warp & 3, r = 32 * (warp >> 2) + lane;
+      for (int w = b + 1; w < nblk; ++w) {
+        const int u = w * kTsNB + r;
+        double cu[16];
 #pragma unroll
-      for (int pp = 0; pp < 16; ++pp)
-        cu[pp] = (w * kTsNB + wi < n) ? T.op(w * kTsNB + wi, u0 + 4 * pp + wq) : 0.0;
+        for (int pp = 0; pp < 16; ++pp) cu[pp] = u < n ? T.op(u, u0 + 4 * pp + part) : 0.0;
 #pragma unroll
-      for (int q = 0; q < V; ++q) {
-        double acc[2] = {0.0, 0.0};
+        for (int q = 0; q < V; ++q) {
+          double acc[2] = {0.0, 0.0};
+#pragma unroll
+          for (int pp = 0; pp < 16; ++pp)
+            acc[pp & 1] = fma(cu[pp], xc[q * np + 4 * pp + part], acc[pp & 1]);
+          P[w & 1][q][part][r] = acc[0] + acc[1];
+        }
+        __syncthreads();
+        if (tid < V * kTsNB) {
+          const int q = tid / kTsNB, e = tid % kTsNB;
+          const double (&p)[4][kTsNB] = P[w & 1][q];
+          ts_x[q * np + w * kTsNB + e] -= (p[0][e] + p[1][e]) + (p[2][e] + p[3][e]);
+        }
+      }
+    } else {
+      for (int w = b + 1; w < nblk; ++w) {
+        double cu[16];
 #pragma unroll
         for (int pp = 0; pp < 16; ++pp)
-          acc[pp & 1] = fma(cu[pp], xc[q * np + 4 * pp + wq], acc[pp & 1]);
-        double s = acc[0] + acc[1];
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (wq == 0) ts_x[q * np + w * kTsNB + wi] -= s;
+          cu[pp] = (w * kTsNB + wi < n) ? T.op(w * kTsNB + wi, u0 + 4 * pp + wq) : 0.0;
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          double acc[2] = {0.0, 0.0};
+#pragma unroll
+          for (int pp = 0; pp < 16; ++pp)
+            acc[pp & 1] = fma(cu[pp], xc[q * np + 4 * pp + wq], acc[pp & 1]);
+          double s = acc[0] + acc[1];
+          s += __shfl_xor_sync(0xffffffffu, s, 1);
+          s += __shfl_xor_sync(0xffffffffu, s, 2);
+          if (wq == 0) ts_x[q * np + w * kTsNB + wi] -= s;
+        }
       }
     }
   }
@@ -377,10 +435,13 @@ trisolve_many_kernel(int n, int nrhs, const double* __restrict__ t, int64_t ldt,
 // vectors: n = 1000 1280 and 1060, 2000 3360 and 3870).
 constexpr int kTmMaxN = 4096;
 
-static int ts_many(int64_t vectors, int n) {
+static int ts_many(int64_t batch, int n, int nrhs) {
+  const int64_t vectors = batch * nrhs;
   if (n > kTmMaxN || 2 * vectors < 3 * sm_count()) return 0;
   const int64_t per_sm = (vectors + sm_count() - 1) / sm_count();
-  return per_sm > 8 || (per_sm > kTmCtas && n <= (per_sm <= 6 ? 1024 : 768)) ? 2 : 1;
+  const bool two = per_sm > 8 || (per_sm > kTmCtas && n <= (per_sm <= 6 ? 1024 : 768));
+  // (a system's odd vector has a CTA of its own: no loss among eight or more)
+  return two && (nrhs % 2 == 0 || nrhs >= 8) ? 2 : 1;
 }
 
 // The whole solve in one launch for n up to 64 kTcMaxBlocks: a cluster of C CTAs
@@ -554,13 +615,17 @@ int trisolve_blocked(int64_t batch, int n, int nrhs, const double* t, int64_t ld
                   "trisolve: launch");
     return check_launch("trisolve");
   }
-  if (const int v = ts_many(batch * nrhs, n)) {
-    auto fn = v == 2 ? trisolve_many_kernel<2> : trisolve_many_kernel<1>;
+  if (const int v = ts_many(batch, n, nrhs)) {
+    auto fn = v == 2 ? trisolve_many_kernel<2, kTmRows> : trisolve_many_kernel<1, kTmRows>;
+    if (trans && nrhs >= kTmShared)
+      fn = v == 2 ? trisolve_many_kernel<2, kTmColumns> : trisolve_many_kernel<1, kTmColumns>;
+    else if (trans)
+      fn = v == 2 ? trisolve_many_kernel<2, kTmSpread> : trisolve_many_kernel<1, kTmSpread>;
     const size_t smem = (size_t)v * nblk * kTsNB * sizeof(double);
     LXGB_CUDA_TRY(ensure_dynamic_smem(reinterpret_cast<const void*>(fn), (int)smem),
                   "trisolve: set smem");
     fn<<<dim3((unsigned)((nrhs + v - 1) / v), (unsigned)batch), kTsThreads, smem, st>>>(
-        n, nrhs, t, ldt, stride_t, fwd, trans, unit, x, stride_x);
+        n, nrhs, t, ldt, stride_t, fwd, unit, x, stride_x);
     return check_launch("trisolve");
   }
   for (int b = 0; b < nblk; ++b) {
